@@ -12,10 +12,11 @@ For each evaluator in ``mbx_b200.specs.SPECS`` this writes
 * ``<name>_pip_s32`` (types in SHIFT_TYPES): the FP32 trie of the type's FP32
   basis (codegen/shift.py), the mixed-precision polynomial.
 
-The tries are generated for STRAIGHT_TYPES only; every evaluator also gets a
-table unit ``<name>_t.cu`` (coefficient adjoint and, without a trie, the
-evaluation itself) over the term tables that ``write_term_tables`` packs into
-one binary embedded in the library.
+The tries are those of the polynomial in the symmetry-adapted variables w
+(codegen/wbasis.py), which has 3 to 8 times fewer terms than in the variables
+of the model.  Every evaluator also gets a table unit ``<name>_t.cu`` (the
+coefficient adjoint) over the term tables that ``write_term_tables`` packs
+into one binary embedded in the library.
 
 The trie.  Every term is a monomial x_v1 x_v2 ... (variables sorted in a fixed
 order); the monomials form a prefix tree.  With P(n) the product along the path
@@ -43,6 +44,7 @@ sys.path.insert(0, os.path.dirname(PKG))
 
 from mbx_b200.specs import SPECS, ONEBODY_SPECS, LP_GAMMA_IN, LP_GAMMA_OUT  # noqa: E402
 from mbx_b200.tables import load_pip  # noqa: E402
+from mbx_b200.codegen.wbasis import by_key as wtable_by_key, emit as emit_transforms, table_key, wtable  # noqa: E402
 
 OUT = os.path.join(PKG, "csrc", "gen")
 
@@ -56,26 +58,30 @@ def lit(v):
 
 
 class Trie:
-    def __init__(self, table):
-        freq = collections.Counter()
-        for t in range(table.nterms):
-            for v in set(table.var[t, :table.deg[t]].tolist()):
-                freq[v] += 1
-        order = [v for v, _ in freq.most_common()] + [v for v in range(table.nvars) if v not in freq]
-        self.rank = {v: i for i, v in enumerate(order)}
-        self.root = {"coef": [], "kids": collections.OrderedDict()}
-        for t in range(table.nterms):
-            mono = sorted(table.var[t, :table.deg[t]].tolist(), key=lambda v: self.rank[v])
-            node = self.root
-            for v in mono:
-                node = node["kids"].setdefault(v, {"coef": [], "kids": collections.OrderedDict()})
-            node["coef"].append((int(table.k[t]), float(table.coef[t])))
-        self._sort(self.root)
+    """The monomials as a tree.  At every node the variable that occurs in
+    the most of the remaining monomials is split off first (a multivariate
+    Horner scheme): fewer inner nodes than one variable order for the whole
+    tree (MB-pol 3b: 1274 against 2249, 16.0k against 19.4k FP64 operations
+    per trimer)."""
 
-    def _sort(self, node):
-        node["kids"] = collections.OrderedDict(sorted(node["kids"].items(), key=lambda kv: self.rank[kv[0]]))
-        for ch in node["kids"].values():
-            self._sort(ch)
+    def __init__(self, table):
+        self.root = self._node([(table.var[t, :table.deg[t]].tolist(), (int(table.k[t]), float(table.coef[t])))
+                                for t in range(table.nterms)])
+
+    def _node(self, terms):
+        node = {"coef": [c for m, c in terms if not m], "kids": collections.OrderedDict()}
+        terms = [(m, c) for m, c in terms if m]
+        while terms:
+            freq = collections.Counter(v for m, _ in terms for v in set(m))
+            best = max(freq, key=lambda v: (freq[v], -v))
+            mine = []
+            for m, c in terms:
+                if best in m:
+                    i = m.index(best)
+                    mine.append((m[:i] + m[i + 1:], c))
+            terms = [(m, c) for m, c in terms if best not in m]
+            node["kids"][best] = self._node(mine)
+        return node
 
     def counts(self):
         leaves = inner = 0
@@ -91,16 +97,7 @@ class Trie:
         return leaves, inner
 
 
-# Code-shape options of the generated evaluators: how the trie is cut into
-# separately compiled pieces ("top": whole top-level subtrees, "terms":
-# contiguous term ranges) and into how many independent FMA chains the leaf sum
-# of a node is split (1 = one serial chain per node; 2 chains measured slower
-# on the MB-pol 3b gradient kernel with the code prefetched: 1.38 vs 1.32 ms
-# back to back, 2048-water trimers).
-SPLIT = "terms"
-ACC_CHAINS = 1
-
-# Mixed precision (paired FP32 trie, the "s" kernels).  "median": the
+# Mixed precision (the "s" kernels).  "median": the
 # polynomial is re-expanded around a symmetric reference point in the middle
 # of liquid data (codegen/shift.py); "identity": the original basis in FP32.
 # Types not listed run FP64 in the mixed mode.  MB-pol 2b is not listed: in
@@ -109,7 +106,7 @@ ACC_CHAINS = 1
 # (the shifted basis does not condition it either).
 SHIFT_TYPES = {"mbpol3b": "median"}
 # Types of SHIFT_TYPES whose mixed kernel is the quadratic form on the tensor
-# cores (codegen/qf.py, csrc/qf_kernel.cuh) instead of the paired FP32 trie:
+# cores (codegen/qf.py, csrc/qf_kernel.cuh):
 # MB-pol 3b, 442 products of degree 2 in the basis (data/mbpol3b.qf.json).
 QF_TYPES = {"mbpol3b"}
 # Optional: n-mers whose first-atom distance is below this radius (A) run the
@@ -127,26 +124,11 @@ def coef_expr(coefs, fp32=False):
         ref = ("coef.f(%d)" if fp32 else "coef[%d]") % k
         if c == 1.0:
             parts.append(ref)
+        elif c == -1.0:
+            parts.append("(-%s)" % ref)
         else:
             parts.append("(%s * %s)" % (ref, lit(c) + ("f" if fp32 else "")))
     return " + ".join(parts) if parts else None
-
-
-def subtree_size(n):
-    return 1 + sum(subtree_size(c) for c in n["kids"].values())
-
-
-def partition(trie, nparts):
-    """Top-level subtrees split into nparts groups of similar size (greedy)."""
-    kids = sorted(trie.root["kids"].items(), key=lambda kv: -subtree_size(kv[1]))
-    nparts = max(1, min(nparts, len(kids)))
-    parts = [[] for _ in range(nparts)]
-    load = [0] * nparts
-    for var, ch in kids:
-        i = load.index(min(load))
-        parts[i].append((var, ch))
-        load[i] += subtree_size(ch)
-    return [p for p in parts if p]
 
 
 def split_terms(trie, nparts):
@@ -177,26 +159,27 @@ def split_terms(trie, nparts):
 
 
 def lock_threads(nvars):
-    """Threads of a lockstep evaluation block.  Up to 32 variables the
-    variables and their gradient accumulators (4 registers per variable) fit
-    under 168 registers, so a block of 384 threads (12 warps per SM) is
-    resident; wider polynomials need the full 255 registers (256 threads)."""
+    """Threads of a lockstep evaluation block.  The kernels wait for
+    instructions more than for anything else, and a block's warps share every
+    fetch, so as many warps as the columns of x and g leave room for in 227 KB
+    of shared memory: 384 threads (168 registers) up to 36 variables, else 256
+    (255 registers), 128 above 56 variables.  MB-pol 3b gradients of 132k
+    trimers: 410 us with 384 threads, 475 with 320, 550 with 256; MB-pol 2b,
+    39k dimers: 81 us with 384, 109 with 256."""
     if nvars > 56:
-        # x and g columns of 256 threads would exceed the 227 KB of shared memory
         return 128
-    return 384 if nvars <= 32 else 256
+    return 384 if nvars <= 36 else 256
 
 
 def parts_for(nterms, nvars=36):
     """Number of separately compiled pieces of a trie.  A single straight-line
-    function of 10^4-10^5 FMAs leaves the register allocator live ranges it
-    cannot fit (kilobytes of spills), and the code of a piece should stay
-    small enough for the instruction cache that the warps of a lockstep block
-    share: ~400 terms per piece in 384-thread blocks, ~600 in 256-thread
-    blocks with shared-memory x/g columns (MB-pol 3b gradient kernel on the
-    2048-water trimers: 1.42/1.39/1.35/1.32/1.47 ms at 300/375/450/600/700
-    terms per piece, and 2.1 ms at 800-900, past the instruction cache)."""
-    per = 400 if lock_threads(nvars) == 384 else 600
+    function of 10^4 FMAs leaves the register allocator live ranges it cannot
+    fit, and the code of a piece should stay small enough for the instruction
+    cache that the warps of a lockstep block share.  Measured on 132k MB-pol 3b
+    trimers (256 threads): 570, 550 and 564 us at 300, 600 and 900 terms a
+    piece.  Small batches are cut by pieces over the SMs (LockPlan), which asks
+    for no larger ones."""
+    per = 400 if nvars <= 32 else 600
     if nvars > 56:
         # a piece loads every variable it uses into registers: fewer terms per
         # piece for the widest polynomials
@@ -204,51 +187,9 @@ def parts_for(nterms, nvars=36):
     return max(1, (nterms + per - 1) // per)
 
 
-# FP64 kernels whose coefficients are copied to shared memory per block (the
-# trie reads them from there instead of the constant bank): measured on the
-# 2048-water trimers, MB-pol 3b 1.37 ms (shared, 450-term pieces) vs 1.58 ms
-# (constant); MB-pol 2b is faster from the constant bank (0.18 vs 0.25 ms).
-SMEM_COEF_TYPES = {"mbpol3b"}
-
-# Types whose tries are generated in the coset form (codegen/coset.py): a
-# polynomial R of ~1/24 of the terms, run once per permutation of a
-# transversal of the symmetry group, so that its code stays in the
-# instruction cache; the kernels' coefficients are scaled on the host.
-# COSET_PIECE_TERMS: terms of R per separately compiled piece.
-# Measured on the 2048-water trimers (L2 flushed between calls, the code
-# prefetch launch in use): MB-pol 3b FP64 1.73 ms in the coset form against
-# 1.36 ms for the full trie, paired FP32 0.96 against 0.91 ms -- with the
-# prefetch the full trie's code is L2-resident already, and the coset form's
-# 10% more arithmetic and per-permutation loads then cost more than its
-# smaller code saves.  No type uses it; the form is kept for polynomials
-# whose trie does not fit in L2.
-COSET_TYPES = set()
-COSET_PIECE_TERMS = 400
-
-
-_COSET = {}
-
-
-def coset_of(name, shifted_basis=False):
-    """(coset form, R table) of an evaluator's polynomial, or of its FP32
-    (shifted) basis."""
-    key = (name, shifted_basis)
-    if key not in _COSET:
-        from mbx_b200.codegen.coset import coset_form, CosetTable
-        spec = SPECS[name]
-        if shifted_basis:
-            from mbx_b200.codegen.shift import ShiftedTable
-            sp = shifted_pip(name)
-            cf = coset_form(spec, ShiftedTable(sp, name), sp.group)
-        else:
-            cf = coset_form(spec, load_pip(name))
-        _COSET[key] = (cf, CosetTable(cf, spec.nvars, name))
-    return _COSET[key]
-
-
-def emit_split(trie, nvars, name, out, nparts, arrays, body, ret="double", perms=None):
+def emit_split(trie, nvars, name, out, nparts, arrays, body, ret="double"):
     """Emits name_partK as __noinline__ functions over strided pointers to the
-    caller's arrays, and the wrappers that call them in turn.
+    caller's arrays, and the dispatcher name_piece.
 
     arrays: [(name, ctype, role)] with role "in" (read: copied into a local
     register array on entry) or "acc" (accumulated: zeroed locally, added to
@@ -258,103 +199,44 @@ def emit_split(trie, nvars, name, out, nparts, arrays, body, ret="double", perms
     lockstep kernels keep x and g there: shared memory instead of the
     thread's stack for the values every piece loads and stores).  body(w,
     subtrees) writes the evaluation of the subtrees into the local arrays and
-    into E.
-
-    perms (coset form, codegen/coset.py): the trie is R and every piece runs
-    its subtrees once per permutation p_t, reading variable v of the caller's
-    arrays at column p_t[v] and adding its gradient there; the permutations
-    sit in a constant-memory table, and a piece's code is reused |T| times in
-    a row while it is in the instruction cache."""
+    into E."""
     import re
     w = out.append
-    zero = {"float": "0.0f", "double": "0.0", "f2_t": "0ull"}
-    e0 = "make_double2(0.0, 0.0)" if ret == "double2" else "0.0"
-    pieces = split_terms(trie, nparts) if SPLIT == "terms" else partition(trie, nparts)
+    zero = {"double": "0.0"}
+    e0 = "0.0"
+    pieces = split_terms(trie, nparts)
     params = ", ".join("%s%s* __restrict__ %sm" % ("const " if role == "in" else "", ct, a) for a, ct, role in arrays)
-    if perms is not None:
-        # the table lives in constant memory and is copied to shared memory
-        # by the lock / piece entry points; the pieces read it with a
-        # non-removable load at every use, so that the 36 column offsets are
-        # not kept in registers across the piece (they would spill)
-        w("// coset form: %d permutations of the %d variables (x_local[v] = x[perm[t][v]])" % (len(perms), nvars))
-        w("static __constant__ int %s_perm[%d] = {%s};" %
-          (name, len(perms) * nvars, ", ".join(str(v) for p in perms for v in p)))
-        w("static __shared__ int %s_sperm[%d];" % (name, len(perms) * nvars))
-        w("__device__ __forceinline__ void %s_load_perm() {" % name)
-        w("    for (int i = threadIdx.x; i < %d; i += blockDim.x) %s_sperm[i] = %s_perm[i];" %
-          (len(perms) * nvars, name, name))
-        w("    __syncthreads();")
-        w("}")
+    constant = coef_expr(trie.root["coef"])
     for i, sub in enumerate(pieces):
         text = []
         body(text.append, sub)
+        if i == 0 and constant:
+            text.append("    E += %s;" % constant)
         code = "\n".join(text)
         w("template <class Coef, int S>")
         w("__device__ __noinline__ %s %s_part%d(const Coef& coef, %s) {" % (ret, name, i, params))
         w("    %s E = %s;" % (ret, e0))
-        pad = "    "
-        if perms is not None:
-            w("#pragma unroll 1")
-            w("    for (int t = 0; t < %d; ++t) {" % len(perms))
-            w("    const int* o = %s_sperm + t * %d;" % (name, nvars))
         for a, ct, role in arrays:
             used = sorted({int(v) for v in re.findall(r"\b%s\[(\d+)\]" % a, code)})
             w("    %s %s[%d];" % (ct, a, nvars))
             for v in used:
-                col = ("lds_pinned(o + %d)" % v) if perms is not None else str(v)
-                w("    %s[%d] = %s;" % (a, v, ("%sm[%s * S]" % (a, col)) if role == "in" else zero[ct]))
+                w("    %s[%d] = %s;" % (a, v, ("%sm[%d * S]" % (a, v)) if role == "in" else zero[ct]))
         w(code)
         for a, ct, role in arrays:
             if role == "acc":
                 used = sorted({int(v) for v in re.findall(r"\b%s\[(\d+)\]" % a, code)})
                 for v in used:
-                    col = ("lds_pinned(o + %d)" % v) if perms is not None else str(v)
-                    if ct == "f2_t":
-                        w("    %sm[%s * S] = f2_add(%sm[%s * S], %s[%d]);" % (a, col, a, col, a, v))
-                    else:
-                        w("    %sm[%s * S] += %s[%d];" % (a, col, a, v))
-        if perms is not None:
-            w("    }")
+                    w("    %sm[%d * S] += %s[%d];" % (a, v, a, v))
         w("    return E;")
         w("}")
 
-    def calls(lock, targs, args):
-        for i in range(len(pieces)):
-            call = "%s_part%d<%s>(coef, %s)" % (name, i, targs, args)
-            bar = " __syncthreads();" if lock else ""
-            if ret == "double2":
-                w("    { const double2 e = %s; E.x += e.x; E.y += e.y; }%s" % (call, bar))
-            else:
-                w("    E += %s;%s" % (call, bar))
-
-    # name(coef, x[], g[]): the pieces in turn over the thread's own arrays
-    sig = ", ".join("%s%s (&%s)[%d]" % ("const " if role == "in" else "", ct, a, nvars) for a, ct, role in arrays)
-    w("template <class Coef>")
-    w("__device__ __forceinline__ %s %s(const Coef& coef, %s) {" % (ret, name, sig))
-    w("    %s E = %s;" % (ret, e0))
-    calls(False, "Coef, 1", ", ".join(a for a, _, _ in arrays))
-    w("    return E;")
-    w("}")
-    # name_lock<S>(coef, xm, gm): over shared arrays [v][S] (pointers at the
-    # thread's column), a block barrier after every piece so that all warps
-    # of a block run the same piece at the same time and share its
-    # instruction fetches
-    w("template <int S, class Coef>")
-    w("__device__ __forceinline__ %s %s_lock(const Coef& coef, %s) {" % (ret, name, params))
-    if perms is not None:
-        w("    %s_load_perm();" % name)
-    w("    %s E = %s;" % (ret, e0))
-    calls(True, "Coef, S", ", ".join("%sm" % a for a, _, _ in arrays))
-    w("    return E;")
-    w("}")
-    # name_piece<S>(k, coef, xm, gm): piece k alone, the same instantiation
-    # as name_lock<S> calls (holder_prime_kernel runs one piece per block to
-    # bring the code of all pieces into L2 in parallel)
-    w("static constexpr int %s_NPIECES = %d;" % (name, len(pieces)))
+    # name_piece<S>(k, coef, xm, gm): piece k over shared arrays [v][S]
+    # (pointers at the thread's column).  The lockstep kernels run the pieces
+    # of a chunk in turn with a block barrier after each, so that all warps of
+    # a block share the instruction fetches of a piece; their prefetch launch
+    # runs one piece per block
     w("template <int S, class Coef>")
     w("__device__ __forceinline__ %s %s_piece(int k, const Coef& coef, %s) {" % (ret, name, params))
-    if perms is not None:
-        w("    %s_load_perm();" % name)
     w("    switch (k) {")
     args = ", ".join("%sm" % a for a, _, _ in arrays)
     for i in range(len(pieces)):
@@ -364,7 +246,7 @@ def emit_split(trie, nvars, name, out, nparts, arrays, body, ret="double", perms
     w("}")
 
 
-def emit_pip(trie, nvars, name, out, nparts=1, perms=None):
+def emit_pip(trie, nvars, name, out, nparts=1):
     """FP64 value + gradient (multivariate Horner trie, reverse mode)."""
     out.append("// %s: polynomial and reverse-mode gradient (multivariate Horner trie)" % name)
 
@@ -379,23 +261,12 @@ def emit_pip(trie, nvars, name, out, nparts=1, perms=None):
                 w("    { const double %s = %s * x[%d];" % (P, pexpr, var))
             ce = coef_expr(n["coef"])
             w("      double %s = %s;" % (V, ce if ce else "0.0"))
-            nleaf = sum(1 for ch in n["kids"].values() if not ch["kids"])
-            split = ACC_CHAINS > 1 and nleaf >= 2 * ACC_CHAINS
-            if split:
-                # leaf sums in ACC_CHAINS independent chains, joined at the end
-                for j in range(1, ACC_CHAINS):
-                    w("      double %s_%d = 0.0;" % (V, j))
-            li = 0
             for cv, ch in n["kids"].items():
                 if ch["kids"]:
                     node(ch, cv, depth + 1, P)
                 else:
                     c = coef_expr(ch["coef"])
-                    acc = V if not split or li % ACC_CHAINS == 0 else "%s_%d" % (V, li % ACC_CHAINS)
-                    li += 1
-                    w("      %s = fma(%s, x[%d], %s); g[%d] = fma(%s, %s, g[%d]);" % (acc, c, cv, acc, cv, c, P, cv))
-            if split:
-                w("      %s += %s;" % (V, " + ".join("%s_%d" % (V, j) for j in range(1, ACC_CHAINS))))
+                    w("      %s = fma(%s, x[%d], %s); g[%d] = fma(%s, %s, g[%d]);" % (V, c, cv, V, cv, c, P, cv))
             if pexpr is None:
                 w("      g[%d] += %s; E = fma(x[%d], %s, E); }" % (var, V, var, V))
             else:
@@ -409,62 +280,7 @@ def emit_pip(trie, nvars, name, out, nparts=1, perms=None):
                 c = coef_expr(ch["coef"])
                 w("    E = fma(%s, x[%d], E); g[%d] += %s;" % (c, var, var, c))
 
-    emit_split(trie, nvars, name, out, nparts, [("x", "double", "in"), ("g", "double", "acc")], body, perms=perms)
-
-
-def emit_pip_f32x2(trie, nvars, name, out, nparts=1, perms=None):
-    """FP32 value + gradient over the trie for two n-mers at once (the low and
-    high halves of every f2_t, paired FP32 instructions): monomials,
-    coefficients and leaf sums in FP32; the top-level products are added to
-    the two energies in FP64."""
-    out.append("// %s: paired FP32 polynomial and reverse-mode gradient (multivariate Horner trie)" % name)
-
-    def cexpr(coefs):
-        if not coefs:
-            return None
-        assert all(c == 1.0 for _, c in coefs)
-        parts = ["coef.f2(%d)" % k for k, _ in coefs]
-        e = parts[0]
-        for p in parts[1:]:
-            e = "f2_add(%s, %s)" % (e, p)
-        return e
-
-    def body(w, subtrees):
-        def node(n, var, depth, pexpr):
-            P = "P%d" % depth
-            V = "V%d" % depth
-            if pexpr is None:
-                w("    { const f2_t %s = x[%d];" % (P, var))
-            else:
-                w("    { const f2_t %s = f2_mul(%s, x[%d]);" % (P, pexpr, var))
-            ce = cexpr(n["coef"])
-            w("      f2_t %s = %s;" % (V, ce if ce else "0ull"))
-            for cv, ch in n["kids"].items():
-                if ch["kids"]:
-                    node(ch, cv, depth + 1, P)
-                else:
-                    c = cexpr(ch["coef"])
-                    w("      { const f2_t c = %s; %s = f2_fma(c, x[%d], %s); g[%d] = f2_fma(c, %s, g[%d]); }" %
-                      (c, V, cv, V, cv, P, cv))
-            if pexpr is None:
-                w("      g[%d] = f2_add(g[%d], %s);" % (var, var, V))
-                w("      E.x = fma((double)f2_lo(x[%d]), (double)f2_lo(%s), E.x); "
-                  "E.y = fma((double)f2_hi(x[%d]), (double)f2_hi(%s), E.y); }" % (var, V, var, V))
-            else:
-                w("      g[%d] = f2_fma(%s, %s, g[%d]); V%d = f2_fma(x[%d], %s, V%d); }" %
-                  (var, pexpr, V, var, depth - 1, var, V, depth - 1))
-
-        for var, ch in subtrees:
-            if ch["kids"]:
-                node(ch, var, 1, None)
-            else:
-                c = cexpr(ch["coef"])
-                w("    { const f2_t c = %s; g[%d] = f2_add(g[%d], c);" % (c, var, var))
-                w("      E.x = fma((double)f2_lo(c), (double)f2_lo(x[%d]), E.x); "
-                  "E.y = fma((double)f2_hi(c), (double)f2_hi(x[%d]), E.y); }" % (var, var))
-
-    emit_split(trie, nvars, name, out, nparts, [("x", "f2_t", "in"), ("g", "f2_t", "acc")], body, ret="double2",
-               perms=perms)
+    emit_split(trie, nvars, name, out, nparts, [("x", "double", "in"), ("g", "double", "acc")], body)
 
 
 def shifted_pip(name):
@@ -488,7 +304,7 @@ def shifted_pip(name):
 _SHIFTED = {}
 
 
-def emit_pip_energy(trie, nvars, name, out, nparts=1, perms=None):
+def emit_pip_energy(trie, nvars, name, out, nparts=1):
     """FP64 value only: plain Horner over the trie."""
     def body(w, subtrees):
         def node(n, var, depth):
@@ -509,7 +325,7 @@ def emit_pip_energy(trie, nvars, name, out, nparts=1, perms=None):
             else:
                 w("    E = fma(%s, x[%d], E);" % (coef_expr(ch["coef"]), var))
 
-    emit_split(trie, nvars, name, out, nparts, [("x", "double", "in")], body, perms=perms)
+    emit_split(trie, nvars, name, out, nparts, [("x", "double", "in")], body)
 
 
 def emit_vars(spec, out):
@@ -568,7 +384,7 @@ def emit_vars(spec, out):
     w("}")
 
 
-def emit_traits(spec, table, straight, out):
+def emit_traits(spec, table, straight, npieces, out):
     """Compile-time description the kernel templates in holder_kernel.cuh use."""
     w = out.append
     n = spec.name
@@ -576,16 +392,16 @@ def emit_traits(spec, table, straight, out):
     first = [0, nat[0], nat[0] + nat[1]]
     ns = len(spec.sites)
     w("struct %s_T {" % n)
-    w("    static constexpr int NBODY = %d, NVARS = %d, NREAL = %d, NSITES = %d, NCOEF = %d, NTERMS = %d;" %
-      (spec.nbody, spec.nvars, spec.nreal, ns, spec.ncoef, table.nterms))
+    w("    static constexpr int NBODY = %d, NVARS = %d, NREAL = %d, NSITES = %d, NCOEF = %d;" %
+      (spec.nbody, spec.nvars, spec.nreal, ns, spec.ncoef))
     w("    static constexpr int NAT0 = %d, NAT1 = %d, NAT2 = %d;" % tuple(nat))
     w("    static constexpr int FIRST0 = %d, FIRST1 = %d, FIRST2 = %d;" % tuple(first))
-    w("    static constexpr int SWITCH_TRIPLE = %d, SKIP = %d, STRAIGHT = %d, DEGREE = %d;" %
+    w("    static constexpr int SWITCH_TRIPLE = %d, SKIP = %d, DEGREE = %d;" %
       ({"pair": 0, "triple": 1, "triple2": 2, "cos2": 3, "none": 0}[spec.switch],
        {"pair_gt": 0, "two_of_three_gt": 1, "all_three_gt": 2, "none": 0}[spec.skip],
        1 if straight else 0, spec.degree))
     w("    static constexpr int TPAIRS = %d;  // (variable, exponent) pairs of a term, at most" %
-      term_pairs_max(table))
+      term_pairs_max(table_key(n)))
     w("    static constexpr double RI = %s, RF = %s;" % (lit(spec.ri), lit(spec.rf)))
     w("    static constexpr int VIRIAL_RAW = %d;  // virial of the unswitched polynomial gradient" %
       (1 if spec.virial == "raw" else 0))
@@ -596,17 +412,13 @@ def emit_traits(spec, table, straight, out):
       (1 if shifted_type else 0, 256 if shifted_type else lock_threads(spec.nvars)))
     w("    static constexpr int NORB = %d;  // coefficients of the FP32 basis" %
       (shifted_pip(n).norb if shifted_type else 1))
-    w("    static constexpr int SMEM_COEF = %d;  // FP64 kernel reads its coefficients from shared memory" %
-      (1 if n in SMEM_COEF_TYPES else 0))
+    w("    static constexpr int NCW = %d;  // coefficients of the polynomial in the w variables" % wtable(n).ncoef)
+    w("    __device__ __forceinline__ static void to_w(double (&x)[%d]) { %s_to_w(x); }" % (spec.nvars, n))
+    w("    __device__ __forceinline__ static void from_w(double (&g)[%d]) { %s_from_w(g); }" % (spec.nvars, n))
 
     if shifted_type:
         w("    __device__ __forceinline__ static void shift(const double (&x)[%d], float (&xf)[%d]) "
           "{ %s_shift(x, xf); }" % (spec.nvars, spec.nvars, n))
-    if shifted_type and n not in QF_TYPES:
-        w("    template <int S, class C> __device__ __forceinline__ static double2 pip_s32_lock(const C& c, "
-          "const f2_t* __restrict__ x, f2_t* __restrict__ g) { return %s_pip_s32_lock<S>(c, x, g); }" % n)
-        w("    template <int S, class C> __device__ __forceinline__ static double2 pip_s32_piece(int k, const C& c, "
-          "const f2_t* __restrict__ x, f2_t* __restrict__ g) { return %s_pip_s32_piece<S>(k, c, x, g); }" % n)
     w("    __device__ __forceinline__ static void sites(const double (&r)[%d][3], double (&s)[%d][3]) { %s_sites(r, s); }" %
       (spec.nreal, ns, n))
     w("    __device__ __forceinline__ static void vars(const double (&s)[%d][3], double (&x)[%d]) { %s_vars(s, x); }" %
@@ -618,19 +430,11 @@ def emit_traits(spec, table, straight, out):
     w("    template <class G, class Q> __device__ __forceinline__ static void chain_q(const double (&s)[%d][3], "
       "const G& g, const Q& q, double (&sg)[%d][3]) { %s_chain_q(s, g, q, sg); }" % (ns, ns, n))
     if straight:
-        w("    template <class C> __device__ __forceinline__ static double pip(const C& c, const double (&x)[%d], "
-          "double (&g)[%d]) { return %s_pip(c, x, g); }" % (spec.nvars, spec.nvars, n))
-        w("    template <class C> __device__ __forceinline__ static double pip_e(const C& c, const double (&x)[%d]) "
-          "{ return %s_pip_e(c, x); }" % (spec.nvars, n))
-        w("    template <int S, class C> __device__ __forceinline__ static double pip_lock(const C& c, "
-          "const double* __restrict__ x, double* __restrict__ g) { return %s_pip_lock<S>(c, x, g); }" % n)
-        w("    template <int S, class C> __device__ __forceinline__ static double pip_e_lock(const C& c, "
-          "const double* __restrict__ x) { return %s_pip_e_lock<S>(c, x); }" % n)
+        w("    static constexpr int NPIECES = %d, NPIECES_E = %d;  // of the two tries" % (npieces, npieces))
         w("    template <int S, class C> __device__ __forceinline__ static double pip_piece(int k, const C& c, "
           "const double* __restrict__ x, double* __restrict__ g) { return %s_pip_piece<S>(k, c, x, g); }" % n)
         w("    template <int S, class C> __device__ __forceinline__ static double pip_e_piece(int k, const C& c, "
           "const double* __restrict__ x) { return %s_pip_e_piece<S>(k, c, x); }" % n)
-
     w("};")
 
 
@@ -647,8 +451,9 @@ def generate(name):
     only the units that include it."""
     spec = SPECS[name] if name in SPECS else ONEBODY_SPECS[name]
     table = load_pip(name)
-    straight = name in STRAIGHT_TYPES
-    trie = Trie(table) if straight else None
+    straight = name in SPECS
+    wt = wtable(name)
+    trie = Trie(wt) if straight else None
     leaves, inner = trie.counts() if straight else (table.nterms, 0)
     head = ["// Generated by mbx_b200/codegen/gen_kernels.py from mbx_b200/specs.py and",
             "// mbx_b200/data/%s.pip.gz -- do not edit." % name]
@@ -657,26 +462,17 @@ def generate(name):
                   "#define %s_STRAIGHT_LINE %d" % (name.upper(), 1 if straight else 0)]
     emit_vars(spec, out)
     nv = spec.nvars
+    nparts = parts_for(wt.nterms, nv) if straight else 0
+    npieces = len(split_terms(trie, nparts)) if straight else 0
+    out.append("// %d terms in the w variables" % wt.nterms)
+    emit_transforms(wt, name, out)
     if straight:
-        out += ["template <class Coef> __device__ __forceinline__ double %s_pip(const Coef&, const double (&)[%d], "
-                "double (&)[%d]);" % (name, nv, nv),
-                "template <class Coef> __device__ __forceinline__ double %s_pip_e(const Coef&, "
-                "const double (&)[%d]);" % (name, nv),
-                "template <int S, class Coef> __device__ __forceinline__ double %s_pip_lock(const Coef&, "
-                "const double* __restrict__, double* __restrict__);" % name,
-                "template <int S, class Coef> __device__ __forceinline__ double %s_pip_e_lock(const Coef&, "
-                "const double* __restrict__);" % name,
-                "template <int S, class Coef> __device__ __forceinline__ double %s_pip_piece(int, const Coef&, "
+        out += ["template <int S, class Coef> __device__ __forceinline__ double %s_pip_piece(int, const Coef&, "
                 "const double* __restrict__, double* __restrict__);" % name,
                 "template <int S, class Coef> __device__ __forceinline__ double %s_pip_e_piece(int, const Coef&, "
                 "const double* __restrict__);" % name]
         if name in SHIFT_TYPES:
             sp = shifted_pip(name)
-            if name not in QF_TYPES:
-                out.append("template <int S, class Coef> __device__ __forceinline__ double2 %s_pip_s32_lock("
-                           "const Coef&, const f2_t* __restrict__, f2_t* __restrict__);" % name)
-                out.append("template <int S, class Coef> __device__ __forceinline__ double2 %s_pip_s32_piece(int, "
-                           "const Coef&, const f2_t* __restrict__, f2_t* __restrict__);" % name)
             out.append("// dx = x - x0, the reference point of the FP32 basis (%s)" % SHIFT_TYPES[name])
             out.append("__device__ __forceinline__ void %s_shift(const double (&x)[%d], float (&xf)[%d]) {" %
                        (name, nv, nv))
@@ -686,46 +482,18 @@ def generate(name):
                 else:
                     out.append("    xf[%d] = (float)(x[%d] - %s);" % (v, v, lit(float(sp.x0[v]))))
             out.append("}")
-    emit_traits(spec, table, straight, out)
+    emit_traits(spec, table, straight, npieces, out)
     os.makedirs(OUT, exist_ok=True)
     write_if_changed(os.path.join(OUT, name + ".cuh"), "\n".join(out) + "\n")
     if straight:
-        nparts = parts_for(table.nterms, spec.nvars)
-        perms = None
-        if name in COSET_TYPES:
-            cf, ctab = coset_of(name)
-            trie = Trie(ctab)
-            perms = cf.perms
-            nparts = max(1, (ctab.nterms + COSET_PIECE_TERMS - 1) // COSET_PIECE_TERMS)
         for suffix, emitter, arg in (("pip", emit_pip, trie), ("pip_e", emit_pip_energy, trie)):
             body = head + ["#pragma once", '#include "%s.cuh"' % name]
-            if perms is not None:
-                body.append("// coset form: %d terms of R x %d permutations (%d terms in the table)" %
-                            (ctab.nterms, len(perms), table.nterms))
-            emitter(arg, nv, "%s_%s" % (name, suffix), body, nparts, perms=perms)
+            emitter(arg, nv, "%s_%s" % (name, suffix), body, nparts)
             write_if_changed(os.path.join(OUT, "%s_%s.cuh" % (name, suffix)), "\n".join(body) + "\n")
         if name in QF_TYPES:
             from mbx_b200.codegen import qf
             write_if_changed(os.path.join(OUT, "%s_qf.cuh" % name),
                              qf.emit_cuda(qf.QuadForm(name, shifted_pip(name)), name, nv))
-        elif name in SHIFT_TYPES:
-            from mbx_b200.codegen.shift import ShiftedTable
-            sp = shifted_pip(name)
-            body = head + ["#pragma once", '#include "%s.cuh"' % name,
-                           "// %d monomials of the %s basis, %d coefficient orbits" %
-                           (len(sp.monos), SHIFT_TYPES[name], sp.norb)]
-            if name in COSET_TYPES:
-                cfs, ctab_s = coset_of(name, shifted_basis=True)
-                body.append("// coset form: %d terms of R x %d permutations" % (ctab_s.nterms, len(cfs.perms)))
-                emit_pip_f32x2(Trie(ctab_s), nv, "%s_pip_s32" % name, body,
-                               max(1, (ctab_s.nterms + COSET_PIECE_TERMS - 1) // COSET_PIECE_TERMS), perms=cfs.perms)
-            else:
-                # ~400 terms per piece: larger pieces spill in the paired form
-                # (2048-water trimers, x/g in shared memory: 0.833/0.818/0.910 ms
-                # at 330/400/480 terms per piece)
-                strie = Trie(ShiftedTable(sp, name))
-                emit_pip_f32x2(strie, nv, "%s_pip_s32" % name, body, max(1, (len(sp.monos) + 399) // 400))
-            write_if_changed(os.path.join(OUT, "%s_pip_s32.cuh" % name), "\n".join(body) + "\n")
     return os.path.join(OUT, name + ".cuh"), leaves, inner
 
 
@@ -737,48 +505,31 @@ TU_HEAD = """// Generated by mbx_b200/codegen/gen_kernels.py -- do not edit.
 #include "../launch_cache.cuh"
 #include "%(name)s.cuh"
 %(include)s
-static __constant__ double c_%(name)s[%(ncoef)d];
-static __constant__ float cf_%(name)s[%(ncoef)d];
+static __constant__ double c_%(name)s[%(ncw)d];
 struct %(name)s_CC {
     __device__ __forceinline__ double operator[](int k) const { return c_%(name)s[k]; }
-    __device__ __forceinline__ float f(int k) const { return cf_%(name)s[k]; }
 };
 
-%(scale_decl)s
-int mbx_set_coef_%(name)s_%(v)s(const double* a, int from_device, cudaStream_t s) {
-    cudaError_t e = cudaSuccess;
-    std::vector<double> h(%(ncoef)d);
-    if (from_device) {
-        e = cudaMemcpyAsync(h.data(), a, sizeof(double) * %(ncoef)d, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return (int)e;
-    } else {
-        for (int k = 0; k < %(ncoef)d; ++k) h[k] = a[k];
-    }
-%(scale_apply)s    e = cudaMemcpyToSymbolAsync(c_%(name)s, h.data(), sizeof(double) * %(ncoef)d, 0, cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return (int)e;
-    // FP32 copy for the mixed-precision leaf sums (a warp-uniform FFMA operand)
-    std::vector<float> f(%(ncoef)d);
-    for (int k = 0; k < %(ncoef)d; ++k) f[k] = (float)h[k];
-    e = cudaMemcpyToSymbolAsync(cf_%(name)s, f.data(), sizeof(float) * %(ncoef)d, 0, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    return (int)e;
+// the coefficients in the w variables (%(ncw)d doubles, on the host or the device)
+int mbx_set_coef_%(name)s_%(v)s(const double* c, int from_device, cudaStream_t s) {
+    return (int)cudaMemcpyToSymbolAsync(c_%(name)s, c, sizeof(double) * %(ncw)d, 0,
+                                        from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s);
 }
 """
 
 LOCK_LAUNCH = """
 int mbx_launch_%(name)s_%(v)s(const HolderArgs& A, int grid, int block, cudaStream_t s) {
     // persistent grid of lockstep blocks: every resident block slot once
-    // (blocks claim chunks of LOCK_THREADS n-mers dynamically); the
+    // (blocks claim units of LOCK_THREADS n-mers dynamically, LockPlan); the
     // variables%(gtext)s of the block's n-mers in dynamic shared memory
-    auto kern = holder_lock_kernel<%(name)s_T, %(name)s_CC, %(mode)s, false>;
+    auto kern = holder_lock_kernel<%(name)s_T, %(name)s_CC, %(mode)s>;
     block = %(name)s_T::LOCK_THREADS;
     const int smem = %(ncol)d * %(name)s_T::NVARS * %(name)s_T::LOCK_THREADS * (int)sizeof(double);
     static LaunchCache lc;
     int sms = 0, bps = 0;
     const int r = launch_facts(lc, kern, block, smem, smem, &sms, &bps);
     if (r) return r;
-    const long need = (A.n + block - 1) / block;
+    const long need = (A.n + block - 1) / block * (A.split ? %(name)s_T::%(npieces)s : 1);
     grid = (int)(need < (long)sms * bps ? need : (long)sms * bps);
     if (grid < 1) grid = 1;
     kern<<<grid, block, smem, s>>>(A);
@@ -789,7 +540,7 @@ int mbx_prime_%(name)s_%(v)s(cudaStream_t s) {
     // code prefetch of the %(what2)s: a launch of the evaluation kernel itself in its
     // prefetch mode (prime_pieces), one warp per SM, every piece run by at
     // least four of them
-    auto kern = holder_lock_kernel<%(name)s_T, %(name)s_CC, %(mode)s, false>;
+    auto kern = holder_lock_kernel<%(name)s_T, %(name)s_CC, %(mode)s>;
     const int smem_full = %(ncol)d * %(name)s_T::NVARS * %(name)s_T::LOCK_THREADS * (int)sizeof(double);
     const int smem = %(name)s_T::NVARS * %(name)s_T::LOCK_THREADS * (int)sizeof(double);
     static LaunchCache lc;
@@ -798,7 +549,7 @@ int mbx_prime_%(name)s_%(v)s(cudaStream_t s) {
     if (r) return r;
     HolderArgs A;
     memset(&A, 0, sizeof(A));
-    A.prime_npieces = %(name)s_%(pipname)s_NPIECES;
+    A.prime_npieces = %(name)s_T::%(npieces)s;
     A.prime_passes = (4 * A.prime_npieces + sms - 1) / sms;
     kern<<<sms, 32, smem, s>>>(A);
     return (int)cudaGetLastError();
@@ -809,58 +560,24 @@ VARIANTS = {
     # variant: (description, body)
     "g": ("FP64 energy + gradient kernel", LOCK_LAUNCH % {
         "name": "%(name)s", "v": "g", "gtext": " and their gradient accumulators", "mode": "HM_GRAD_FP64",
-        "ncol": 2, "what2": "FP64 gradient trie", "pipname": "pip"}),
+        "ncol": 2, "what2": "FP64 gradient trie", "npieces": "NPIECES"}),
     "e": ("FP64 energy-only kernel", LOCK_LAUNCH % {
         "name": "%(name)s", "v": "e", "gtext": "", "mode": "HM_ENERGY",
-        "ncol": 1, "what2": "FP64 energy trie", "pipname": "pip_e"}),
+        "ncol": 1, "what2": "FP64 energy trie", "npieces": "NPIECES_E"}),
 }
 
-# The table unit of every evaluator: the coefficient adjoint and, for the
-# evaluators without straight-line code, the table-driven evaluation, both
-# reading the polynomial's term table (csrc/term_table.cuh) and its
-# coefficients from global memory.
+# The adjoint unit of every evaluator: the variables of its n-mers for the
+# coefficient adjoint (csrc/table_kernels.cu does the rest from the tables).
 TABLE_TU = """// Generated by mbx_b200/codegen/gen_kernels.py -- do not edit.
-// Table-driven kernels (term table in global memory) of the %(name)s evaluator.
-#include <cstring>
+// Variables of the %(name)s evaluator for the coefficient adjoint.
 #include "../holder_kernel.cuh"
-#include "../launch_cache.cuh"
 #include "%(name)s.cuh"
 
-int mbx_launch_%(name)s_c(const HolderArgs& A, const double* w, double* out, int grid, int block, cudaStream_t s) {
-    // coefficient adjoint: dynamic shared memory = per-coefficient sums +
-    // the variable columns of the block's four warps
-    auto kern = holder_dcoef_table_kernel<%(name)s_T>;
-    const int smem = (%(name)s_T::NCOEF + 4 * 32 * %(name)s_T::NVARS) * (int)sizeof(double);
-    static LaunchCache lc;
-    int sms = 0, bps = 0;
-    const int r = launch_facts(lc, kern, 0, smem, 0, &sms, &bps);
-    if (r) return r;
-    kern<<<grid, 128, smem, s>>>(A, w, out);
-    return (int)cudaGetLastError();
-}
-%(warp)s"""
-
-TABLE_WARP = """
-int mbx_launch_%(name)s_w(const HolderArgs& A, int grads, int grid, cudaStream_t s) {
-    if (%(name)s_T::NTERMS > 100000) {
-        // very large table, few n-mers: a warp per n-mer
-        holder_table_kernel<%(name)s_T, 4><<<grid, 128, 0, s>>>(A, grads);
-        return (int)cudaGetLastError();
-    }
-    // a lane per n-mer; x and gradient columns of four warps in dynamic shared memory
-    auto kern = holder_table_lane_kernel<%(name)s_T>;
-    const int smem = 4 * 2 * %(name)s_T::NVARS * 32 * (int)sizeof(double);
-    static LaunchCache lc;
-    int sms = 0, bps = 0;
-    const int r = launch_facts(lc, kern, 128, smem, smem, &sms, &bps);
-    if (r) return r;
-    const long need = (A.n + 127) / 128;
-    const int g = (int)(need < (long)sms * bps ? (need > 0 ? need : 1) : (long)sms * bps);
-    kern<<<g, 128, smem, s>>>(A, grads);
+int mbx_launch_%(name)s_c(const HolderArgs& A, const double* w, long first, int count, double* wv, cudaStream_t s) {
+    holder_wvars_kernel<%(name)s_T><<<(count + 127) / 128, 128, 0, s>>>(A, w, first, count, wv);
     return (int)cudaGetLastError();
 }
 """
-
 
 ONEBODY_TU = """// Generated by mbx_b200/codegen/gen_kernels.py -- do not edit.
 // Table-driven 1-body kernel of the %(name)s evaluator.
@@ -886,130 +603,19 @@ int mbx_launch_%(name)s_o(const HolderArgs& A, int grid, int block, cudaStream_t
 """
 
 
-# Evaluators with straight-line (generated Horner trie) kernels: the water
-# and methane-water polynomials of MB-pol / MB-nrg the timed path runs.  All
-# others run the table-driven kernels: their tries would add minutes of
-# compile time each for types no timed workload uses.
-STRAIGHT_TYPES = ("mbpol2b", "mbpol3b", "ch4h2o2b", "ch4h2o3b")
-
-
 def variants_of(name):
     from mbx_b200.specs import KERNEL_ALIASES
     if name in ONEBODY_SPECS:
         return "o"
     name = KERNEL_ALIASES.get(name, name)
-    if name in STRAIGHT_TYPES:
-        return "ge" + ("s" if name in SHIFT_TYPES else "") + "t"
-    return "wt"
-
-
-SHIFT_TU = """// Generated by mbx_b200/codegen/gen_kernels.py -- do not edit.
-// Paired FP32 (%(basis)s basis) energy + gradient kernel for the %(name)s evaluator.
-#include <cstring>
-#include <vector>
-#include "../holder_kernel.cuh"
-#include "../launch_cache.cuh"
-#include "%(name)s.cuh"
-#include "%(name)s_pip_s32.cuh"
-
-// one coefficient per monomial orbit of the basis, as an FP32 pair (c, c)
-// for the paired instructions
-static __constant__ f2_t cs_%(name)s[%(norb)d];
-static __constant__ double cs0_%(name)s[1];        // constant term (FP64)
-struct %(name)s_CS {
-    __device__ __forceinline__ f2_t f2(int k) const { return cs_%(name)s[k]; }
-    __device__ __forceinline__ double b0() const { return cs0_%(name)s[0]; }
-};
-
-// b = F a: the basis coefficients are linear in the fitted ones.  Row j of F
-// (entries sF_row[j] .. sF_row[j+1]) lists (k, factor); sF0 is the constant.
-static const int sF_row_%(name)s[%(norb1)d] = {%(rows)s};
-static const int sF_k_%(name)s[%(nnz)d] = {%(ks)s};
-static const double sF_f_%(name)s[%(nnz)d] = {%(fs)s};
-static const int sF0_k_%(name)s[%(nnz0)d] = {%(k0)s};
-static const double sF0_f_%(name)s[%(nnz0)d] = {%(f0)s};
-// per-orbit factor of the kernel's coefficients (1, or the coset-form scale)
-static const double sscale_%(name)s[%(norb)d] = {%(sscale)s};
-
-int mbx_set_coef_%(name)s_s(const double* a, int from_device, cudaStream_t s) {
-    std::vector<double> h(%(ncoef)d);
-    cudaError_t e = cudaSuccess;
-    if (from_device) {
-        e = cudaMemcpyAsync(h.data(), a, sizeof(double) * %(ncoef)d, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return (int)e;
-    } else {
-        for (int k = 0; k < %(ncoef)d; ++k) h[k] = a[k];
-    }
-    std::vector<unsigned long long> b(%(norb)d);
-    for (int j = 0; j < %(norb)d; ++j) {
-        double acc = 0.0;
-        for (int q = sF_row_%(name)s[j]; q < sF_row_%(name)s[j + 1]; ++q) acc += sF_f_%(name)s[q] * h[sF_k_%(name)s[q]];
-        const float f = (float)(acc * sscale_%(name)s[j]);
-        unsigned int u;
-        memcpy(&u, &f, sizeof(u));
-        b[j] = (unsigned long long)u | ((unsigned long long)u << 32);
-    }
-    double b0 = 0.0;
-    for (int q = 0; q < %(nnz0)d; ++q) b0 += sF0_f_%(name)s[q] * h[sF0_k_%(name)s[q]];
-    e = cudaMemcpyToSymbolAsync(cs_%(name)s, b.data(), sizeof(unsigned long long) * %(norb)d, 0,
-                                cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyToSymbolAsync(cs0_%(name)s, &b0, sizeof(double), 0, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    return (int)e;
-}
-
-int mbx_launch_%(name)s_s(const HolderArgs& A, int grid, int block, cudaStream_t s) {
-    // three kernels (holder_kernel.cuh): the FP64 variables at full
-    // occupancy, the paired FP32 trie in a persistent grid of lockstep blocks
-    // (two n-mers per thread, every resident block slot once, the paired
-    // variables and gradient accumulators of the block in dynamic shared
-    // memory), the FP64 chain rule and sums at full occupancy; A.ps holds the
-    // scratch between them (capacity A.ps.cap >= A.n)
-    if (!A.ps.dx || !A.ps.q || A.ps.cap < A.n) return (int)cudaErrorInvalidValue;
-    auto kern = pair_trie_kernel<%(name)s_T, %(name)s_CS>;
-    block = %(name)s_T::LOCK_THREADS_S;
-    const int smem = 2 * %(name)s_T::NVARS * %(name)s_T::LOCK_THREADS_S * (int)sizeof(f2_t);
-    static LaunchCache lc;
-    int sms = 0, bps = 0;
-    const int r = launch_facts(lc, kern, block, smem, smem, &sms, &bps);
-    if (r) return r;
-    const long wide = (long)sms * 16;
-    const long gv = (A.n + 255) / 256, gf = (A.n + 127) / 128;
-    pair_vars_kernel<%(name)s_T><<<(int)(gv < wide ? (gv > 0 ? gv : 1) : wide), 256, 0, s>>>(A);
-    const long need = (A.n + 2 * block - 1) / (2 * block);
-    grid = (int)(need < (long)sms * bps ? need : (long)sms * bps);
-    if (grid < 1) grid = 1;
-    kern<<<grid, block, smem, s>>>(A);
-    pair_finish_kernel<%(name)s_T><<<(int)(gf < wide ? (gf > 0 ? gf : 1) : wide), 128, 0, s>>>(A);
-    return (int)cudaGetLastError();
-}
-
-int mbx_prime_%(name)s_s(cudaStream_t s) {
-    // code prefetch of the paired FP32 trie: a launch of the evaluation kernel itself in its
-    // prefetch mode (prime_pieces), one warp per SM, every piece run by at
-    // least four of them
-    auto kern = pair_trie_kernel<%(name)s_T, %(name)s_CS>;
-    const int smem_full = 2 * %(name)s_T::NVARS * %(name)s_T::LOCK_THREADS_S * (int)sizeof(f2_t);
-    const int smem = %(name)s_T::NVARS * %(name)s_T::LOCK_THREADS_S * (int)sizeof(f2_t);
-    static LaunchCache lc;
-    int sms = 0, bps = 0;
-    const int r = launch_facts(lc, kern, 0, smem_full, 0, &sms, &bps);
-    if (r) return r;
-    HolderArgs A;
-    memset(&A, 0, sizeof(A));
-    A.prime_npieces = %(name)s_pip_s32_NPIECES;
-    A.prime_passes = (4 * A.prime_npieces + sms - 1) / sms;
-    kern<<<sms, 32, smem, s>>>(A);
-    return (int)cudaGetLastError();
-}
-"""
+    return "ge" + ("s" if name in SHIFT_TYPES else "") + "t"
 
 
 QF_TU = """// Generated by mbx_b200/codegen/gen_kernels.py -- do not edit.
 // Mixed-precision evaluation of the %(name)s polynomial on the tensor cores
 // (quadratic form over the %(basis)s FP32 basis, csrc/qf_kernel.cuh).
+#include <cuda_fp16.h>
+
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -1026,6 +632,13 @@ static const double sF_f_%(name)s[%(nnz)d] = {%(fs)s};
 static const int sF0_k_%(name)s[%(nnz0)d] = {%(k0)s};
 static const double sF0_f_%(name)s[%(nnz0)d] = {%(f0)s};
 %(tables)s
+// the same for the device
+static __device__ const int dF_row_%(name)s[%(norb1)d] = {%(rows)s};
+static __device__ const int dF_k_%(name)s[%(nnz)d] = {%(ks)s};
+static __device__ const double dF_f_%(name)s[%(nnz)d] = {%(fs)s};
+static __device__ const int dF0_k_%(name)s[%(nnz0)d] = {%(k0)s};
+static __device__ const double dF0_f_%(name)s[%(nnz0)d] = {%(f0)s};
+%(dtables)s
 // IEEE binary16 of x, rounded to nearest even (subnormals kept; |x| < 65504 here)
 static unsigned short qf_half(double x) {
     const unsigned short sign = std::signbit(x) ? 0x8000 : 0;
@@ -1117,26 +730,103 @@ int mbx_qf_image_%(name)s(const double* a, unsigned char* img, float* colf, doub
     return 0;
 }
 
-int mbx_set_coef_%(name)s_s(const double* a, int from_device, cudaStream_t s) {
-    std::vector<double> h(%(ncoef)d);
-    cudaError_t e = cudaSuccess;
-    if (from_device) {
-        e = cudaMemcpyAsync(h.data(), a, sizeof(double) * %(ncoef)d, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return (int)e;
-    } else {
-        for (int k = 0; k < %(ncoef)d; ++k) h[k] = a[k];
+// The same on the device (mbx_set_coefficients): the steps of the host
+// builder above, operation for operation (every product and sum rounded on
+// its own), so that both write the same bytes.
+static __device__ double qfd_a_%(name)s[%(ncoef)d], qfd_b_%(name)s[%(norb)d];
+static __device__ double qfd_C_%(name)s[%(name)s_Q::NB * %(name)s_Q::NB];
+static __device__ int qfd_sj_%(name)s[%(name)s_Q::NB];
+static __device__ float qfd_colf_%(name)s[%(name)s_Q::NB];   // to constant memory by a copy
+static __device__ double qfd_b0_%(name)s[1];
+
+// a warp per row; the terms of a row are added in order, as on the host
+__global__ void k_qf_b_%(name)s() {
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (j > %(norb)d) return;
+    const bool c0 = j == %(norb)d;   // the constant term
+    const int b = c0 ? 0 : dF_row_%(name)s[j], e = c0 ? %(nnz0)d : dF_row_%(name)s[j + 1];
+    double acc = 0.0;
+    for (int q0 = b; q0 < e; q0 += 32) {
+        const int q = q0 + lane;
+        double p = 0.0;
+        if (q < e)
+            p = c0 ? __dmul_rn(dF0_f_%(name)s[q], qfd_a_%(name)s[dF0_k_%(name)s[q]])
+                   : __dmul_rn(dF_f_%(name)s[q], qfd_a_%(name)s[dF_k_%(name)s[q]]);
+        for (int i = 0; i < 32 && q0 + i < e; ++i) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, p, i));
     }
-    std::vector<unsigned char> img((size_t)%(name)s_Q::IMAGE_BYTES);
-    std::vector<float> colf(%(name)s_Q::NB);
-    double b0 = 0.0;
-    mbx_qf_image_%(name)s(h.data(), img.data(), colf.data(), &b0);
-    e = cudaMemcpyToSymbolAsync(qf_img_%(name)s, img.data(), img.size(), 0, cudaMemcpyHostToDevice, s);
+    if (lane == 0) (c0 ? qfd_b0_%(name)s[0] : qfd_b_%(name)s[j]) = acc;
+}
+
+// C' = D C D from zeroed C: every monomial has an entry (i, j) of its own
+__global__ void k_qf_c_%(name)s() {
+    constexpr int NB = %(name)s_Q::NB;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= dqf_nmono_%(name)s) return;
+    const int i = dqf_mi_%(name)s[q], j = dqf_mj_%(name)s[q];
+    const double c = qfd_b_%(name)s[dqf_mo_%(name)s[q]];
+    const int t = dqf_t_%(name)s[i] + dqf_t_%(name)s[j];
+    const double v = ldexp(i == j ? c : 0.5 * c, t);
+    qfd_C_%(name)s[i * NB + j] = v;
+    qfd_C_%(name)s[j * NB + i] = v;
+}
+
+// column exponents and factors: a warp per column
+__global__ void k_qf_cols_%(name)s() {
+    constexpr int NB = %(name)s_Q::NB;
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (j >= NB) return;
+    double m = 0.0;
+    for (int i = lane; i < NB; i += 32) m = fmax(m, fabs(qfd_C_%(name)s[i * NB + j]));
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane) return;
+    int sj = 0;
+    if (m > 0.0) {
+        int e;
+        frexp(m, &e);
+        sj = 14 - e;
+    }
+    qfd_sj_%(name)s[j] = sj;
+    qfd_colf_%(name)s[j] = (float)ldexp(1.0, -(sj + dqf_t_%(name)s[j]));
+}
+
+// the image: a thread per (K block, column, k)
+__global__ void k_qf_image_%(name)s() {
+    constexpr int NB = %(name)s_Q::NB;
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= %(name)s_Q::KS * NB * 16) return;
+    const int kk = idx %% 16, n = idx / 16 %% NB, s = idx / (16 * NB);
+    int p = 0;
+    while (p + 1 < %(name)s_Q::NPASS && n >= %(name)s_Q::pass_col(p + 1)) ++p;
+    const int width = %(name)s_Q::pass_n(p), nn = n - %(name)s_Q::pass_col(p);
+    double x = ldexp(qfd_C_%(name)s[(16 * s + kk) * NB + n], qfd_sj_%(name)s[n]);
+    unsigned char* st = qf_img_%(name)s + %(name)s_Q::chunk_offset(s, p);
+    const size_t off = (size_t)(nn / 8) * 128 + (size_t)(kk / 8) * (width / 8) * 128 + (nn %% 8) * 16 + (kk %% 8) * 2;
+    const int parts = %(name)s_Q::parts(s);
+    for (int pt = 0; pt < parts; ++pt) {
+        const __half h = __double2half(x);
+        *reinterpret_cast<__half*>(st + (size_t)pt * width * 32 + off) = h;
+        x -= (double)__half2float(h);
+    }
+}
+
+int mbx_set_coef_%(name)s_s(const double* a, int from_device, cudaStream_t s) {
+    cudaError_t e = cudaMemcpyToSymbolAsync(qfd_a_%(name)s, a, sizeof(double) * %(ncoef)d, 0,
+                                            from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s);
+    void *C = nullptr, *colf = nullptr, *b0 = nullptr;
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&C, qfd_C_%(name)s);
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&colf, qfd_colf_%(name)s);
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&b0, qfd_b0_%(name)s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(C, 0, sizeof(qfd_C_%(name)s), s);
+    if (e != cudaSuccess) return (int)e;
+    constexpr int NB = %(name)s_Q::NB;
+    k_qf_b_%(name)s<<<((%(norb)d + 1) * 32 + 127) / 128, 128, 0, s>>>();
+    k_qf_c_%(name)s<<<(qf_nmono_%(name)s + 127) / 128, 128, 0, s>>>();
+    k_qf_cols_%(name)s<<<(NB * 32 + 127) / 128, 128, 0, s>>>();
+    k_qf_image_%(name)s<<<(%(name)s_Q::KS * NB * 16 + 127) / 128, 128, 0, s>>>();
+    e = cudaGetLastError();
     if (e == cudaSuccess)
-        e = cudaMemcpyToSymbolAsync(qf_colf_%(name)s, colf.data(), sizeof(float) * colf.size(), 0,
-                                    cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(qf_b0_%(name)s, &b0, sizeof(double), 0, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        e = cudaMemcpyToSymbolAsync(qf_colf_%(name)s, colf, sizeof(float) * NB, 0, cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(qf_b0_%(name)s, b0, sizeof(double), 0, cudaMemcpyDeviceToDevice, s);
     return (int)e;
 }
 
@@ -1186,28 +876,9 @@ def write_qf_tu(name, path):
          "fs": ",".join(repr(float(f)) for f in fs),
          "k0": ",".join(map(str, k0)) if k0 else "0",
          "f0": ",".join(repr(float(sp.const_F[k])) for k in k0) if k0 else "0.0",
-         "tables": qf.emit_host_tables(q, name)}
+         "tables": qf.emit_tables(q, name, "static const", "qf"),
+         "dtables": qf.emit_tables(q, name, "static __device__ const", "dqf")}
     write_tu(path, QF_TU % d)
-
-
-def write_shift_tu(name, path):
-    sp = shifted_pip(name)
-    rows, ks, fs = [0], [], []
-    for row in sp.F:
-        for k, f in sorted(row.items()):
-            ks.append(k)
-            fs.append(f)
-        rows.append(len(ks))
-    k0 = sorted(sp.const_F)
-    d = {"name": name, "NAME": name.upper(), "basis": SHIFT_TYPES[name], "norb": sp.norb, "norb1": sp.norb + 1,
-         "ncoef": SPECS[name].ncoef, "nnz": len(ks), "nnz0": max(1, len(k0)),
-         "rows": ",".join(map(str, rows)), "ks": ",".join(map(str, ks)),
-         "fs": ",".join(repr(float(f)) for f in fs),
-         "k0": ",".join(map(str, k0)) if k0 else "0",
-         "sscale": ",".join(repr(float(x)) for x in (coset_of(name, True)[0].scale if name in COSET_TYPES
-                                                       else np.ones(sp.norb))),
-         "f0": ",".join(repr(float(sp.const_F[k])) for k in k0) if k0 else "0.0"}
-    write_tu(path, SHIFT_TU % d)
 
 
 def write_tu(path, text):
@@ -1226,30 +897,19 @@ def write_kernels_cu(name):
         return [path]
     spec = SPECS[name]
     for v in variants_of(name):
-        if v == "w":
-            continue   # part of the table unit
         if v == "s":
             path = os.path.join(OUT, "%s_s.cu" % name)
-            if name in QF_TYPES:
-                write_qf_tu(name, path)
-            else:
-                write_shift_tu(name, path)
+            write_qf_tu(name, path)
             paths.append(path)
             continue
         path = os.path.join(OUT, "%s_%s.cu" % (name, v))
         if v == "t":
-            d = {"name": name, "warp": TABLE_WARP % {"name": name} if "w" in variants_of(name) else ""}
-            write_tu(path, TABLE_TU % d)
+            write_tu(path, TABLE_TU % {"name": name})
         else:
             what, body = VARIANTS[v]
-            d = {"name": name, "NAME": name.upper(), "ncoef": spec.ncoef, "v": v, "what": what,
-                 "include": '#include "%s_%s.cuh"\n' % (name, inc[v]), "scale_decl": "", "scale_apply": ""}
-            if name in COSET_TYPES:
-                cf, _ = coset_of(name)
-                d["scale_decl"] = ("// coset form: the kernels take a_k * scale_k (codegen/coset.py)\n"
-                                   "static const double coset_scale_%s[%d] = {%s};\n" %
-                                   (name, spec.ncoef, ", ".join(repr(float(x)) for x in cf.scale)))
-                d["scale_apply"] = "    for (int k = 0; k < %d; ++k) h[k] *= coset_scale_%s[k];\n" % (spec.ncoef, name)
+            wt = wtable(name)
+            d = {"name": name, "NAME": name.upper(), "ncw": wt.ncoef, "v": v, "what": what,
+                 "include": '#include "%s_%s.cuh"\n' % (name, inc[v])}
             write_tu(path, (TU_HEAD + body) % d)
         paths.append(path)
     return paths
@@ -1268,37 +928,50 @@ def term_runs(vars_):
 
 @__import__("functools").lru_cache(maxsize=None)
 def _table_runs(table_name):
-    t = load_pip(table_name)
+    t = wtable_by_key(table_name)
     return [term_runs(t.var[q, :t.deg[q]].tolist()) for q in range(t.nterms)]
 
 
-def term_pairs_max(table):
-    return max(1, max(len(r) for r in _table_runs(table.name)))
+def term_pairs_max(table_name):
+    return max(1, max(len(r) for r in _table_runs(table_name)))
 
 
 def table_names():
-    """Term tables in registry order (an evaluator sharing another's table
-    refers to the same entry), then the 1-body evaluators' tables."""
+    """Keys of the term tables in registry order (evaluators with the same
+    key share an entry), the plain tables of the evaluators with a reference
+    point (for caller-supplied variables), the 1-body evaluators' last."""
     from mbx_b200.specs import KERNEL_ALIASES
     names = []
-    for n in SPECS:
-        t = SPECS[KERNEL_ALIASES.get(n, n)].pip_table
-        if t not in names:
-            names.append(t)
-    for n, sp in ONEBODY_SPECS.items():
-        if sp.pip_table not in names:
-            names.append(sp.pip_table)
+    kern = [KERNEL_ALIASES.get(n, n) for n in SPECS]
+    for key in [table_key(n) for n in kern] + [SPECS[n].pip_table for n in kern] + \
+            [table_key(n) for n in ONEBODY_SPECS]:
+        if key not in names:
+            names.append(key)
     return names
 
 
 def write_term_tables():
-    """Every evaluator's term table (csrc/term_table.cuh encoding) in one
-    binary file, embedded in the library by terms_blob.cpp (.incbin), plus the
-    index of the tables."""
+    """Every polynomial's term table in the w variables (csrc/term_table.cuh
+    encoding), its coefficient map c = F a and its transform w = W x, in one
+    binary file, embedded in the library by terms_blob.cpp (.incbin), plus
+    the index of the tables."""
     blob = bytearray()
     index = []
+
+    def put(array):
+        off = len(blob)
+        blob.extend(array.tobytes())
+        blob.extend(b"\0" * (-len(blob) % 16))
+        return off
+
+    def csr(rows):
+        """(row starts, columns, factors) of rows {column: factor}"""
+        start = np.cumsum([0] + [len(r) for r in rows]).astype(np.int32)
+        return (start, np.array([k for r in rows for k in r], np.int32),
+                np.array([f for r in rows for f in r.values()], np.float64))
+
     for tname in table_names():
-        t = load_pip(tname)
+        t = wtable_by_key(tname)
         runs = _table_runs(tname)
         words = np.zeros((t.nterms, 4), np.int32)
         words[:, 0] = t.k
@@ -1313,25 +986,50 @@ def write_term_tables():
                 packed[i >> 1] |= ((v & 255) | (e << 8)) << (16 * (i & 1))
             for j in range(3):
                 words[q, 1 + j] = packed[j] - (1 << 32) if packed[j] >= 1 << 31 else packed[j]
-        off_terms = len(blob)
-        blob += words.tobytes()
-        off_coef = len(blob)
-        blob += np.ascontiguousarray(t.coef, np.float64).tobytes()
-        pad = (-len(blob)) % 16
-        blob += b"\0" * pad
-        index.append((tname, off_terms, off_coef, t.nterms, term_pairs_max(t)))
+        offs = [put(words), put(np.ascontiguousarray(t.coef, np.float64))]
+        fr, fk, ff = csr(t.F)
+        offs += [put(fr), put(fk), put(ff)]
+        for M in (t.W, t.W.T):
+            wr, wk, wf = csr([{v: M[i, v] for v in range(t.nvars) if M[i, v] != 0.0} for i in range(t.nvars)])
+            # column v with sign s as s (v + 1)
+            offs += [put(wr), put(((wk + 1) * wf).astype(np.int32))]
+        offs.append(put(np.ascontiguousarray(t.w0, np.float64)))
+        # half-monomials of the coefficient adjoint: up to three (variable,
+        # exponent) byte pairs each (255: unused), and per term its two of them
+        basis, pairs = t.halves
+        half = np.zeros((len(basis), 2), np.int32)
+        for i, m in enumerate(basis):
+            rr = term_runs(list(m))
+            if len(rr) > 3:
+                raise ValueError("%s: half-monomial %s has more than three distinct variables" % (tname, m))
+            rr = rr + [(255, 0)] * (3 - len(rr))
+            half[i] = [sum(v << (8 * n) for n, (v, _) in enumerate(rr)), sum(e << (8 * n) for n, (_, e) in enumerate(rr))]
+        offs += [put(half), put(np.array([i | (j << 16) for i, j in pairs], np.int32))]
+        # F transposed, over the terms: fitted coefficient k takes sign * F_jk
+        # of every term of orbit j
+        by_k = [{} for _ in range(max((k for r in t.F for k in r), default=0) + 1)]
+        for q in range(t.nterms):
+            for k, f in t.F[int(t.k[q])].items():
+                by_k[k][q] = f * float(t.coef[q])
+        offs += [put(a) for a in csr(by_k + [{}] * (t.nfit - len(by_k)))]
+        index.append((tname, t.nterms, term_pairs_max(tname), t.ncoef, len(basis), offs))
     bin_path = os.path.join(OUT, "terms.bin")
     old = open(bin_path, "rb").read() if os.path.exists(bin_path) else None
     if old != bytes(blob):
         with open(bin_path, "wb") as f:
             f.write(bytes(blob))
     lines = ["// Generated by mbx_b200/codegen/gen_kernels.py -- do not edit.", "#pragma once",
-             "// term tables in terms.bin: (name, byte offset of the int4 terms, of the",
-             "// double multiplicities, number of terms, (variable, exponent) pairs per term at most)",
-             "struct TermTableInfo { const char* name; long off_terms, off_tcoef, nterms; int pairs; };",
+             "// term tables in terms.bin: name, number of terms, (variable, exponent) pairs per",
+             "// term at most, coefficients in the w variables; byte offsets of the int4 terms, the",
+             "// double signs, the rows of F (starts, columns, factors), of W and of its transpose",
+             "// (starts, signed columns), of w0, of the half-monomials, of the terms' pairs of them and of the",
+             "// terms of every fitted coefficient (starts, terms, factors)",
+             "struct TermTableInfo { const char* name; long nterms; int pairs, ncw, nhalf; long off_terms, off_tcoef, "
+             "off_frow, off_fk, off_ff, off_wrow, off_w, off_wtrow, off_wt, off_w0, off_half, off_pair, "
+             "off_ftrow, off_ftk, off_ftf; };",
              "static const TermTableInfo mbx_term_tables[] = {"]
-    for tname, ot, oc, nt, npair in index:
-        lines.append('    {"%s", %d, %d, %d, %d},' % (tname, ot, oc, nt, npair))
+    for tname, nt, npair, ncw, nhalf, offs in index:
+        lines.append('    {"%s", %d, %d, %d, %d, %s},' % (tname, nt, npair, ncw, nhalf, ", ".join(map(str, offs))))
     lines.append("};")
     lines.append("static const int mbx_num_term_tables = %d;" % len(index))
     lines.append("static const long mbx_terms_bytes = %d;" % len(blob))
@@ -1397,19 +1095,15 @@ def write_registry():
         vs = variants_of(name)
         if name in KERNEL_ALIASES:
             vs = ""   # runs the kernels of KERNEL_ALIASES[name], declared there
-        for v in "gesw":
-            if v not in vs:
-                continue
-            if v in "ges":
+        for v in "ges":
+            if v in vs:
                 lines.append("int mbx_launch_%s_%s(const HolderArgs& A, int grid, int block, cudaStream_t s);" %
                              (name, v))
                 lines.append("int mbx_prime_%s_%s(cudaStream_t s);" % (name, v))
                 lines.append("int mbx_set_coef_%s_%s(const double* a, int from_device, cudaStream_t s);" % (name, v))
-            else:
-                lines.append("int mbx_launch_%s_w(const HolderArgs& A, int grads, int grid, cudaStream_t s);" % name)
         if "t" in vs:
-            lines.append("int mbx_launch_%s_c(const HolderArgs& A, const double* w, double* out, int grid, "
-                         "int block, cudaStream_t s);" % name)
+            lines.append("int mbx_launch_%s_c(const HolderArgs& A, const double* w, long first, int count, double* wv, "
+                         "cudaStream_t s);" % name)
         fit = load_fit(name)
         lines.append("static const double mbx_fit_%s[%d] = {" % (name, len(fit)))
         for i in range(0, len(fit), 4):
@@ -1429,14 +1123,14 @@ def write_registry():
             # the table unit ("t") holds the coefficient adjoint ("c")
             have = ("t" in vs) if v == "c" else (v in vs)
             return ("mbx_%s_%s_%s" % (kind, kern, v)) if have else "nullptr"
-        lines.append('    {"%s", %d, {"%s", "%s", "%s"}, %s, %d, %d, %d, %d, mbx_fit_%s, %s, %s, %s, %s, %s, %s,' %
+        lines.append('    {"%s", %d, {"%s", "%s", "%s"}, %s, %d, %d, %d, %d, mbx_fit_%s, %s, %s, %s, %s, %s,' %
                      (name, spec.nbody, ids[0], ids[1], ids[2], lit(spec.rf), skip, spec.ncoef, spec.nreal,
                       spec.nvars, name, fn("g", "launch"), fn("e", "launch"), fn("c", "launch"),
-                      fn("w", "launch"), fn("s", "launch"), lit(MIXED_FP64_RADIUS.get(name, 0.0))))
+                      fn("s", "launch"), lit(MIXED_FP64_RADIUS.get(name, 0.0))))
         lines.append("     %s, %s, %s," % (fn("g", "prime"), fn("e", "prime"), fn("s", "prime")))
-        lines.append("     {%s, nullptr, nullptr, nullptr, nullptr}, %d, %d}," %
-                     (", ".join(fn(v, "set_coef") for v in "ges"), tables.index(SPECS[kern].pip_table),
-                      names.index(kern)))
+        lines.append("     {%s}, %s, %d, %d, %d}," %
+                     (", ".join(fn(v, "set_coef") for v in "ge"), fn("s", "set_coef"),
+                      tables.index(table_key(kern)), tables.index(SPECS[kern].pip_table), names.index(kern)))
     lines.append("};")
     lines.append("static const int mbx_num_evaluators = %d;" % len(SPECS))
     # host builders of the tensor-core operands of the mixed mode (QF_TYPES)
@@ -1463,7 +1157,7 @@ def write_registry():
     mon_of = {v: k for k, v in ONEBODY_DISPATCH.items()}
     lines.append("static const OneBodyInfo mbx_onebody[] = {%s};" % ", ".join(
         '{"%s", "%s", %d, mbx_fit_%s, %d, mbx_launch_%s_o}' %
-        (name, mon_of[name], sp.ncoef, name, tables.index(sp.pip_table), name)
+        (name, mon_of[name], sp.ncoef, name, tables.index(table_key(name)), name)
         for name, sp in ONEBODY_SPECS.items()))
     lines.append("static const int mbx_num_onebody = %d;" % len(ONEBODY_SPECS))
     # real atoms per monomer id (SetUpMonomers, bblock/sys_tools.cpp:133-254)
@@ -1493,8 +1187,8 @@ def main(argv=None, quiet=False):
             continue
         path, leaves, inner = generate(n)
         keep.add(os.path.basename(path))
-        if n in STRAIGHT_TYPES:
-            for v in ("pip", "pip_e", "qf" if n in QF_TYPES else "pip_s32"):
+        if n in SPECS:
+            for v in ("pip", "pip_e", "qf"):
                 keep.add("%s_%s.cuh" % (n, v))
         keep.update(os.path.basename(p) for p in write_kernels_cu(n))
         if not quiet:

@@ -497,18 +497,21 @@ def emit_cuda(q, name, nvars):
     return "\n".join(L) + "\n"
 
 
-def emit_host_tables(q, name):
-    """C++ arrays for the host-side assembly of C from the orbit coefficients:
-    per shifted monomial its (i, j) basis entry and orbit; the exponents t."""
+def emit_tables(q, name, kind, prefix):
+    """C++ arrays for the assembly of C from the orbit coefficients: per
+    shifted monomial its (i, j) basis entry and orbit; the exponents t.
+    kind: their storage class; prefix: of their names."""
     mi = ",".join(str(i) for i, _ in q.ij)
     mj = ",".join(str(j) for _, j in q.ij)
     mo = ",".join(str(int(o)) for o in q.sp.orbit_of)
+    assert len(set(q.ij)) == len(q.ij)
+    d = {"k": kind, "p": prefix, "n": name, "m": len(q.ij)}
     L = ["// quadratic form: entry (i, j) of every shifted monomial, its orbit; exponents t",
-         "static const int qf_nmono_%s = %d;" % (name, len(q.ij)),
-         "static const short qf_mi_%s[%d] = {%s};" % (name, len(q.ij), mi),
-         "static const short qf_mj_%s[%d] = {%s};" % (name, len(q.ij), mj),
-         "static const short qf_mo_%s[%d] = {%s};" % (name, len(q.ij), mo),
-         "static const signed char qf_t_%s[%d] = {%s};" % (name, q.npad, ",".join(str(int(x)) for x in q.t))]
+         "static constexpr int %(p)s_nmono_%(n)s = %(m)d;" % d,
+         "%(k)s short %(p)s_mi_%(n)s[%(m)d] = {" % d + mi + "};",
+         "%(k)s short %(p)s_mj_%(n)s[%(m)d] = {" % d + mj + "};",
+         "%(k)s short %(p)s_mo_%(n)s[%(m)d] = {" % d + mo + "};",
+         "%(k)s signed char %(p)s_t_%(n)s[%(w)d] = {" % dict(d, w=q.npad) + ",".join(str(int(x)) for x in q.t) + "};"]
     return "\n".join(L) + "\n"
 
 

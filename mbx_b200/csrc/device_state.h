@@ -1,13 +1,13 @@
 // Library state kept once per device and shared by every context on it.
 //
-// * The fitted coefficients of the straight-line kernels live in their
+// * The coefficients of the straight-line kernels live in their
 //   __constant__ banks, which exist once per device.  They are loaded with
 //   the models' fitted values the first time anything runs on a device
 //   (mbx_device_constants); that step copies to constant memory only and
 //   allocates nothing, so the allocation-free entry point can take it too.
 // * The term tables of all evaluators (one embedded binary) and a copy of
-//   every evaluator's coefficients in global memory, read by the
-//   table-driven kernels, are uploaded on the first context creation on a
+//   every evaluator's coefficients in global memory, fitted and in the w
+//   variables (the latter read by the table-driven kernels), are uploaded on the first context creation on a
 //   device (mbx_device_tables; allocates once per device, freed at exit).
 //
 // mbx_set_coefficients changes the coefficients of an evaluator on its
@@ -22,7 +22,8 @@
 
 struct DeviceTables {
     const unsigned char* blob = nullptr;   // device copy of the term-table binary
-    double* coef = nullptr;                // every evaluator's coefficients, at coef_off[evaluator]
+    double* coef = nullptr;                // every evaluator's fitted coefficients
+    double* cw = nullptr;                  // and its coefficients in the w variables (c = F a)
 };
 
 // Loads the fitted coefficients into the constant banks of device dev (once).

@@ -14,20 +14,21 @@
 // scatter steps of System::Get2B/Get3B (bblock/system.cpp:2425-2725,
 // 2769-3073).
 //
-// The evaluators without straight-line code (the CH4-CH4 polynomial with its
-// 201k terms and the widened MB-nrg types) are evaluated by a warp per n-mer
-// that walks the polynomial's term table (holder_table_kernel below).
+// The polynomial is that in the symmetry-adapted variables w
+// (mbx_b200/codegen/wbasis.py): T::to_w takes the variables x to w, T::from_w
+// the gradient back.  It has 3 to 8 times fewer terms (MB-pol 3b gradients of
+// 132k trimers: 1.36 ms in x, 0.41 ms in w; the types that had no
+// straight-line code ran from their term tables, 1 M NaCl 29 ms a step, now
+// 1.2).
 #pragma once
 #include "holder_common.cuh"
 #include "term_table.cuh"
 
 // Precision / output modes.
-// HM_GRAD_SHIFT32 names the paired FP32 kernels (pair_*_kernel) where a
-// template needs to tell the two gradient kernels apart.
-enum { HM_ENERGY = 0, HM_GRAD_FP64 = 1, HM_GRAD_SHIFT32 = 4 };
+enum { HM_ENERGY = 0, HM_GRAD_FP64 = 1 };
 
 // Scratch of the mixed-precision evaluation (three kernels: variables, the
-// paired FP32 trie, chain rule), for up to cap n-mers: the shifted FP32
+// polynomial on the tensor cores, chain rule), for up to cap n-mers: the shifted FP32
 // variables and the trie's gradient, variable-major ([v * cap + t]), the
 // polynomial's value and whether the n-mer is within the evaluator's cutoff.
 struct PairScratch {
@@ -44,7 +45,9 @@ struct HolderArgs {
     long n;                    // number of n-mers (capacity when n_dev is set)
     const int* n_dev;          // optional device-side count (read by the kernel, clamped to n)
     const int* status;         // optional: a nonzero word means the n-mer build failed; do nothing
-    int* counter;              // work counter (zeroed before the launch): warps claim chunks of 32 n-mers
+    int* counter;              // work counter (zeroed before the launch): blocks claim units (LockPlan)
+    int split;                 // 1: the last round's chunks may be cut by trie pieces (sums in another order;
+                               // e_per, where given, zeroed before the launch)
     const int4* nmers;         // system input: (m0, m1, m2, anchor slot), holder order
     const double* xyz;         // system input: site array (3 per site); AoS input: [n][NREAL*3]
     const int* first_index;    // system input: first site of every monomer
@@ -67,13 +70,6 @@ struct HolderArgs {
     // prime_pieces): of the rest only out (null) is read
     int prime_passes, prime_npieces;
     PairScratch ps;            // mixed precision: scratch of the three kernels
-};
-
-// Coefficient source: a global pointer, read through the read-only path.
-struct GlobalCoef {
-    const double* __restrict__ p;
-    __device__ __forceinline__ double operator[](int k) const { return __ldg(p + k); }
-    __device__ __forceinline__ float f(int k) const { return (float)__ldg(p + k); }
 };
 
 __device__ __forceinline__ double ld_volatile(const double* p) {
@@ -276,10 +272,12 @@ __device__ __forceinline__ void chain_rule(const double (&s)[T::NSITES][3], cons
 }
 
 // Everything after the polynomial: chain rule, switch, virial, scatter.  g:
-// dP/dv as chain_rule takes it.
+// dP/dv as chain_rule takes it.  share: ep and g are a part of the n-mer's
+// polynomial whose rest is added by other threads (per-n-mer outputs by
+// atomics, e_per zeroed before the launch).
 template <class T, class G>
 __device__ __forceinline__ void finish_nmer(const HolderArgs& A, long t, double ep, const G& g, bool grads,
-                                            double (&acc)[7]) {
+                                            double (&acc)[7], bool share = false) {
     double r[T::NREAL][3];
     load_nmer<T, true>(A, t, r);
     double d[3][3], rr[3];
@@ -319,7 +317,10 @@ __device__ __forceinline__ void finish_nmer(const HolderArgs& A, long t, double 
         if (!T::VIRIAL_RAW) virial();
     }
     const double es = sw * ep;
-    if (A.e_per) A.e_per[t] = es;
+    if (A.e_per) {
+        if (share) atomicAdd(A.e_per + t, es);
+        else A.e_per[t] = es;
+    }
     v[0] = es;
     if (A.conf_out) {
         conf_accumulate(A.conf_out + 8 * __ldg(A.mon_conf + __ldg(A.nmers + t).x), v);
@@ -333,7 +334,10 @@ __device__ __forceinline__ void finish_nmer(const HolderArgs& A, long t, double 
 #pragma unroll
         for (int i = 0; i < T::NREAL; ++i)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) p[3 * i + c] += tg[i][c];
+            for (int c = 0; c < 3; ++c) {
+                if (share) atomicAdd(p + 3 * i + c, tg[i][c]);
+                else p[3 * i + c] += tg[i][c];
+            }
         return;
     }
     const int4 nm = __ldg(A.nmers + t);
@@ -359,46 +363,21 @@ __device__ __forceinline__ long nmer_count(const HolderArgs& A) {
     return c < A.n ? c : A.n;
 }
 
-// The polynomial (and its gradient) in the precision mode of the kernel, with
-// a block barrier after every separately compiled piece of the trie; x and
-// the gradient accumulators in shared memory, [v][thread], at the thread's
-// column (xs, gs).
-template <class T, int MODE, class C>
-__device__ __forceinline__ double run_pip_lock(const C& coef, const double* xs, double* gs) {
-    if constexpr (MODE == HM_ENERGY) {
-        return T::template pip_e_lock<T::LOCK_THREADS>(coef, xs);
-    } else {
-        static_assert(MODE == HM_GRAD_FP64, "unknown mode");
-        return T::template pip_lock<T::LOCK_THREADS>(coef, xs, gs);
-    }
-}
-
 // Dynamic shared memory of the lockstep kernels (their x/g columns).
 extern __shared__ __align__(16) unsigned char mbx_dyn_smem[];
 
-// FP64 coefficients copied from constant to shared memory once per block
-// (types with T::SMEM_COEF).
-template <class CC>
-struct SharedCoef {
-    const double* p;
-    __device__ __forceinline__ double operator[](int k) const { return p[k]; }
-};
-
-// Code prefetch mode of the lockstep kernels.  Their trie is ~10^5
-// instructions of straight-line code.  Once other work has evicted it from
-// L2 (the rest of an MD step between two force calls), the first pass of
-// each SM through it waits on DRAM for every instruction fetch: ~0.4 ms of a
-// 1.3 ms FP64 evaluation of the 2048-water trimers, ~0.5 ms of the 0.8 ms
-// paired FP32 one.  An SM only gains from code that SMs of its own half of
-// the chip have fetched (one block through the whole trie beforehand
-// recovers half; a block on every SM, all of it).  A prefetch launch of the
-// same kernel (ptxas compiles a __noinline__ piece separately for every
-// kernel that calls it, so only the kernel's own launch fetches the code the
-// evaluation runs) has one warp per block run piece (block + j * grid) mod
-// npieces in pass j: every piece fetched by several SMs spread over the chip,
-// all pieces at once.  It is launched beside the n-mer search, ahead of the
-// evaluation.  The lanes' x and g columns share one [v][L] array (x at
-// columns 0-31, g at 32-63) of zeros; the results are discarded.
+// Code prefetch mode of the lockstep kernels.  Once other work has evicted a
+// trie's code from L2 (the rest of an MD step between two force calls), the
+// first pass of each SM through it waits on DRAM for every instruction fetch.
+// An SM only gains from code that SMs of its own half of the chip have
+// fetched.  A prefetch launch of the same kernel (ptxas compiles a
+// __noinline__ piece separately for every kernel that calls it, so only the
+// kernel's own launch fetches the code the evaluation runs) has one warp per
+// block run piece (block + j * grid) mod npieces in pass j: every piece
+// fetched by several SMs spread over the chip, all pieces at once.  It is
+// launched beside the n-mer search, ahead of the evaluation.  The lanes' x and
+// g columns share one [v][L] array (x at columns 0-31, g at 32-63) of zeros;
+// the results are discarded.
 template <int L, class V, class Piece>
 __device__ __forceinline__ void prime_pieces(const HolderArgs& A, int nvars, Piece&& piece) {
     static_assert(L >= 64, "x and g columns of the prefetch overlap");
@@ -420,56 +399,75 @@ __device__ __forceinline__ void prime_pieces(const HolderArgs& A, int nvars, Pie
     if (A.out) A.out[threadIdx.x] = sum;   // null in a prefetch launch; keeps the calls
 }
 
+// The work of a lockstep grid of nslot blocks over nchunk chunks of n-mers
+// and npiece pieces of the trie: whole chunks in full rounds, then the chunks
+// of the last, partial round cut by pieces, so that the blocks that would
+// otherwise be idle take a share of the polynomial each (value and gradient
+// are sums over the pieces; every share ends with its own chain rule, switch
+// and scatter).
+struct LockPlan {
+    long whole, units;
+    int parts;
+    __device__ __forceinline__ LockPlan(long nchunk, long nslot, int npiece, bool split) {
+        whole = split ? nchunk / nslot * nslot : nchunk;
+        const long rest = nchunk - whole;
+        parts = rest > 0 ? (int)(nslot / rest < npiece ? nslot / rest : npiece) : 1;
+        units = whole + rest * parts;
+    }
+    // chunk and pieces [k0, k1) of unit u
+    __device__ __forceinline__ long unit(long u, int npiece, int& k0, int& k1) const {
+        if (u < whole) {
+            k0 = 0;
+            k1 = npiece;
+            return u;
+        }
+        const long v = u - whole;
+        const int p = (int)(v % parts);
+        k0 = p * npiece / parts;
+        k1 = (p + 1) * npiece / parts;
+        return whole + v / parts;
+    }
+};
+
 // One n-mer per thread, all warps of a block in lockstep through the trie:
-// the straight-line polynomial is ~10^5 instructions, far more than the
+// the straight-line polynomial is thousands of instructions, more than the
 // instruction cache holds, so the block's warps go through it piece by piece
 // together (a barrier after each piece) and one fetch of a piece's code serves
 // all of them.  Threads without an n-mer (past the end, or beyond the
-// evaluator's cutoff) run the pieces on zero variables and discard the result.
-// Persistent grid; a block claims chunks of blockDim.x n-mers from
-// A.counter (or strides statically without it).
-template <class T, class CC, int MODE, bool CUSTOM>
+// evaluator's cutoff) run the pieces on zero variables and discard the result;
+// warps of such threads only keep the barriers.  Persistent grid; a block
+// claims units (LockPlan) from A.counter (or strides statically without it).
+template <class T, class CC, int MODE>
 __global__ void __launch_bounds__(T::LOCK_THREADS, 1) holder_lock_kernel(const HolderArgs A) {
     constexpr bool grads = (MODE == HM_GRAD_FP64);
     constexpr int L = T::LOCK_THREADS;   // == blockDim.x
+    constexpr int NP = grads ? T::NPIECES : T::NPIECES_E;
     double* xs = reinterpret_cast<double*>(mbx_dyn_smem) + threadIdx.x;
     double* gs = xs + T::NVARS * L;      // used in gradient mode only
-    __shared__ long s_base;
-    __shared__ double s_coef[T::SMEM_COEF ? T::NCOEF : 1];
-    if constexpr (T::SMEM_COEF && !CUSTOM) {
-        for (int k = threadIdx.x; k < T::NCOEF; k += blockDim.x) s_coef[k] = CC{}[k];
-        __syncthreads();
-    }
-    if constexpr (!CUSTOM) {
-        if (A.prime_passes > 0) {
-            prime_pieces<L, double>(A, T::NVARS, [&](int k, const double* x, double* g) -> double {
-                if constexpr (MODE == HM_ENERGY) {
-                    if constexpr (T::SMEM_COEF) return T::template pip_e_piece<L>(k, SharedCoef<CC>{s_coef}, x);
-                    else return T::template pip_e_piece<L>(k, CC{}, x);
-                } else {
-                    if constexpr (T::SMEM_COEF) return T::template pip_piece<L>(k, SharedCoef<CC>{s_coef}, x, g);
-                    else return T::template pip_piece<L>(k, CC{}, x, g);
-                }
-            });
-            return;
-        }
+    __shared__ long s_unit;
+    const auto piece = [&](int k, const double* x, double* g) -> double {
+        if constexpr (MODE == HM_ENERGY) return T::template pip_e_piece<L>(k, CC{}, x);
+        else return T::template pip_piece<L>(k, CC{}, x, g);
+    };
+    if (A.prime_passes > 0) {
+        prime_pieces<L, double>(A, T::NVARS, piece);
+        return;
     }
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     const long n = nmer_count(A);
-    long static_next = blockIdx.x * (long)blockDim.x;
+    const LockPlan plan((n + L - 1) / L, gridDim.x, NP, A.split != 0);
+    long u = blockIdx.x;
     for (;;) {
-        long base;
         if (A.counter) {
-            if (threadIdx.x == 0) s_base = atomicAdd(A.counter, (int)blockDim.x);
+            if (threadIdx.x == 0) s_unit = atomicAdd(A.counter, 1);
             __syncthreads();
-            base = s_base;
+            u = s_unit;
             __syncthreads();
-        } else {
-            base = static_next;
-            static_next += (long)gridDim.x * blockDim.x;
         }
-        if (base >= n) break;
-        const long t = base + threadIdx.x;
+        if (u >= plan.units) break;
+        int k0, k1;
+        const long t = plan.unit(u, NP, k0, k1) * L + threadIdx.x;
+        const bool shared_nmer = k1 - k0 < NP;   // other blocks hold the rest of this n-mer's polynomial
         bool live = t < n;
         {
             double x[T::NVARS];
@@ -486,6 +484,7 @@ __global__ void __launch_bounds__(T::LOCK_THREADS, 1) holder_lock_kernel(const H
                     double s[T::NSITES][3];
                     T::sites(r, s);
                     T::vars(s, x);
+                    T::to_w(x);
                 }
             }
 #pragma unroll
@@ -494,16 +493,21 @@ __global__ void __launch_bounds__(T::LOCK_THREADS, 1) holder_lock_kernel(const H
                 if (grads) gs[v * L] = 0.0;
             }
         }
-        double ep;
-        if constexpr (CUSTOM) ep = run_pip_lock<T, MODE>(GlobalCoef{A.coef}, xs, gs);
-        else if constexpr (T::SMEM_COEF) ep = run_pip_lock<T, MODE>(SharedCoef<CC>{s_coef}, xs, gs);
-        else ep = run_pip_lock<T, MODE>(CC{}, xs, gs);
+        const bool busy = __any_sync(0xffffffffu, live);
+        double ep = 0.0;
+#pragma unroll 1
+        for (int k = k0; k < k1; ++k) {
+            if (busy) ep += piece(k, xs, gs);
+            __syncthreads();
+        }
         if (live) {
             double g[T::NVARS];
 #pragma unroll
             for (int v = 0; v < T::NVARS; ++v) g[v] = grads ? gs[v * L] : 0.0;
-            finish_nmer<T>(A, t, ep, g, grads, acc);
+            T::from_w(g);
+            finish_nmer<T>(A, t, ep, g, grads, acc, shared_nmer);
         }
+        u += gridDim.x;
     }
     block_reduce_add<7>(acc, A.out);
 }
@@ -548,18 +552,16 @@ __device__ __forceinline__ bool nmer_vars_f32(const HolderArgs& A, long t, long 
 }
 
 // Mixed-precision evaluation in three kernels.  The FP64 work around the
-// polynomial (gather, image, variables; later the switch, chain rule,
-// virial and scatter) is latency-bound and needs many warps, the paired FP32
-// trie needs few warps with all registers in lockstep; in one kernel both
-// ran at 8 warps per SM, so the FP64 parts took ~0.2 of the ~0.9 ms the
-// 2048-water trimers take.  Here:
+// polynomial (gather, image, variables; later the switch, chain rule, virial
+// and scatter) is latency-bound and needs many warps, the tensor-core kernel
+// takes whole SMs:
 //   pair_vars_kernel    one n-mer per thread at full occupancy: the FP64
 //                       variables, shifted to the FP32 basis, into A.ps.dx
-//   pair_trie_kernel    the paired FP32 trie in lockstep blocks (two n-mers
-//                       per thread), dx in, gradient and value out
+//   qf_eval_kernel      the polynomial (qf_kernel.cuh), dx in, gradient and
+//                       value out
 //   pair_finish_kernel  one n-mer per thread at full occupancy: switch,
 //                       chain rule (FP64), virial, scatter, energy sums
-// The variables, switch, chain rule and sums stay FP64 as before.
+// The variables, switch, chain rule and sums stay FP64.
 template <class T>
 __global__ void __launch_bounds__(256, 2) pair_vars_kernel(const HolderArgs A) {
     const long n = nmer_count(A);
@@ -577,67 +579,6 @@ __global__ void __launch_bounds__(256, 2) pair_vars_kernel(const HolderArgs A) {
     }
 }
 
-// Coefficient pairs of the FP32 basis copied from constant to shared memory
-// once per block (a shared-memory operand costs fewer instructions per leaf
-// than a constant-bank one in the paired form).
-template <class CC>
-struct SharedPairs {
-    const f2_t* p;
-    __device__ __forceinline__ f2_t f2(int k) const { return p[k]; }
-    __device__ __forceinline__ double b0() const { return CC{}.b0(); }
-};
-
-// The paired FP32 trie: two n-mers per thread, one in each half of the
-// paired FP32 registers, through the type's FP32-basis trie (T::SHIFTED) in
-// lockstep blocks; a block claims chunks of 2 x blockDim.x n-mers.
-template <class T, class CC>
-__global__ void __launch_bounds__(T::LOCK_THREADS_S, 1) pair_trie_kernel(const HolderArgs A) {
-    constexpr int L = T::LOCK_THREADS_S;   // == blockDim.x
-    f2_t* xs = reinterpret_cast<f2_t*>(mbx_dyn_smem) + threadIdx.x;
-    f2_t* gs = xs + T::NVARS * L;
-    __shared__ long s_base;
-    __shared__ f2_t s_coef[T::NORB];
-    for (int k = threadIdx.x; k < T::NORB; k += blockDim.x) s_coef[k] = CC{}.f2(k);
-    __syncthreads();
-    const SharedPairs<CC> coef{s_coef};
-    if (A.prime_passes > 0) {
-        prime_pieces<L, f2_t>(A, T::NVARS, [&](int k, const f2_t* x, f2_t* g) -> double {
-            const double2 e = T::template pip_s32_piece<L>(k, coef, x, g);
-            return e.x + e.y;
-        });
-        return;
-    }
-    const long n = nmer_count(A);
-    const long cap = A.ps.cap;
-    const long chunk = 2L * blockDim.x;
-    for (;;) {
-        if (threadIdx.x == 0) s_base = atomicAdd(A.counter, (int)chunk);
-        __syncthreads();
-        const long base = s_base;
-        __syncthreads();
-        if (base >= n) break;
-        const long t0 = base + threadIdx.x, t1 = t0 + blockDim.x;
-#pragma unroll
-        for (int v = 0; v < T::NVARS; ++v) {
-            const float lo = t0 < n ? A.ps.dx[v * cap + t0] : 0.0f;
-            const float hi = t1 < n ? A.ps.dx[v * cap + t1] : 0.0f;
-            xs[v * L] = f2_pack(lo, hi);
-            gs[v * L] = 0ull;
-        }
-        const double2 ep = T::template pip_s32_lock<L>(coef, xs, gs);
-        if (t0 < n) {
-#pragma unroll
-            for (int v = 0; v < T::NVARS; ++v) A.ps.g[v * cap + t0] = f2_lo(gs[v * L]);
-            A.ps.ep[t0] = coef.b0() + ep.x;
-        }
-        if (t1 < n) {
-#pragma unroll
-            for (int v = 0; v < T::NVARS; ++v) A.ps.g[v * cap + t1] = f2_hi(gs[v * L]);
-            A.ps.ep[t1] = coef.b0() + ep.y;
-        }
-    }
-}
-
 template <class T>
 __global__ void __launch_bounds__(128, 4) pair_finish_kernel(const HolderArgs A) {
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -648,126 +589,6 @@ __global__ void __launch_bounds__(128, 4) pair_finish_kernel(const HolderArgs A)
         // the chain rule from the radial factors pair_vars_kernel stored: no
         // square root, exponential or division per variable here
         finish_nmer<T>(A, t, A.ps.ep[t], PairFactors{{A.ps.g, cap, t}, {A.ps.q, cap, t}}, true, acc);
-    }
-    block_reduce_add<7>(acc, A.out);
-}
-
-// Table-driven evaluation (evaluators without straight-line code): a warp
-// per n-mer, lane l taking terms l, l+32, ... of the term table
-// (term_table.cuh); the n-mer's variables and gradient accumulators live in
-// shared memory, the gradient summed with shared-memory atomics.  The rest
-// (gather, image, variables, switch, chain rule, scatter) is the same code
-// as the straight-line kernels.
-template <class T, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) holder_table_kernel(const HolderArgs A, int grads) {
-    __shared__ double xs[WARPS][T::NVARS];
-    __shared__ double gs[WARPS][T::NVARS];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    const long stride = (long)gridDim.x * WARPS;
-    const long n = nmer_count(A);
-    for (long t = blockIdx.x * (long)WARPS + w; t < n; t += stride) {
-        double r[T::NREAL][3];
-        load_nmer<T, false>(A, t, r);
-        double d[3][3], rr[3];
-        if (pair_dists<T>(r, d, rr)) {
-            if (lane == 0 && A.e_per) A.e_per[t] = 0.0;
-            continue;
-        }
-        if (lane == 0) {
-            double s[T::NSITES][3], x[T::NVARS];
-            T::sites(r, s);
-            T::vars(s, x);
-#pragma unroll
-            for (int v = 0; v < T::NVARS; ++v) { xs[w][v] = x[v]; gs[w][v] = 0.0; }
-        }
-        __syncwarp();
-        const auto xv = [&](int v) { return xs[w][v]; };
-        double e = 0.0;
-        for (long q = lane; q < A.nterms; q += 32) {
-            const int4 tm = __ldg(A.terms + q);
-            const double c = __ldg(A.coef + tm.x) * __ldg(A.tcoef + q);
-            if (grads)
-                e += term_value_grad<T::TPAIRS>(tm, c, xv, [&](int v, double dv) { atomicAdd(&gs[w][v], dv); });
-            else
-                e += term_value<T::TPAIRS>(tm, c, xv);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-        __syncwarp();
-        if (lane == 0) {
-            double g[T::NVARS];
-#pragma unroll
-            for (int v = 0; v < T::NVARS; ++v) g[v] = gs[w][v];
-            finish_nmer<T>(A, t, e, g, grads != 0, acc);
-        }
-        __syncwarp();
-    }
-    block_reduce_add<7>(acc, A.out);
-}
-
-// Table-driven evaluation, a lane per n-mer: the warp walks the whole term
-// table in step, every lane applying each term to its own n-mer, whose
-// variables and gradient accumulators sit in shared-memory columns [v][lane]
-// (conflict-free, no atomics).  This is the form for the many-n-mer buckets
-// of a liquid (a warp per n-mer would serialise on shared-memory atomics of
-// the few variables); the 201k-term CH4-CH4 table, with few dimers per box,
-// keeps the warp-per-n-mer form above.  Dynamic shared memory:
-// 4 warps x 2 x NVARS x 32 doubles.
-template <class T>
-__global__ void __launch_bounds__(128) holder_table_lane_kernel(const HolderArgs A, int grads) {
-    double* xc = reinterpret_cast<double*>(mbx_dyn_smem) + ((threadIdx.x >> 5) * 2 * T::NVARS) * 32 +
-                 (threadIdx.x & 31);
-    double* gc = xc + T::NVARS * 32;
-    double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-    const long n = nmer_count(A);
-    for (long base = blockIdx.x * (long)blockDim.x; base < n; base += (long)gridDim.x * blockDim.x) {
-        const long t = base + threadIdx.x;
-        bool live = t < n;
-        {
-            double x[T::NVARS];
-#pragma unroll
-            for (int v = 0; v < T::NVARS; ++v) x[v] = 0.0;
-            if (live) {
-                double r[T::NREAL][3];
-                load_nmer<T, false>(A, t, r);
-                double d[3][3], rr[3];
-                if (pair_dists<T>(r, d, rr)) {
-                    if (A.e_per) A.e_per[t] = 0.0;
-                    live = false;
-                } else {
-                    double s[T::NSITES][3];
-                    T::sites(r, s);
-                    T::vars(s, x);
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < T::NVARS; ++v) {
-                xc[v * 32] = x[v];
-                gc[v * 32] = 0.0;
-            }
-        }
-        __syncwarp();
-        double e = 0.0;
-        if (__any_sync(0xffffffffu, live)) {
-            const auto xv = [&](int v) { return xc[v * 32]; };
-            for (long q = 0; q < A.nterms; ++q) {
-                const int4 tm = __ldg(A.terms + q);
-                const double c = __ldg(A.coef + tm.x) * __ldg(A.tcoef + q);
-                if (grads)
-                    e += term_value_grad<T::TPAIRS>(tm, c, xv, [&](int v, double dv) { gc[v * 32] += dv; });
-                else
-                    e += term_value<T::TPAIRS>(tm, c, xv);
-            }
-        }
-        __syncwarp();
-        if (live) {
-            double g[T::NVARS];
-#pragma unroll
-            for (int v = 0; v < T::NVARS; ++v) g[v] = grads ? gc[v * 32] : 0.0;
-            finish_nmer<T>(A, t, e, g, grads != 0, acc);
-        }
-        __syncwarp();
     }
     block_reduce_add<7>(acc, A.out);
 }
@@ -805,6 +626,7 @@ __global__ void __launch_bounds__(128) onebody_table_kernel(const HolderArgs A) 
                     for (int c = 0; c < 3; ++c) r[i][c] = p[3 * i + c];
                 T::sites(r, s);
                 T::vars(s, x);
+                T::to_w(x);
             }
 #pragma unroll
             for (int v = 0; v < T::NVARS; ++v) {
@@ -832,6 +654,7 @@ __global__ void __launch_bounds__(128) onebody_table_kernel(const HolderArgs A) 
                 double g[T::NVARS];
 #pragma unroll
                 for (int v = 0; v < T::NVARS; ++v) g[v] = gc[v * 32];
+                T::from_w(g);
                 double sg[T::NSITES][3];
                 T::chain(s, g, sg);
                 const int ia[6] = {0, 0, 0, 1, 1, 2}, ib[6] = {0, 1, 2, 1, 2, 2};
@@ -854,64 +677,32 @@ __global__ void __launch_bounds__(128) onebody_table_kernel(const HolderArgs A) 
     block_reduce_add<7>(acc, A.out);
 }
 
-// Gradient with respect to the linear coefficients: out[k] += sum over n-mers
-// of w[n] * sw(n) * dP/da_k(x(n)), the monomials recomputed from the
-// coordinates (adjoint of E = sum_n sw(n) P(a, x(n)) for refitting), from the
-// term table.  A lane per n-mer, its variables in a shared-memory column; the
-// warp walks the table (sorted by coefficient) in step, and at the end of a
-// coefficient's terms the lanes' sums are reduced across the warp into a
-// per-block shared array, added to out at the end.
-// Dynamic shared memory: NCOEF doubles + 4 warps x NVARS x 32 doubles.
+// First step of the coefficient adjoint (coef_adjoint_kernel has the second):
+// the w variables of n-mers first .. first + count and, as row NVARS, their
+// weight times the switch (0 beyond the evaluator's cutoff), variable-major in
+// wv with stride count.  One n-mer per thread.
 template <class T>
-__global__ void __launch_bounds__(128) holder_dcoef_table_kernel(const HolderArgs A, const double* __restrict__ w,
-                                                                 double* __restrict__ out) {
-    double* part = reinterpret_cast<double*>(mbx_dyn_smem);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double* xcol = part + T::NCOEF + (warp * T::NVARS) * 32 + lane;
-    for (int k = threadIdx.x; k < T::NCOEF; k += blockDim.x) part[k] = 0.0;
-    __syncthreads();
-    const long nt = nmer_count(A);
-    for (long base = blockIdx.x * (long)blockDim.x; base < nt; base += (long)gridDim.x * blockDim.x) {
-        const long t = base + threadIdx.x;
-        double scale = 0.0;
-        double x[T::NVARS];
+__global__ void __launch_bounds__(128) holder_wvars_kernel(const HolderArgs A, const double* __restrict__ w,
+                                                           long first, int count, double* __restrict__ wv) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const long t = first + i;
+    double x[T::NVARS];
 #pragma unroll
-        for (int v = 0; v < T::NVARS; ++v) x[v] = 0.0;
-        if (t < nt) {
-            double r[T::NREAL][3];
-            load_nmer<T, false>(A, t, r);
-            double d[3][3], rr[3];
-            if (!pair_dists<T>(r, d, rr)) {
-                double s[T::NSITES][3];
-                T::sites(r, s);
-                T::vars(s, x);
-                double tg[T::NREAL][3];
-                scale = apply_switch<T>(d, rr, 0.0, tg, false) * (w ? w[t] : 1.0);
-            }
-        }
-#pragma unroll
-        for (int v = 0; v < T::NVARS; ++v) xcol[v * 32] = x[v];
-        __syncwarp();
-        if (__any_sync(0xffffffffu, scale != 0.0)) {
-            const auto xv = [&](int v) { return xcol[v * 32]; };
-            double sum = 0.0;
-            int4 tm = __ldg(A.terms);
-            for (long q = 0; q < A.nterms; ++q) {
-                const int4 nx = q + 1 < A.nterms ? __ldg(A.terms + q + 1) : make_int4(-1, 0, 0, 0);
-                sum += term_value<T::TPAIRS>(tm, __ldg(A.tcoef + q), xv);
-                if (nx.x != tm.x) {
-                    double v = sum * scale;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                    if (lane == 0 && v != 0.0) atomicAdd(&part[tm.x], v);
-                    sum = 0.0;
-                }
-                tm = nx;
-            }
-        }
-        __syncwarp();
+    for (int v = 0; v < T::NVARS; ++v) x[v] = 0.0;
+    double scale = 0.0;
+    double r[T::NREAL][3];
+    load_nmer<T, false>(A, t, r);
+    double d[3][3], rr[3];
+    if (!pair_dists<T>(r, d, rr)) {
+        double s[T::NSITES][3];
+        T::sites(r, s);
+        T::vars(s, x);
+        T::to_w(x);
+        double tg[T::NREAL][3];
+        scale = apply_switch<T>(d, rr, 0.0, tg, false) * (w ? w[t] : 1.0);
     }
-    __syncthreads();
-    for (int k = threadIdx.x; k < T::NCOEF; k += blockDim.x)
-        if (part[k] != 0.0) atomicAdd(out + k, part[k]);
+#pragma unroll
+    for (int v = 0; v < T::NVARS; ++v) wv[(size_t)v * count + i] = x[v];
+    wv[(size_t)T::NVARS * count + i] = scale;
 }

@@ -36,13 +36,35 @@ int mbx_launch_ps1b(const OneBodyArgs& A, int sms, cudaStream_t s);
 
 // Generic table-driven polynomial over caller-supplied variables
 // (table_kernels.cu).
-int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double* e, const int4* terms,
-                          const double* tcoef, long nterms, const double* coef, int pairs, int sms, cudaStream_t s);
+struct PolyTable {
+    const int4* terms;
+    const double* tcoef;
+    long nterms;
+    int pairs;
+    const double* coef;
+    const int *wrow, *w, *wtrow, *wt;
+    const double* w0;
+};
+int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double* e, const PolyTable& P, int sms,
+                          cudaStream_t s);
+
+// Coefficient adjoint over n-mers whose w variables are in wv (table_kernels.cu).
+struct AdjointTable {
+    const int4* terms;
+    const double* tcoef;
+    int nterms, nhalf, nvars, ncoef;
+    const int2* half;
+    const unsigned* pair;
+    const int *ftrow, *ftk;
+    const double* ftf;
+};
+int mbx_coef_adjoint_blocks(const AdjointTable& P, int sms);
+int mbx_launch_coef_adjoint(const double* wv, int count, const AdjointTable& P, double* work, double* out, int sms,
+                            cudaStream_t s);
 
 typedef int (*launch_fn)(const HolderArgs&, int, int, cudaStream_t);
-typedef int (*dcoef_fn)(const HolderArgs&, const double*, double*, int, int, cudaStream_t);
+typedef int (*dcoef_fn)(const HolderArgs&, const double*, long, int, double*, cudaStream_t);
 typedef int (*prime_fn)(cudaStream_t);
-typedef int (*warp_fn)(const HolderArgs&, int, int, cudaStream_t);
 typedef int (*setcoef_fn)(const double*, int, cudaStream_t);
 
 struct EvaluatorInfo {
@@ -53,14 +75,15 @@ struct EvaluatorInfo {
     int skip;
     int ncoef, nreal, nvars;
     const double* fit;
-    launch_fn g, e;   // straight-line FP64 kernels (energy + gradient, energy only), or null
-    dcoef_fn c;       // coefficient adjoint (table-driven)
-    warp_fn w;        // table-driven evaluation of the types without straight-line kernels, or null
+    launch_fn g, e;   // straight-line FP64 kernels (energy + gradient, energy only)
+    dcoef_fn c;       // variables of the coefficient adjoint
     launch_fn s;      // FP32 kernel of the mixed mode (FP32 basis), or null
     double split_r;   // mixed mode: n-mers with first-atom distance below this run in FP64 (0: none)
     prime_fn pg, pe, ps;   // code prefetch of the g, e and s kernels (holder_prime_kernel), or null
-    setcoef_fn set[7];     // constant-memory coefficient setters of the straight-line kernels
-    int table;        // term table (mbx_term_tables)
+    setcoef_fn set[2];     // constant-memory coefficient setters of the g and e kernels (w coefficients)
+    setcoef_fn set_s;      // of the s kernel (fitted coefficients), or null
+    int table;        // term table (mbx_term_tables) of the kernels
+    int ptable;       // the same without a reference point, for caller-supplied variables (mbx_poly)
     int kern;         // evaluator whose kernels and coefficients this one runs (itself or an alias target)
 };
 
@@ -109,28 +132,100 @@ constexpr int kMaxDevices = 64;
 std::mutex g_dev_mu;
 bool g_dev_constants[kMaxDevices] = {false};
 DeviceTables g_dev_tables[kMaxDevices];
-long g_coef_off[256];
-long g_coef_off_1b[16];
-long g_coef_total = -1;
+// offsets of every evaluator's fitted coefficients and of its coefficients in
+// the w variables (c = F a) in DeviceTables::coef and ::cw
+long g_coef_off[256], g_cw_off[256], g_cp_off[256];   // g_cp_off: those of ptable
+long g_coef_off_1b[16], g_cw_off_1b[16];
+long g_coef_total = -1, g_cw_total = 0;
 
 void coef_layout() {
     if (g_coef_total >= 0) return;
-    long off = 0;
+    long off = 0, cw = 0;
     for (int i = 0; i < mbx_num_evaluators; ++i) {
         g_coef_off[i] = off;
+        g_cw_off[i] = g_cp_off[i] = cw;
         off += mbx_evaluators[i].ncoef;
+        cw += mbx_term_tables[mbx_evaluators[i].table].ncw;
+        if (mbx_evaluators[i].ptable != mbx_evaluators[i].table) {
+            g_cp_off[i] = cw;
+            cw += mbx_term_tables[mbx_evaluators[i].ptable].ncw;
+        }
     }
     for (int i = 0; i < mbx_num_onebody; ++i) {
         g_coef_off_1b[i] = off;
+        g_cw_off_1b[i] = cw;
         off += mbx_onebody[i].ncoef;
+        cw += mbx_term_tables[mbx_onebody[i].table].ncw;
     }
     g_coef_total = off;
+    g_cw_total = cw;
 }
 
 }  // namespace
 
 // The embedded term tables (gen/terms_blob.cpp).
 extern "C" const unsigned char mbx_terms_blob[];
+
+// Sum of products in twice the working precision (error-free transformations,
+// Ogita, Rump and Oishi 2005): c = F a cancels in the types with a reference
+// point, and an error in c is the same for every n-mer.
+struct Sum2 {
+    double hi = 0.0, lo = 0.0;
+    __host__ __device__ void add(double x, double y) {
+#ifdef __CUDA_ARCH__
+        const double p = __dmul_rn(x, y), e = __fma_rn(x, y, -p);
+        const double s = __dadd_rn(hi, p), z = __dsub_rn(s, hi);
+        const double t = __dadd_rn(__dsub_rn(hi, __dsub_rn(s, z)), __dsub_rn(p, z));
+        lo = __dadd_rn(lo, __dadd_rn(t, e));
+#else
+        const volatile double p = x * y, e = std::fma(x, y, -p);
+        const volatile double s = hi + p, z = s - hi;
+        const volatile double u = s - z, t = (hi - u) + (p - z);
+        lo += t + e;
+#endif
+        hi = s;
+    }
+};
+
+// c = F a of a term table, on the host and on the device.
+static std::vector<double> w_coefficients(int table, const double* a) {
+    const TermTableInfo& T = mbx_term_tables[table];
+    const int* row = reinterpret_cast<const int*>(mbx_terms_blob + T.off_frow);
+    const int* k = reinterpret_cast<const int*>(mbx_terms_blob + T.off_fk);
+    const double* f = reinterpret_cast<const double*>(mbx_terms_blob + T.off_ff);
+    std::vector<double> c(T.ncw);
+    for (int j = 0; j < T.ncw; ++j) {
+        Sum2 s;
+        for (int q = row[j]; q < row[j + 1]; ++q) s.add(f[q], a[k[q]]);
+        c[j] = s.hi + s.lo;
+    }
+    return c;
+}
+
+// (a warp per row: each lane a strand of the row, the strands joined in order)
+__global__ void k_w_coefficients(const int* __restrict__ row, const int* __restrict__ k, const double* __restrict__ f,
+                                 int ncw, const double* __restrict__ a, double* __restrict__ c) {
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (j >= ncw) return;
+    Sum2 s;
+    for (int q = row[j] + lane; q < row[j + 1]; q += 32) s.add(f[q], a[k[q]]);
+    Sum2 t;
+    for (int i = 0; i < 32; ++i) {
+        t.add(__shfl_sync(0xffffffffu, s.hi, i), 1.0);
+        t.lo += __shfl_sync(0xffffffffu, s.lo, i);
+    }
+    if (lane == 0) c[j] = t.hi + t.lo;
+}
+
+// The device's w coefficients of a term table from the fitted ones at a.
+static cudaError_t launch_w_coefficients(const unsigned char* blob, int table, const double* a, double* c,
+                                         cudaStream_t s) {
+    const TermTableInfo& T = mbx_term_tables[table];
+    k_w_coefficients<<<(T.ncw + 3) / 4, 128, 0, s>>>(
+        reinterpret_cast<const int*>(blob + T.off_frow), reinterpret_cast<const int*>(blob + T.off_fk),
+        reinterpret_cast<const double*>(blob + T.off_ff), T.ncw, a, c);
+    return cudaGetLastError();
+}
 
 std::mutex& mbx_device_mutex() { return g_dev_mu; }
 
@@ -150,8 +245,12 @@ static int device_constants_locked(int dev) {
     for (int i = 0; i < mbx_num_evaluators && rc == MBX_OK; ++i) {
         const EvaluatorInfo& E = mbx_evaluators[i];
         if (E.kern != i) continue;   // an alias shares its target's kernels and coefficients
-        for (int v = 0; v < 7; ++v)
-            if (E.set[v] && E.set[v](E.fit, 0, nullptr) != 0) rc = MBX_ECUDA;
+        const std::vector<double> c = w_coefficients(E.table, E.fit);
+        for (int v = 0; v < 2; ++v)
+            if (E.set[v] && E.set[v](c.data(), 0, nullptr) != 0) rc = MBX_ECUDA;
+        if (E.set_s && E.set_s(E.fit, 0, nullptr) != 0) rc = MBX_ECUDA;
+        // c and the staging of its copies must outlive them
+        if (cudaStreamSynchronize(nullptr) != cudaSuccess) rc = MBX_ECUDA;
     }
     if (rc == MBX_OK && cudaDeviceSynchronize() != cudaSuccess) rc = MBX_ECUDA;
     if (rc == MBX_OK) g_dev_constants[dev] = true;
@@ -176,23 +275,37 @@ int mbx_device_tables(int dev, DeviceTables* out) {
         if (cur != dev && cudaSetDevice(dev) != cudaSuccess) return MBX_ECUDA;
         void* blob = nullptr;
         void* coef = nullptr;
+        void* cw = nullptr;
         cudaError_t e = cudaMalloc(&blob, (size_t)mbx_terms_bytes);
         if (e == cudaSuccess) e = cudaMalloc(&coef, (size_t)g_coef_total * sizeof(double));
+        if (e == cudaSuccess) e = cudaMalloc(&cw, (size_t)g_cw_total * sizeof(double));
         if (e == cudaSuccess) e = cudaMemcpy(blob, mbx_terms_blob, (size_t)mbx_terms_bytes, cudaMemcpyHostToDevice);
-        for (int i = 0; i < mbx_num_evaluators && e == cudaSuccess; ++i)
-            e = cudaMemcpy(static_cast<double*>(coef) + g_coef_off[i], mbx_evaluators[i].fit,
-                           mbx_evaluators[i].ncoef * sizeof(double), cudaMemcpyHostToDevice);
-        for (int i = 0; i < mbx_num_onebody && e == cudaSuccess; ++i)
-            e = cudaMemcpy(static_cast<double*>(coef) + g_coef_off_1b[i], mbx_onebody[i].fit,
-                           mbx_onebody[i].ncoef * sizeof(double), cudaMemcpyHostToDevice);
+        // the fitted coefficients of all evaluators, in one copy each
+        std::vector<double> ha(g_coef_total), hc(g_cw_total);
+        auto put = [&](int table, const double* fit, int ncoef, long off, long off_cw) {
+            std::copy(fit, fit + ncoef, ha.begin() + off);
+            const std::vector<double> c = w_coefficients(table, fit);
+            std::copy(c.begin(), c.end(), hc.begin() + off_cw);
+        };
+        for (int i = 0; i < mbx_num_evaluators; ++i) {
+            const EvaluatorInfo& E = mbx_evaluators[i];
+            put(E.table, E.fit, E.ncoef, g_coef_off[i], g_cw_off[i]);
+            if (E.ptable != E.table) put(E.ptable, E.fit, E.ncoef, g_coef_off[i], g_cp_off[i]);
+        }
+        for (int i = 0; i < mbx_num_onebody; ++i)
+            put(mbx_onebody[i].table, mbx_onebody[i].fit, mbx_onebody[i].ncoef, g_coef_off_1b[i], g_cw_off_1b[i]);
+        if (e == cudaSuccess) e = cudaMemcpy(coef, ha.data(), ha.size() * sizeof(double), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(cw, hc.data(), hc.size() * sizeof(double), cudaMemcpyHostToDevice);
         if (cur != dev) cudaSetDevice(cur);
         if (e != cudaSuccess) {
             if (blob) cudaFree(blob);
             if (coef) cudaFree(coef);
+            if (cw) cudaFree(cw);
             return MBX_ECUDA;
         }
         T.blob = static_cast<const unsigned char*>(blob);
         T.coef = static_cast<double*>(coef);
+        T.cw = static_cast<double*>(cw);
     }
     *out = T;
     return MBX_OK;
@@ -949,14 +1062,15 @@ static HolderArgs base_args(mbx_ctx* c) {
     return A;
 }
 
-// Term table and global-memory coefficients of evaluator E on the context's
-// device, for the table-driven kernels.
-static void table_args(mbx_ctx* c, const EvaluatorInfo* E, HolderArgs& A) {
-    const TermTableInfo& T = mbx_term_tables[E->table];
+// Term table and global-memory coefficients (w variables) of evaluator E on
+// the context's device, for the table-driven kernels (plain: without a
+// reference point).
+static void table_args(mbx_ctx* c, const EvaluatorInfo* E, HolderArgs& A, bool plain = false) {
+    const TermTableInfo& T = mbx_term_tables[plain ? E->ptable : E->table];
     A.terms = reinterpret_cast<const int4*>(c->tables.blob + T.off_terms);
     A.tcoef = reinterpret_cast<const double*>(c->tables.blob + T.off_tcoef);
     A.nterms = T.nterms;
-    if (!A.coef) A.coef = c->tables.coef + mbx_coef_offset(E->kern);
+    A.coef = c->tables.cw + (plain ? g_cp_off : g_cw_off)[E->kern];
 }
 
 static int launch_eval(mbx_ctx* c, const EvaluatorInfo* E, HolderArgs A, int flags, int* kernels,
@@ -964,19 +1078,12 @@ static int launch_eval(mbx_ctx* c, const EvaluatorInfo* E, HolderArgs A, int fla
     const bool grads = !(flags & MBX_NO_GRADS);
     const bool mixed = (flags & MBX_MIXED) != 0;
     const int block = 128;
-    if (E->w) {
-        table_args(c, E, A);
-        long nw = A.n;
-        int grid = (int)std::min<long>((nw + 3) / 4, (long)c->sm_count * 8);
-        RCHK(c, E->w(A, grads ? 1 : 0, std::max(grid, 1), c->stream));
-        ++*kernels;
-        return MBX_OK;
-    }
     // mixed mode: the FP32-basis kernel where the type has one; FP64 for the
     // short-range bucket of a split type, for a split type's AoS input (no
     // builder to separate the short-range n-mers) and for types without one
     const bool fp32 = mixed && !near && E->s && !(A.aos && E->split_r > 0);
     launch_fn fn = !grads ? E->e : fp32 ? E->s : E->g;
+    A.split = A.aos ? 0 : 1;   // (per-n-mer outputs stay the same from call to call)
     if (!fn) return fail(c, MBX_ENOTSUP, std::string("no kernel for ") + E->name);
     if (fn == E->s) {
         // scratch of the three mixed-precision kernels for up to A.n n-mers
@@ -1018,7 +1125,6 @@ static int launch_prime(mbx_ctx* c, int nbody, int flags, int* kernels) {
         const bool near = c->bucket_near[nbody][b];
         if (near && !mixed) continue;
         const EvaluatorInfo* E = c->bucket_eval[nbody][b];
-        if (E->w) continue;
         const bool fp32 = mixed && !near && E->s;
         const prime_fn fn = !grads ? E->pe : fp32 ? E->ps : E->pg;
         if (!fn || std::find(done, done + ndone, fn) != done + ndone) continue;
@@ -1246,7 +1352,7 @@ static int onebody_term(mbx_ctx* c, double* X, double* G, double* energy, double
             H.terms = reinterpret_cast<const int4*>(c->tables.blob + T.off_terms);
             H.tcoef = reinterpret_cast<const double*>(c->tables.blob + T.off_tcoef);
             H.nterms = T.nterms;
-            H.coef = c->tables.coef + g_coef_off_1b[i];
+            H.coef = c->tables.cw + g_cw_off_1b[i];
             RCHK(c, mbx_onebody[i].launch(H, 0, 128, c->stream));
             ++*kernels;
         }
@@ -1692,8 +1798,24 @@ extern "C" int mbx_evaluate_dcoef(mbx_ctx* c, const char* name, long n, const do
     A.xyz = X;
     table_args(c, E, A);
     if (n > 0) {
-        const int grid = (int)std::max<long>(1, std::min<long>((n + 127) / 128, (long)c->sm_count * 2));
-        RCHK(c, E->c(A, W, O, grid, 128, c->stream));
+        // the variables of up to kAdjointChunk n-mers at a time in scratch, with
+        // the blocks' sums per term
+        constexpr long kAdjointChunk = 32768;
+        const TermTableInfo& T = mbx_term_tables[E->table];
+        const int chunk = (int)std::min(n, kAdjointChunk);
+        const AdjointTable P{A.terms, A.tcoef, (int)A.nterms, T.nhalf, E->nvars, E->ncoef,
+                             reinterpret_cast<const int2*>(c->tables.blob + T.off_half),
+                             reinterpret_cast<const unsigned*>(c->tables.blob + T.off_pair),
+                             reinterpret_cast<const int*>(c->tables.blob + T.off_ftrow),
+                             reinterpret_cast<const int*>(c->tables.blob + T.off_ftk),
+                             reinterpret_cast<const double*>(c->tables.blob + T.off_ftf)};
+        const size_t nv = (size_t)(E->nvars + 1) * chunk;
+        CUCHK(c, c->coef_ws.ensure(nv + (size_t)mbx_coef_adjoint_blocks(P, c->sm_count) * A.nterms + A.nterms));
+        for (long first = 0; first < n; first += chunk) {
+            const int count = (int)std::min<long>(chunk, n - first);
+            RCHK(c, E->c(A, W, first, count, c->coef_ws.p, c->stream));
+            RCHK(c, mbx_launch_coef_adjoint(c->coef_ws.p, count, P, c->coef_ws.p + nv, O, c->sm_count, c->stream));
+        }
     }
     if (!dev) {
         std::vector<double> tmp(E->ncoef);
@@ -1741,9 +1863,12 @@ extern "C" int mbx_poly(mbx_ctx* c, const char* name, long nd, const double* x, 
     }
     if (nd > 0) {
         HolderArgs A = base_args(c);
-        table_args(c, E, A);
-        RCHK(c, mbx_launch_poly_table(nd, E->nvars, X, G, Ev, A.terms, A.tcoef, A.nterms, A.coef,
-                                      mbx_term_tables[E->table].pairs, c->sm_count, c->stream));
+        table_args(c, E, A, true);
+        const TermTableInfo& T = mbx_term_tables[E->ptable];
+        auto ints = [&](long off) { return reinterpret_cast<const int*>(c->tables.blob + off); };
+        const PolyTable P{A.terms, A.tcoef, A.nterms, T.pairs, A.coef, ints(T.off_wrow), ints(T.off_w), ints(T.off_wtrow),
+                          ints(T.off_wt), reinterpret_cast<const double*>(c->tables.blob + T.off_w0)};
+        RCHK(c, mbx_launch_poly_table(nd, E->nvars, X, G, Ev, P, c->sm_count, c->stream));
     }
     if (!dev && nd > 0) {
         CUCHK(c, cudaMemcpyAsync(e, Ev, nd * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1765,10 +1890,18 @@ extern "C" int mbx_set_coefficients(mbx_ctx* c, const char* name, const double* 
     // context's) before changing them, under the device-state lock
     std::lock_guard<std::mutex> lock(mbx_device_mutex());
     CUCHK(c, cudaDeviceSynchronize());
-    for (int v = 0; v < 7; ++v)
-        if (K->set[v]) RCHK(c, K->set[v](src, dev ? 1 : 0, c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->tables.coef + mbx_coef_offset(E->kern), src, E->ncoef * sizeof(double),
-                             dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->stream));
+    // fitted coefficients -> w coefficients -> the kernels' constant banks,
+    // all on the device
+    double* A = c->tables.coef + mbx_coef_offset(E->kern);
+    double* W = c->tables.cw + g_cw_off[E->kern];
+    CUCHK(c, cudaMemcpyAsync(A, src, E->ncoef * sizeof(double), dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                             c->stream));
+    CUCHK(c, launch_w_coefficients(c->tables.blob, K->table, A, W, c->stream));
+    if (K->ptable != K->table)
+        CUCHK(c, launch_w_coefficients(c->tables.blob, K->ptable, A, c->tables.cw + g_cp_off[E->kern], c->stream));
+    for (int v = 0; v < 2; ++v)
+        if (K->set[v]) RCHK(c, K->set[v](W, 1, c->stream));
+    if (K->set_s) RCHK(c, K->set_s(A, 1, c->stream));
     CUCHK(c, cudaStreamSynchronize(c->stream));
     return MBX_OK;
 }

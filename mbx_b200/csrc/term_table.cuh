@@ -4,22 +4,19 @@
 // A polynomial of the reference's generated-polynomial convention is linear
 // in its fitted coefficients a (poly_2b_v6x::eval(nd, a, x),
 // potential/2b/poly-2b-v6x.h:78; poly_3b_v2x::eval(a, x), poly-3b-v2x.h:73;
-// the MB-nrg eval(a, x) / eval(x, a) programs).  Expanded, it is
-//     P(a, x) = sum_t a[k_t] * c_t * prod_i x[v_t,i]^e_t,i
-// over its terms t.  A table holds one int4 per term plus its multiplicity
-// c_t (a double):
-//     x: k_t (index of the fitted coefficient; the table is sorted by k)
+// the MB-nrg eval(a, x) / eval(x, a) programs).  In the symmetry-adapted
+// variables w (mbx_b200/codegen/wbasis.py) it is
+//     P = sum_t c[k_t] s_t prod_i w[v_t,i]^e_t,i,   c = F a,
+// over its terms t.  A table holds one int4 per term plus its sign s_t (a
+// double):
+//     x: k_t (index of the coefficient; the table is sorted by k)
 //     y, z, w: six (variable, exponent) byte pairs, low byte the variable
 //              (255: unused), high byte the exponent, in the order the
 //              variables appear in the term
-// Six pairs cover every table of the library (at most six distinct
-// variables per term; a single variable may carry an exponent up to 23).
+// Six pairs cover every table of the library.
 //
-// Three uses share the decoding below: the warp-per-n-mer evaluation of the
-// evaluators without straight-line code (holder_table_kernel), the adjoint
-// with respect to the coefficients (holder_dcoef_table_kernel) and the
-// generated-polynomial entry point over caller-supplied variables
-// (poly_table_kernel).
+// Used by the generated-polynomial entry point over caller-supplied variables
+// (poly_table_kernel) and the 1-body kernels.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -399,7 +399,7 @@ def emit_traits(spec, table, straight, npieces, out):
     w("    static constexpr int SWITCH_TRIPLE = %d, SKIP = %d, DEGREE = %d;" %
       ({"pair": 0, "triple": 1, "triple2": 2, "cos2": 3, "none": 0}[spec.switch],
        {"pair_gt": 0, "two_of_three_gt": 1, "all_three_gt": 2, "none": 0}[spec.skip],
-       1 if straight else 0, spec.degree))
+       spec.degree))
     w("    static constexpr int TPAIRS = %d;  // (variable, exponent) pairs of a term, at most" %
       term_pairs_max(table_key(n)))
     w("    static constexpr double RI = %s, RF = %s;" % (lit(spec.ri), lit(spec.rf)))
@@ -1005,13 +1005,14 @@ def write_term_tables():
             rr = rr + [(255, 0)] * (3 - len(rr))
             half[i] = [sum(v << (8 * n) for n, (v, _) in enumerate(rr)), sum(e << (8 * n) for n, (_, e) in enumerate(rr))]
         offs += [put(half), put(np.array([i | (j << 16) for i, j in pairs], np.int32))]
-        # F transposed, over the terms: fitted coefficient k takes sign * F_jk
-        # of every term of orbit j
-        by_k = [{} for _ in range(max((k for r in t.F for k in r), default=0) + 1)]
-        for q in range(t.nterms):
-            for k, f in t.F[int(t.k[q])].items():
-                by_k[k][q] = f * float(t.coef[q])
-        offs += [put(a) for a in csr(by_k + [{}] * (t.nfit - len(by_k)))]
+        # first term of every coefficient (the table is sorted by them), and F
+        # transposed
+        offs.append(put(np.searchsorted(t.k, np.arange(t.ncoef + 1)).astype(np.int32)))
+        by_k = [{} for _ in range(t.nfit)]
+        for j, row in enumerate(t.F):
+            for k, f in row.items():
+                by_k[k][j] = f
+        offs += [put(a) for a in csr(by_k)]
         index.append((tname, t.nterms, term_pairs_max(tname), t.ncoef, len(basis), offs))
     bin_path = os.path.join(OUT, "terms.bin")
     old = open(bin_path, "rb").read() if os.path.exists(bin_path) else None
@@ -1022,11 +1023,11 @@ def write_term_tables():
              "// term tables in terms.bin: name, number of terms, (variable, exponent) pairs per",
              "// term at most, coefficients in the w variables; byte offsets of the int4 terms, the",
              "// double signs, the rows of F (starts, columns, factors), of W and of its transpose",
-             "// (starts, signed columns), of w0, of the half-monomials, of the terms' pairs of them and of the",
-             "// terms of every fitted coefficient (starts, terms, factors)",
+             "// (starts, signed columns), of w0, of the half-monomials, of the terms' pairs of them, of the",
+             "// first term of every coefficient and of the rows of F transposed",
              "struct TermTableInfo { const char* name; long nterms; int pairs, ncw, nhalf; long off_terms, off_tcoef, "
              "off_frow, off_fk, off_ff, off_wrow, off_w, off_wtrow, off_wt, off_w0, off_half, off_pair, "
-             "off_ftrow, off_ftk, off_ftf; };",
+             "off_first, off_ftrow, off_ftk, off_ftf; };",
              "static const TermTableInfo mbx_term_tables[] = {"]
     for tname, nt, npair, ncw, nhalf, offs in index:
         lines.append('    {"%s", %d, %d, %d, %d, %s},' % (tname, nt, npair, ncw, nhalf, ", ".join(map(str, offs))))

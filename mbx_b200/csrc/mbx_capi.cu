@@ -52,10 +52,10 @@ int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double
 struct AdjointTable {
     const int4* terms;
     const double* tcoef;
-    int nterms, nhalf, nvars, ncoef;
+    int nterms, nhalf, nvars, ncoef, ncw;
     const int2* half;
     const unsigned* pair;
-    const int *ftrow, *ftk;
+    const int *first, *ftrow, *ftk;
     const double* ftf;
 };
 int mbx_coef_adjoint_blocks(const AdjointTable& P, int sms);
@@ -1803,14 +1803,15 @@ extern "C" int mbx_evaluate_dcoef(mbx_ctx* c, const char* name, long n, const do
         constexpr long kAdjointChunk = 32768;
         const TermTableInfo& T = mbx_term_tables[E->table];
         const int chunk = (int)std::min(n, kAdjointChunk);
-        const AdjointTable P{A.terms, A.tcoef, (int)A.nterms, T.nhalf, E->nvars, E->ncoef,
+        const AdjointTable P{A.terms, A.tcoef, (int)A.nterms, T.nhalf, E->nvars, E->ncoef, T.ncw,
                              reinterpret_cast<const int2*>(c->tables.blob + T.off_half),
                              reinterpret_cast<const unsigned*>(c->tables.blob + T.off_pair),
+                             reinterpret_cast<const int*>(c->tables.blob + T.off_first),
                              reinterpret_cast<const int*>(c->tables.blob + T.off_ftrow),
                              reinterpret_cast<const int*>(c->tables.blob + T.off_ftk),
                              reinterpret_cast<const double*>(c->tables.blob + T.off_ftf)};
         const size_t nv = (size_t)(E->nvars + 1) * chunk;
-        CUCHK(c, c->coef_ws.ensure(nv + (size_t)mbx_coef_adjoint_blocks(P, c->sm_count) * A.nterms + A.nterms));
+        CUCHK(c, c->coef_ws.ensure(nv + (size_t)mbx_coef_adjoint_blocks(P, c->sm_count) * A.nterms + A.nterms + T.ncw));
         for (long first = 0; first < n; first += chunk) {
             const int count = (int)std::min<long>(chunk, n - first);
             RCHK(c, E->c(A, W, first, count, c->coef_ws.p, c->stream));

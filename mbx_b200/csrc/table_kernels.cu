@@ -6,8 +6,8 @@
 // x[v * nd + i]; the per-configuration MB-nrg eval(a, x, g) programs are the
 // nd = 1 case), served for every evaluator from its term table in the w
 // variables (term_table.cuh) and the coefficients currently set on the
-// device: x is transformed to w, the gradient back.  A warp per configuration: lane l takes terms l, l+32, ...;
-// the configuration's variables and gradient accumulators sit in shared
+// device: x is transformed to w, the gradient back.  A warp per
+// configuration: lane l takes terms l, l+32, ...; the configuration's variables and gradient accumulators sit in shared
 // memory (gradient by shared-memory atomics), the energy is reduced across
 // the warp.
 #include <cuda_runtime.h>
@@ -103,9 +103,9 @@ int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double
 // go to shared memory once; then every thread multiplies the pairs of its own
 // MBX_ADJ_Q terms, and keeps one sum per term in registers over all of the
 // block's n-mers, so that nothing is reduced across threads.  The blocks' sums
-// are added up in a fixed order (adjoint_terms_kernel), and every fitted
-// coefficient takes the sums of its terms (adjoint_out_kernel): the result is
-// the same from call to call.  Bound by the shared-memory reads of two
+// are added up in a fixed order (adjoint_terms_kernel), then the terms of
+// every coefficient (adjoint_coef_kernel) and F^T of those
+// (adjoint_out_kernel): the result is the same from call to call.  Bound by the shared-memory reads of two
 // scattered doubles per term and n-mer: 20000 MB-pol 3b trimers (7425 terms)
 // 180 us, where walking the 33525 terms in x, a lane per n-mer, took 14 ms.
 #define MBX_ADJ_THREADS 512
@@ -115,10 +115,10 @@ int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double
 struct AdjointTable {
     const int4* terms;
     const double* tcoef;
-    int nterms, nhalf, nvars, ncoef;
+    int nterms, nhalf, nvars, ncoef, ncw;
     const int2* half;
     const unsigned* pair;
-    const int *ftrow, *ftk;   // terms of every fitted coefficient, and their factors
+    const int *first, *ftrow, *ftk;   // first term of every coefficient; rows of F transposed
     const double* ftf;
 };
 
@@ -194,13 +194,23 @@ __global__ void __launch_bounds__(256) adjoint_terms_kernel(const double* __rest
     }
 }
 
-// out[k] += sum over the terms of fitted coefficient k; a warp per coefficient.
-__global__ void __launch_bounds__(128) adjoint_out_kernel(const AdjointTable P, const double* __restrict__ sum,
+// dc[j] = signed sum over the terms of coefficient j.
+__global__ void __launch_bounds__(128) adjoint_coef_kernel(const AdjointTable P, const double* __restrict__ sum,
+                                                           double* __restrict__ dc) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= P.ncw) return;
+    double v = 0.0;
+    for (int t = P.first[j]; t < P.first[j + 1]; ++t) v = fma(P.tcoef[t], sum[t], v);
+    dc[j] = v;
+}
+
+// out += F^T dc; a warp per fitted coefficient.
+__global__ void __launch_bounds__(128) adjoint_out_kernel(const AdjointTable P, const double* __restrict__ dc,
                                                           double* __restrict__ out) {
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (k >= P.ncoef) return;
     double v = 0.0;
-    for (int q = P.ftrow[k] + lane; q < P.ftrow[k + 1]; q += 32) v = fma(P.ftf[q], sum[P.ftk[q]], v);
+    for (int q = P.ftrow[k] + lane; q < P.ftrow[k + 1]; q += 32) v = fma(P.ftf[q], dc[P.ftk[q]], v);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane == 0) out[k] += v;
@@ -218,7 +228,7 @@ int mbx_coef_adjoint_blocks(const AdjointTable& P, int sms) {
     return (2 * sms + ny - 1) / ny;
 }
 
-// work: (mbx_coef_adjoint_blocks + 1) * nterms doubles
+// work: (mbx_coef_adjoint_blocks + 1) * nterms + ncw doubles
 int mbx_launch_coef_adjoint(const double* wv, int count, const AdjointTable& P, double* work, double* out, int sms,
                             cudaStream_t s) {
     const size_t smem = ((size_t)(P.nvars + 1) * MBX_ADJ_N + 2 * (size_t)P.nhalf * (MBX_ADJ_N + 1)) * sizeof(double);
@@ -231,6 +241,8 @@ int mbx_launch_coef_adjoint(const double* wv, int count, const AdjointTable& P, 
     double* sum = work + (size_t)most * P.nterms;
     coef_adjoint_kernel<<<dim3(nx, adjoint_ranges(P)), MBX_ADJ_THREADS, smem, s>>>(wv, count, P, work);
     adjoint_terms_kernel<<<(P.nterms + 31) / 32, dim3(32, 8), 0, s>>>(work, nx, P.nterms, sum);
-    adjoint_out_kernel<<<(P.ncoef + 3) / 4, 128, 0, s>>>(P, sum, out);
+    double* dc = sum + P.nterms;
+    adjoint_coef_kernel<<<(P.ncw + 127) / 128, 128, 0, s>>>(P, sum, dc);
+    adjoint_out_kernel<<<(P.ncoef + 3) / 4, 128, 0, s>>>(P, dc, out);
     return (int)cudaGetLastError();
 }

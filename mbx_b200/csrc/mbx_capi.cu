@@ -355,11 +355,25 @@ struct BuildScratch {
         nb.release();
     }
 };
-// pinned result block (h_out, 64 doubles): [0..7) term energy + virial, [8]
-// listed n-mers, then the bucket counts (ints) and the status words (2 ints)
-#define MBX_H_COUNTS 9
-#define MBX_H_STATUS (MBX_H_COUNTS + (MBX_MAX_BUCKETS + 1) / 2)
-static_assert(MBX_H_STATUS + 1 <= 64, "pinned result block too small");
+// Control block of a term, one device buffer cleared by one memset and copied
+// back by one copy (offsets in doubles; h_out is its pinned mirror): energy +
+// virial, listed n-mers (2 counters), the bucket counts (ints) and the status
+// words (2 ints) are results; the work counters of the evaluation kernels
+// (ints) follow.
+#define MBX_CTL_OUT 0
+#define MBX_CTL_LISTED 16
+#define MBX_CTL_COUNTS 20
+#define MBX_CTL_STATUS (MBX_CTL_COUNTS + (MBX_MAX_BUCKETS + 1) / 2)
+#define MBX_CTL_RESULTS (MBX_CTL_STATUS + 2)
+#define MBX_CTL_COUNTERS MBX_CTL_RESULTS
+#define MBX_CTL_SIZE (MBX_CTL_COUNTERS + (MBX_MAX_BUCKETS + 1) / 2)
+static_assert(MBX_CTL_SIZE <= 64, "pinned result block too small");
+
+// A part of the control block.
+template <class T>
+struct CtlPart {
+    T* p = nullptr;
+};
 
 struct mbx_ctx {
     int device = 0;
@@ -402,8 +416,10 @@ struct mbx_ctx {
     long bucket_cap[4][MBX_MAX_BUCKETS];
 
     // work buffers
-    DevBuf<double> xyz, grad, out, coef_ws;
-    DevBuf<int> bucket_count, status, counters;
+    DevBuf<double> xyz, grad, ctl, coef_ws;
+    CtlPart<double> out;
+    CtlPart<int> bucket_count, status, counters;
+    CtlPart<unsigned long long> listed;
     BuildScratch scratch;   // of every search (a batch searches all its configurations at once)
     // code prefetch of a term's evaluation kernels, beside its n-mer search
     cudaStream_t prime_stream = nullptr;
@@ -414,7 +430,6 @@ struct mbx_ctx {
     unsigned long gen = 0, child_gen = ~0ul;
     cudaEvent_t ev_fork = nullptr;
     DevBuf<int4> buckets, list;
-    DevBuf<unsigned long long> listed;
     DeviceTables tables;   // per-device term tables and coefficients (shared, not owned)
     DevBuf<unsigned char> pair_scratch;   // between the three mixed-precision kernels
     int nb_cap = 192;
@@ -422,7 +437,7 @@ struct mbx_ctx {
     struct Knobs {
         int nb_warps = 4, nb_unroll = 2, tri_threads = 128, dim_threads = 128;
     } knobs[4];         // per term (indexed by nbody)
-    double* h_out = nullptr;  // pinned: [0..7] term outputs, [8..15] counters
+    double* h_out = nullptr;  // pinned mirror of the control block's results
     double* h_grad = nullptr;  // pinned staging of the gradient of a call with host arrays
     size_t h_grad_n = 0;
     cudaEvent_t ev[3];
@@ -507,10 +522,12 @@ int mbx_create(mbx_ctx** out, int device, void* stream) {
     CUCHK(c, cudaEventCreateWithFlags(&c->prime_fork, cudaEventDisableTiming));
     CUCHK(c, cudaEventCreateWithFlags(&c->prime_join, cudaEventDisableTiming));
 
-    CUCHK(c, c->out.ensure(64));
-    CUCHK(c, c->status.ensure(4));
-    CUCHK(c, c->counters.ensure(MBX_MAX_BUCKETS));
-    CUCHK(c, c->listed.ensure(4));
+    CUCHK(c, c->ctl.ensure(64));
+    c->out.p = c->ctl.p + MBX_CTL_OUT;
+    c->listed.p = reinterpret_cast<unsigned long long*>(c->ctl.p + MBX_CTL_LISTED);
+    c->bucket_count.p = reinterpret_cast<int*>(c->ctl.p + MBX_CTL_COUNTS);
+    c->status.p = reinterpret_cast<int*>(c->ctl.p + MBX_CTL_STATUS);
+    c->counters.p = reinterpret_cast<int*>(c->ctl.p + MBX_CTL_COUNTERS);
     for (int nb = 0; nb < 4; ++nb)
         for (int b = 0; b < MBX_MAX_BUCKETS; ++b) c->bucket_cap[nb][b] = 0;
     // the fitted coefficients (constant banks, per device: loaded by the
@@ -532,9 +549,9 @@ int mbx_destroy(mbx_ctx* c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     DevBuf<int>* ib[] = {&c->d_first, &c->d_nat, &c->d_tag, &c->d_type, &c->d_members[0], &c->d_members[1],
-                         &c->d_query[0], &c->d_query[1], &c->bucket_count, &c->status, &c->counters};
+                         &c->d_query[0], &c->d_query[1]};
     for (auto* b : ib) b->release();
-    DevBuf<double>* db[] = {&c->xyz, &c->grad, &c->out, &c->coef_ws};
+    DevBuf<double>* db[] = {&c->xyz, &c->grad, &c->ctl, &c->coef_ws};
     for (auto* b : db) b->release();
     c->scratch.release();
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -548,7 +565,6 @@ int mbx_destroy(mbx_ctx* c) {
     c->pair_scratch.release();
     c->buckets.release();
     c->list.release();
-    c->listed.release();
     c->d_conf_bp.release();
     c->d_mon_conf.release();
     for (auto& g : c->d_bgrid) g.release();
@@ -838,6 +854,17 @@ static CellGrid make_grid(const BoxParams& bp, double rc, int nmem) {
                              vol / std::sqrt(ca[0] * ca[0] + ca[1] * ca[1] + ca[2] * ca[2]),
                              vol / std::sqrt(ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2])};
         for (int k = 0; k < 3; ++k) g.n[k] = std::max(1, std::min(64, (int)std::floor(h[k] / rc)));
+        // GetFractionalCoordinates (kdtree/kdtree_utils.h:165-190): its
+        // factors, which depend on the box alone
+        const double A = a[0], B = std::sqrt(b[0] * b[0] + b[1] * b[1]);
+        const double C = std::sqrt(cc[0] * cc[0] + cc[1] * cc[1] + cc[2] * cc[2]);
+        const double gamma = std::acos(a[0] * b[0] / A / B), beta = std::acos(a[0] * cc[0] / A / C);
+        const double alpha = std::acos((b[0] * cc[0] + b[1] * cc[1]) / B / C);
+        const double x = std::cos(alpha), y = std::cos(beta), z = std::cos(gamma), sz = std::sin(gamma);
+        const double omega = A * B * C * std::sqrt(1 - x * x - y * y - z * z + 2 * x * y * z);
+        const double f[6] = {1 / A, z / A / sz, B * C * (x * z - y) / omega / sz, 1 / B / sz,
+                             A * C * (y * z - x) / omega / sz, A * B * sz / omega};
+        for (int k = 0; k < 6; ++k) g.frac[k] = f[k];
         // one cloud point per candidate when every axis has 3 or more cells,
         // each wider than the cutoff by a margin far above rounding (the
         // search then tests only the copy the cell's wrap implies)
@@ -849,7 +876,6 @@ static CellGrid make_grid(const BoxParams& bp, double rc, int nmem) {
         const int n = std::max(3, std::min(32, (int)std::ceil(std::cbrt((double)nmem / 2.0))));
         for (int k = 0; k < 3; ++k) {
             g.n[k] = n;
-            g.lo[k] = rc;
             g.inv_extent[k] = 1.0 / rc;
         }
     }
@@ -857,9 +883,8 @@ static CellGrid make_grid(const BoxParams& bp, double rc, int nmem) {
 }
 
 // Bucket capacities (grown on overflow; first guess from the query count)
-// and offsets of one term; zeroes the bucket counters and the status word.
+// and offsets of one term; zeroes the control block.
 static int prepare_buckets(mbx_ctx* c, int nbody, long nq_guess, long list_cap) {
-    CUCHK(c, c->bucket_count.ensure(MBX_MAX_BUCKETS));
     long total = 0;
     for (int b = 0; b < c->nbucket[nbody]; ++b) {
         if (c->bucket_cap[nbody][b] == 0) c->bucket_cap[nbody][b] = std::max(nq_guess, 1L) * (nbody == 2 ? 40 : 80);
@@ -873,11 +898,14 @@ static int prepare_buckets(mbx_ctx* c, int nbody, long nq_guess, long list_cap) 
         off += c->bucket_cap[nbody][b];
     }
     if (list_cap > 0) CUCHK(c, c->list.ensure(list_cap));
-    CUCHK(c, cudaMemsetAsync(c->bucket_count.p, 0, MBX_MAX_BUCKETS * sizeof(int), c->stream));
-    CUCHK(c, cudaMemsetAsync(c->listed.p, 0, 4 * sizeof(unsigned long long), c->stream));
-    CUCHK(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
+    CUCHK(c, cudaMemsetAsync(c->ctl.p, 0, MBX_CTL_SIZE * sizeof(double), c->stream));
     return MBX_OK;
 }
+
+// Searches up to this many members and cells build their cell list in one
+// block (k_cells_small): the launches between four kernels cost more than the
+// other SMs would save.
+constexpr int kSmallSearch = 1024;
 
 // One search: the monomers members[0..nmem) (global ids) searched around
 // the queries query[0..nq) (positions in members), in box bp.
@@ -912,15 +940,22 @@ static int launch_build_scope(mbx_ctx* c, int nbody, const BuildScope& S, const 
     CUCHK(c, B.cell_fill.ensure(ncell + 1));
     CUCHK(c, B.nb_count.ensure(std::max(nq, 1)));
     CUCHK(c, B.nb.ensure((size_t)std::max(nq, 1) * c->nb_cap));
-    CUCHK(c, cudaMemsetAsync(B.cell_count.p, 0, (ncell + 1) * sizeof(int), st));
     const int T = 128;
-    k_cloud<<<(nmem + T - 1) / T, T, 0, st>>>(xyz, c->d_first.p, S.members, nmem, S.bp, cg, B.cloud.p,
-                                                     B.cell_of.p, B.copy_dir.p);
-    k_cell_count<<<(nmem + T - 1) / T, T, 0, st>>>(B.cell_of.p, nmem, B.cell_count.p);
-    k_cell_scan<<<1, 1024, 0, st>>>(B.cell_count.p, ncell, B.cell_start.p, B.cell_fill.p);
-    k_cell_fill<<<(nmem + T - 1) / T, T, 0, st>>>(B.cell_of.p, nmem, B.cell_fill.p, B.cell_items.p);
-    k_cell_sort<<<(ncell * 32 + T - 1) / T, T, 0, st>>>(B.cell_start.p, ncell, B.cell_items.p,
-                                                                B.cell_sorted.p);
+    if (nmem <= kSmallSearch && ncell <= kSmallSearch) {
+        // the whole cell list in one block
+        k_cells_small<<<1, 1024, 0, st>>>(xyz, c->d_first.p, S.members, nmem, S.bp, cg, ncell, B.cloud.p, B.cell_of.p,
+                                          B.copy_dir.p, B.cell_count.p, B.cell_start.p, B.cell_fill.p, B.cell_items.p,
+                                          B.cell_sorted.p);
+        *kernels += 1;
+    } else {
+        CUCHK(c, cudaMemsetAsync(B.cell_count.p, 0, (ncell + 1) * sizeof(int), st));
+        k_cloud<<<(nmem + T - 1) / T, T, 0, st>>>(xyz, c->d_first.p, S.members, nmem, S.bp, cg, B.cloud.p, B.cell_of.p,
+                                                  B.copy_dir.p, B.cell_count.p);
+        k_cell_scan<<<1, 1024, 0, st>>>(B.cell_count.p, ncell, B.cell_start.p, B.cell_fill.p);
+        k_cell_fill<<<(nmem + T - 1) / T, T, 0, st>>>(B.cell_of.p, nmem, B.cell_fill.p, B.cell_items.p);
+        k_cell_sort<<<(ncell * 32 + T - 1) / T, T, 0, st>>>(B.cell_start.p, ncell, B.cell_items.p, B.cell_sorted.p);
+        *kernels += 4;
+    }
     // neighbour search: warps per query and unroll depth are tunable; one
     // warp when four staging areas would not fit in shared memory
     const auto& K = c->knobs[nbody];
@@ -949,7 +984,7 @@ static int launch_build_scope(mbx_ctx* c, int nbody, const BuildScope& S, const 
             c->status.p);
     }
     CUCHK(c, cudaGetLastError());
-    *kernels += 8;
+    *kernels += 2;
     return MBX_OK;
 }
 
@@ -1020,8 +1055,7 @@ static int launch_build_batch(mbx_ctx* c, int nbody, const double* xyz, int* ker
     CUCHK(c, cudaMemsetAsync(B.cell_count.p, 0, (ncell + 1) * sizeof(int), st));
     const int T = 128;
     k_cloud_batch<<<(nmem + T - 1) / T, T, 0, st>>>(xyz, c->d_first.p, nmem, c->d_mon_conf.p, c->d_bgrid[nbody].p,
-                                                    B.cloud.p, B.cell_of.p, B.copy_dir.p);
-    k_cell_count<<<(nmem + T - 1) / T, T, 0, st>>>(B.cell_of.p, nmem, B.cell_count.p);
+                                                    B.cloud.p, B.cell_of.p, B.copy_dir.p, B.cell_count.p);
     k_cell_scan<<<1, 1024, 0, st>>>(B.cell_count.p, ncell, B.cell_start.p, B.cell_fill.p);
     k_cell_fill<<<(nmem + T - 1) / T, T, 0, st>>>(B.cell_of.p, nmem, B.cell_fill.p, B.cell_items.p);
     k_cell_sort<<<(int)(((long)ncell * 32 + T - 1) / T), T, 0, st>>>(B.cell_start.p, ncell, B.cell_items.p,
@@ -1051,7 +1085,7 @@ static int launch_build_batch(mbx_ctx* c, int nbody, const double* xyz, int* ker
                                                     c->buckets.p, c->bucket_count.p, c->status.p);
     }
     CUCHK(c, cudaGetLastError());
-    *kernels += 8;
+    *kernels += 6;
     return MBX_OK;
 }
 
@@ -1110,17 +1144,20 @@ static int launch_eval(mbx_ctx* c, const EvaluatorInfo* E, HolderArgs A, int fla
     return MBX_OK;
 }
 
-// Code prefetch (holder_prime_kernel) of the evaluation kernels that a term's
-// buckets will launch, forked from the context stream onto the prime stream
-// so that it runs beside the n-mer search; prime_join marks its end and the
-// first evaluation waits for it.  Same kernel choice as launch_eval.
-static int launch_prime(mbx_ctx* c, int nbody, int flags, int* kernels) {
+// Code prefetch of the evaluation kernels that a term's buckets will launch
+// (prime_pieces), on the prime stream beside the n-mer search.  It reads and
+// writes no data, so nothing waits for it, except in a graph capture (capture),
+// where the prime stream has to be forked from the context's stream and joined
+// again (prime_join).  Same kernel choice as launch_eval.
+static int launch_prime(mbx_ctx* c, int nbody, int flags, int* kernels, bool capture = false) {
     const bool grads = !(flags & MBX_NO_GRADS);
     const bool mixed = (flags & MBX_MIXED) != 0;
     prime_fn done[MBX_MAX_BUCKETS];
     int ndone = 0;
-    CUCHK(c, cudaEventRecord(c->prime_fork, c->stream));
-    CUCHK(c, cudaStreamWaitEvent(c->prime_stream, c->prime_fork, 0));
+    if (capture) {
+        CUCHK(c, cudaEventRecord(c->prime_fork, c->stream));
+        CUCHK(c, cudaStreamWaitEvent(c->prime_stream, c->prime_fork, 0));
+    }
     for (int b = 0; b < c->nbucket[nbody]; ++b) {
         const bool near = c->bucket_near[nbody][b];
         if (near && !mixed) continue;
@@ -1132,7 +1169,7 @@ static int launch_prime(mbx_ctx* c, int nbody, int flags, int* kernels) {
         RCHK(c, fn(c->prime_stream));
         ++*kernels;
     }
-    CUCHK(c, cudaEventRecord(c->prime_join, c->prime_stream));
+    if (capture) CUCHK(c, cudaEventRecord(c->prime_join, c->prime_stream));
     return MBX_OK;
 }
 
@@ -1147,10 +1184,7 @@ static int term_enqueue(mbx_ctx* c, int nbody, int use_ghost, double* X, double*
     if (r) return r;
     r = launch_build(c, nbody, use_ghost, X, 0, kernels, mixed);
     if (r) return r;
-    CUCHK(c, cudaStreamWaitEvent(c->stream, c->prime_join, 0));
     CUCHK(c, cudaEventRecord(c->ev[1], c->stream));
-    CUCHK(c, cudaMemsetAsync(c->out.p, 0, 16 * sizeof(double), c->stream));
-    CUCHK(c, cudaMemsetAsync(c->counters.p, 0, MBX_MAX_BUCKETS * sizeof(int), c->stream));
     long off = 0;
     for (int b = 0; b < c->nbucket[nbody]; ++b) {
         HolderArgs A = base_args(c);
@@ -1169,13 +1203,7 @@ static int term_enqueue(mbx_ctx* c, int nbody, int use_ghost, double* X, double*
         if (r) return r;
     }
     CUCHK(c, cudaEventRecord(c->ev[2], c->stream));
-    // results: energy + virial, counters, status
-    CUCHK(c, cudaMemcpyAsync(c->h_out, c->out.p, 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->h_out + 8, c->listed.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                             c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->h_out + MBX_H_COUNTS, c->bucket_count.p, MBX_MAX_BUCKETS * sizeof(int), cudaMemcpyDeviceToHost,
-                             c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->h_out + MBX_H_STATUS, c->status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CUCHK(c, cudaMemcpyAsync(c->h_out, c->ctl.p, MBX_CTL_RESULTS * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     return MBX_OK;
 }
 
@@ -1186,9 +1214,9 @@ static int term_enqueue(mbx_ctx* c, int nbody, int use_ghost, double* X, double*
 // and the timing recorded.
 static int term_finish(mbx_ctx* c, int nbody, double* energy, double* virial, int kernels) {
     int status[2];
-    memcpy(status, c->h_out + MBX_H_STATUS, sizeof(status));
+    memcpy(status, c->h_out + MBX_CTL_STATUS, sizeof(status));
     int counts[MBX_MAX_BUCKETS];
-    memcpy(counts, c->h_out + MBX_H_COUNTS, sizeof(counts));
+    memcpy(counts, c->h_out + MBX_CTL_COUNTS, sizeof(counts));
     if (status[0] & MBX_STATUS_WAIT_TIMEOUT)
         return -fail(c, MBX_ECUDA, "an evaluation kernel's barrier wait timed out (results discarded)");
     if (status[0]) {
@@ -1202,7 +1230,7 @@ static int term_finish(mbx_ctx* c, int nbody, double* energy, double* virial, in
         return 1;
     }
     unsigned long long listed;
-    memcpy(&listed, c->h_out + 8, sizeof(listed));
+    memcpy(&listed, c->h_out + MBX_CTL_LISTED, sizeof(listed));
     c->last_listed[nbody] = (long)listed;
     long ev = 0;
     for (int b = 0; b < c->nbucket[nbody]; ++b) ev += counts[b];
@@ -1718,8 +1746,7 @@ extern "C" int mbx_evaluate(mbx_ctx* c, const char* name, long n, const double* 
             EP = e_buf.p;
         }
     }
-    CUCHK(c, cudaMemsetAsync(c->out.p, 0, 16 * sizeof(double), c->stream));
-    CUCHK(c, cudaMemsetAsync(c->counters.p, 0, sizeof(int), c->stream));
+    CUCHK(c, cudaMemsetAsync(c->ctl.p, 0, MBX_CTL_SIZE * sizeof(double), c->stream));
     HolderArgs A = base_args(c);
     A.counter = c->counters.p;
     A.bp.use_pbc = 0;
@@ -1730,15 +1757,13 @@ extern "C" int mbx_evaluate(mbx_ctx* c, const char* name, long n, const double* 
     A.out = c->out.p;
     A.e_per = EP;
     int kernels = 0;
-    CUCHK(c, cudaMemsetAsync(c->status.p, 0, sizeof(int), c->stream));
     CUCHK(c, cudaEventRecord(c->ev[1], c->stream));
     if (n > 0) {
         r = launch_eval(c, E, A, grads ? (flags & MBX_MIXED) : (flags | MBX_NO_GRADS), &kernels);
         if (r) return r;
     }
     CUCHK(c, cudaEventRecord(c->ev[2], c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->h_out, c->out.p, 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->h_out + MBX_H_STATUS, c->status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CUCHK(c, cudaMemcpyAsync(c->h_out, c->ctl.p, MBX_CTL_RESULTS * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     std::vector<double> gt, et;
     if (grads && !dev) {
         gt.resize(nx);
@@ -1747,7 +1772,7 @@ extern "C" int mbx_evaluate(mbx_ctx* c, const char* name, long n, const double* 
     if (e_per && !dev && n > 0) CUCHK(c, cudaMemcpyAsync(e_per, EP, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CUCHK(c, cudaStreamSynchronize(c->stream));
     int status0;
-    memcpy(&status0, c->h_out + MBX_H_STATUS, sizeof(int));
+    memcpy(&status0, c->h_out + MBX_CTL_STATUS, sizeof(int));
     if (status0 & MBX_STATUS_WAIT_TIMEOUT)
         return fail(c, MBX_ECUDA, "an evaluation kernel's barrier wait timed out (results discarded)");
     if (grads && !dev)
@@ -1983,15 +2008,13 @@ static int batch_sequence(mbx_ctx* c, int nbody, double* X, double* G, bool grad
     }
     int r = prepare_buckets(c, nbody, c->nmon, 0);
     if (r) return r;
-    r = launch_prime(c, nbody, (mixed ? MBX_MIXED : 0) | (grads ? 0 : MBX_NO_GRADS), kernels);
+    r = launch_prime(c, nbody, (mixed ? MBX_MIXED : 0) | (grads ? 0 : MBX_NO_GRADS), kernels, true);
     if (r) return r;
     // every configuration's search in one set of launches
     r = launch_build_batch(c, nbody, X, kernels, mixed);
     if (r) return r;
     CUCHK(c, cudaStreamWaitEvent(c->stream, c->prime_join, 0));
     CUCHK(c, cudaMemsetAsync(c->conf_out.p, 0, 8 * (size_t)c->nconf * sizeof(double), c->stream));
-    CUCHK(c, cudaMemsetAsync(c->out.p, 0, 16 * sizeof(double), c->stream));
-    CUCHK(c, cudaMemsetAsync(c->counters.p, 0, MBX_MAX_BUCKETS * sizeof(int), c->stream));
     long off = 0;
     for (int b = 0; b < c->nbucket[nbody]; ++b) {
         HolderArgs A = base_args(c);
@@ -2015,11 +2038,7 @@ static int batch_sequence(mbx_ctx* c, int nbody, double* X, double* G, bool grad
     }
     CUCHK(c, cudaMemcpyAsync(c->h_conf, c->conf_out.p, 8 * (size_t)c->nconf * sizeof(double), cudaMemcpyDeviceToHost,
                              c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->h_out + 8, c->listed.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                             c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->h_out + MBX_H_COUNTS, c->bucket_count.p, MBX_MAX_BUCKETS * sizeof(int), cudaMemcpyDeviceToHost,
-                             c->stream));
-    CUCHK(c, cudaMemcpyAsync(c->h_out + MBX_H_STATUS, c->status.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CUCHK(c, cudaMemcpyAsync(c->h_out, c->ctl.p, MBX_CTL_RESULTS * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     return MBX_OK;
 }
 
@@ -2028,9 +2047,9 @@ static int batch_sequence(mbx_ctx* c, int nbody, double* X, double* G, bool grad
 // capacities are grown and 1 is returned (run it again).
 static int batch_check(mbx_ctx* c, int nbody) {
     int status[2];
-    memcpy(status, c->h_out + MBX_H_STATUS, sizeof(status));
+    memcpy(status, c->h_out + MBX_CTL_STATUS, sizeof(status));
     int counts[MBX_MAX_BUCKETS];
-    memcpy(counts, c->h_out + MBX_H_COUNTS, sizeof(counts));
+    memcpy(counts, c->h_out + MBX_CTL_COUNTS, sizeof(counts));
     if (status[0] & MBX_STATUS_WAIT_TIMEOUT)
         return -fail(c, MBX_ECUDA, "an evaluation kernel's barrier wait timed out (results discarded)");
     if (status[0]) {
@@ -2043,7 +2062,7 @@ static int batch_check(mbx_ctx* c, int nbody) {
         return 1;
     }
     unsigned long long listed;
-    memcpy(&listed, c->h_out + 8, sizeof(listed));
+    memcpy(&listed, c->h_out + MBX_CTL_LISTED, sizeof(listed));
     c->last_listed[nbody] = (long)listed;
     long ev = 0;
     for (int b = 0; b < c->nbucket[nbody]; ++b) ev += counts[b];

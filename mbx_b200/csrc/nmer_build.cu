@@ -34,19 +34,13 @@ __device__ __forceinline__ double dist2_rn(double a0, double a1, double a2, doub
     return __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
 }
 
-// GetFractionalCoordinates (kdtree/kdtree_utils.h:165-190); only the signs of
-// its results matter (they choose which periodic copies exist).
-__device__ void frac_coords(const double* box, const double (&pt)[3], double (&c)[3]) {
-    const double A = box[0];
-    const double B = sqrt(box[3] * box[3] + box[4] * box[4]);
-    const double C = sqrt(box[6] * box[6] + box[7] * box[7] + box[8] * box[8]);
-    const double AdotB = box[0] * box[3], AdotC = box[0] * box[6], BdotC = box[3] * box[6] + box[4] * box[7];
-    const double gamma = acos(AdotB / A / B), beta = acos(AdotC / A / C), alpha = acos(BdotC / B / C);
-    const double ca = cos(alpha), cb = cos(beta), cg = cos(gamma), sg = sin(gamma);
-    const double omega = A * B * C * sqrt(1 - ca * ca - cb * cb - cg * cg + 2 * ca * cb * cg);
-    c[0] = 1 / A * pt[0] - cg / A / sg * pt[1] + B * C * (ca * cg - cb) / omega / sg * pt[2];
-    c[1] = 1 / B / sg * pt[1] + A * C * (cb * cg - ca) / omega / sg * pt[2];
-    c[2] = A * B * sg / omega * pt[2];
+// GetFractionalCoordinates (kdtree/kdtree_utils.h:165-190) from the box's
+// factors (CellGrid::frac); only the signs of its results matter (they choose
+// which periodic copies exist).
+__device__ __forceinline__ void frac_coords(const double (&f)[6], const double (&pt)[3], double (&c)[3]) {
+    c[0] = __dadd_rn(__dsub_rn(__dmul_rn(f[0], pt[0]), __dmul_rn(f[1], pt[1])), __dmul_rn(f[2], pt[2]));
+    c[1] = __dadd_rn(__dmul_rn(f[3], pt[1]), __dmul_rn(f[4], pt[2]));
+    c[2] = __dmul_rn(f[5], pt[2]);
 }
 
 }  // namespace
@@ -100,7 +94,7 @@ __device__ __forceinline__ int cloud_point(const double* __restrict__ xyz, const
         f[2] = __dsub_rn(f[2], floor(__dadd_rn(f[2], 0.5)));
         to_cart_rn(bp.box, f, p);
         double uvw[3];
-        frac_coords(bp.box, p, uvw);
+        frac_coords(cg.frac, p, uvw);
         // per axis: the copy at -1 exists if uvw > 0, at +1 if uvw < 0; at
         // uvw == 0 both are made and the +1 copy overwrites (loop order 0,-1,1)
         int sgn[3];
@@ -149,34 +143,36 @@ __device__ __forceinline__ int cloud_point(const double* __restrict__ xyz, const
 
 __global__ void k_cloud(const double* __restrict__ xyz, const int* __restrict__ first_index,
                         const int* __restrict__ members, int nmem, BoxParams bp, CellGrid cg,
-                        double* __restrict__ cloud, int* __restrict__ cell_of, int* __restrict__ copy_dir) {
+                        double* __restrict__ cloud, int* __restrict__ cell_of, int* __restrict__ copy_dir,
+                        int* __restrict__ cell_count) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nmem) return;
     int dir;
-    cell_of[q] = cloud_point(xyz, first_index, members[q], q, bp, cg, cloud, dir);
+    const int cell = cloud_point(xyz, first_index, members[q], q, bp, cg, cloud, dir);
+    cell_of[q] = cell;
     copy_dir[q] = dir;
+    atomicAdd(cell_count + cell, 1);
 }
 
 __global__ void k_cloud_batch(const double* __restrict__ xyz, const int* __restrict__ first_index, int nmem,
                               const int* __restrict__ conf_of, const BatchGrid* __restrict__ grids,
-                              double* __restrict__ cloud, int* __restrict__ cell_of, int* __restrict__ copy_dir) {
+                              double* __restrict__ cloud, int* __restrict__ cell_of, int* __restrict__ copy_dir,
+                              int* __restrict__ cell_count) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nmem) return;
     const BatchGrid& G = grids[conf_of[q]];
     int dir;
-    cell_of[q] = G.cell_off + cloud_point(xyz, first_index, q, q, G.bp, G.cg, cloud, dir);
+    const int cell = G.cell_off + cloud_point(xyz, first_index, q, q, G.bp, G.cg, cloud, dir);
+    cell_of[q] = cell;
     copy_dir[q] = dir;
+    atomicAdd(cell_count + cell, 1);
 }
 
+namespace {
 
-__global__ void k_cell_count(const int* __restrict__ cell_of, int nmem, int* __restrict__ cell_count) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < nmem) atomicAdd(cell_count + cell_of[q], 1);
-}
-
-// Exclusive scan of the cell counts in one block (cell grids here are small).
-__global__ void k_cell_scan(const int* __restrict__ cell_count, int ncell, int* __restrict__ cell_start,
-                            int* __restrict__ cell_fill) {
+// Exclusive scan of the cell counts by one block of 1024 threads (cell grids
+// here are small).
+__device__ __forceinline__ void scan_cells(const int* cell_count, int ncell, int* cell_start, int* cell_fill) {
     __shared__ int warp_sums[32];
     __shared__ int carry;
     if (threadIdx.x == 0) carry = 0;
@@ -213,21 +209,12 @@ __global__ void k_cell_scan(const int* __restrict__ cell_count, int ncell, int* 
     if (threadIdx.x == 0) cell_start[ncell] = carry;
 }
 
-__global__ void k_cell_fill(const int* __restrict__ cell_of, int nmem, int* __restrict__ cell_fill,
-                            int* __restrict__ cell_items) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < nmem) cell_items[atomicAdd(cell_fill + cell_of[q], 1)] = q;
-}
-
-// The items of every cell in ascending order (k_cell_fill places them in
-// atomic order): the neighbour lists, and with them the slot order of every
-// n-mer, are then the same from run to run.  One warp per cell; an item's
-// place is the number of smaller items of its cell (all items differ).
-__global__ void k_cell_sort(const int* __restrict__ cell_start, int ncell, const int* __restrict__ items,
-                            int* __restrict__ sorted) {
+// The items of cell c in ascending order (they are placed in atomic order):
+// the neighbour lists, and with them the slot order of every n-mer, are then
+// the same from run to run.  One warp; an item's place is the number of
+// smaller items of its cell (all items differ).
+__device__ __forceinline__ void sort_cell(int c, const int* cell_start, const int* items, int* sorted) {
     const int lane = threadIdx.x & 31;
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (c >= ncell) return;
     const int b = cell_start[c], n = cell_start[c + 1] - b;
     for (int i0 = 0; i0 < n; i0 += 32) {
         const int i = i0 + lane;
@@ -236,6 +223,46 @@ __global__ void k_cell_sort(const int* __restrict__ cell_start, int ncell, const
         for (int j = 0; j < n; ++j) rank += items[b + j] < v;
         if (i < n) sorted[b + rank] = v;
     }
+}
+
+}  // namespace
+
+__global__ void k_cell_scan(const int* __restrict__ cell_count, int ncell, int* __restrict__ cell_start,
+                            int* __restrict__ cell_fill) {
+    scan_cells(cell_count, ncell, cell_start, cell_fill);
+}
+
+__global__ void k_cell_fill(const int* __restrict__ cell_of, int nmem, int* __restrict__ cell_fill,
+                            int* __restrict__ cell_items) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < nmem) cell_items[atomicAdd(cell_fill + cell_of[q], 1)] = q;
+}
+
+__global__ void k_cell_sort(const int* __restrict__ cell_start, int ncell, const int* __restrict__ items,
+                            int* __restrict__ sorted) {
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (c < ncell) sort_cell(c, cell_start, items, sorted);
+}
+
+__global__ void __launch_bounds__(1024) k_cells_small(const double* xyz, const int* first_index, const int* members,
+                                                      int nmem, BoxParams bp, CellGrid cg, int ncell, double* cloud,
+                                                      int* cell_of, int* copy_dir, int* cell_count, int* cell_start,
+                                                      int* cell_fill, int* cell_items, int* cell_sorted) {
+    for (int i = threadIdx.x; i < ncell; i += blockDim.x) cell_count[i] = 0;
+    __syncthreads();
+    for (int q = threadIdx.x; q < nmem; q += blockDim.x) {
+        int dir;
+        const int cell = cloud_point(xyz, first_index, members[q], q, bp, cg, cloud, dir);
+        cell_of[q] = cell;
+        copy_dir[q] = dir;
+        atomicAdd(cell_count + cell, 1);
+    }
+    __syncthreads();
+    scan_cells(cell_count, ncell, cell_start, cell_fill);
+    __syncthreads();
+    for (int q = threadIdx.x; q < nmem; q += blockDim.x) cell_items[atomicAdd(cell_fill + cell_of[q], 1)] = q;
+    __syncthreads();
+    for (int c = threadIdx.x >> 5; c < ncell; c += blockDim.x >> 5) sort_cell(c, cell_start, cell_items, cell_sorted);
 }
 
 // Matches of one query monomer: NW warps of a block split the 27 surrounding

@@ -23,8 +23,8 @@ struct CellGrid {
     int n[3];
     int one_copy;          // PBC, n >= 3 on every axis and cells wider than the cutoff (with a margin):
                            // of a member's eight cloud points only the one its cell's wrap implies can match
-    double lo[3];          // unused
     double inv_extent[3];  // no PBC: 1 / cell edge of the hashed grid
+    double frac[6];        // PBC: factors of GetFractionalCoordinates (k_cloud)
 };
 
 struct NbEntry {
@@ -63,12 +63,16 @@ struct BatchGrid {
 
 __global__ void k_fix_monomers(double* xyz, const int* first_index, const int* nat, int nmon, BoxParams bp);
 __global__ void k_cloud(const double* xyz, const int* first_index, const int* members, int nmem, BoxParams bp,
-                        CellGrid cg, double* cloud, int* cell_of, int* copy_dir);
+                        CellGrid cg, double* cloud, int* cell_of, int* copy_dir, int* cell_count);
+// k_cloud and the cell kernels below for a small search (nmem members, ncell
+// cells), in one block.
+__global__ void k_cells_small(const double* xyz, const int* first_index, const int* members, int nmem, BoxParams bp,
+                              CellGrid cg, int ncell, double* cloud, int* cell_of, int* copy_dir, int* cell_count,
+                              int* cell_start, int* cell_fill, int* cell_items, int* cell_sorted);
 // The same for a batch: members are the batch's monomers in order (member
 // position = monomer), each with the grid of its configuration conf_of[q].
 __global__ void k_cloud_batch(const double* xyz, const int* first_index, int nmem, const int* conf_of,
-                              const BatchGrid* grids, double* cloud, int* cell_of, int* copy_dir);
-__global__ void k_cell_count(const int* cell_of, int nmem, int* cell_count);
+                              const BatchGrid* grids, double* cloud, int* cell_of, int* copy_dir, int* cell_count);
 __global__ void k_cell_scan(const int* cell_count, int ncell, int* cell_start, int* cell_fill);
 __global__ void k_cell_fill(const int* cell_of, int nmem, int* cell_fill, int* cell_items);
 __global__ void k_cell_sort(const int* cell_start, int ncell, const int* items, int* sorted);

@@ -116,19 +116,31 @@ QF_TYPES = {"mbpol3b"}
 MIXED_FP64_RADIUS = {}
 
 
-def coef_expr(coefs, fp32=False):
-    """Sum of coef[k]*c for the terms ending exactly at a node (FP32: the
-    float copy of the coefficients, coef.f(k))."""
-    parts = []
-    for k, c in coefs:
-        ref = ("coef.f(%d)" if fp32 else "coef[%d]") % k
-        if c == 1.0:
-            parts.append(ref)
-        elif c == -1.0:
-            parts.append("(-%s)" % ref)
-        else:
-            parts.append("(%s * %s)" % (ref, lit(c) + ("f" if fp32 else "")))
-    return " + ".join(parts) if parts else None
+# Terms up to which a trie reads its coefficients in the order of its leaves
+# (one constant per leaf, sign included: consecutive constants, fetched in
+# pairs) instead of one per orbit; a unit's constant memory holds 8192 doubles.
+LEAF_ORDER_TERMS = 8000
+
+
+class Coefficients:
+    """Names of the coefficients in a trie's code: coef[orbit], or coef[i] in
+    the order of emission (leaves lists the (orbit, sign) of every i)."""
+
+    def __init__(self, by_leaf):
+        self.by_leaf = by_leaf
+        self.leaves = []
+
+    def __call__(self, coefs):
+        """Sum of the coefficients of the terms ending at a node, None without one."""
+        parts = []
+        for k, c in coefs:
+            assert c in (1.0, -1.0)
+            if self.by_leaf:
+                parts.append("coef[%d]" % len(self.leaves))
+                self.leaves.append((k, c))
+            else:
+                parts.append("coef[%d]" % k if c > 0 else "(-coef[%d])" % k)
+        return " + ".join(parts) if parts else None
 
 
 def split_terms(trie, nparts):
@@ -187,7 +199,7 @@ def parts_for(nterms, nvars=36):
     return max(1, (nterms + per - 1) // per)
 
 
-def emit_split(trie, nvars, name, out, nparts, arrays, body, ret="double"):
+def emit_split(trie, nvars, name, out, nparts, arrays, body, coef_expr, ret="double"):
     """Emits name_partK as __noinline__ functions over strided pointers to the
     caller's arrays, and the dispatcher name_piece.
 
@@ -246,7 +258,7 @@ def emit_split(trie, nvars, name, out, nparts, arrays, body, ret="double"):
     w("}")
 
 
-def emit_pip(trie, nvars, name, out, nparts=1):
+def emit_pip(trie, nvars, name, out, coef_expr, nparts=1):
     """FP64 value + gradient (multivariate Horner trie, reverse mode)."""
     out.append("// %s: polynomial and reverse-mode gradient (multivariate Horner trie)" % name)
 
@@ -280,7 +292,7 @@ def emit_pip(trie, nvars, name, out, nparts=1):
                 c = coef_expr(ch["coef"])
                 w("    E = fma(%s, x[%d], E); g[%d] += %s;" % (c, var, var, c))
 
-    emit_split(trie, nvars, name, out, nparts, [("x", "double", "in"), ("g", "double", "acc")], body)
+    emit_split(trie, nvars, name, out, nparts, [("x", "double", "in"), ("g", "double", "acc")], body, coef_expr)
 
 
 def shifted_pip(name):
@@ -304,7 +316,7 @@ def shifted_pip(name):
 _SHIFTED = {}
 
 
-def emit_pip_energy(trie, nvars, name, out, nparts=1):
+def emit_pip_energy(trie, nvars, name, out, coef_expr, nparts=1):
     """FP64 value only: plain Horner over the trie."""
     def body(w, subtrees):
         def node(n, var, depth):
@@ -325,7 +337,7 @@ def emit_pip_energy(trie, nvars, name, out, nparts=1):
             else:
                 w("    E = fma(%s, x[%d], E);" % (coef_expr(ch["coef"]), var))
 
-    emit_split(trie, nvars, name, out, nparts, [("x", "double", "in")], body)
+    emit_split(trie, nvars, name, out, nparts, [("x", "double", "in")], body, coef_expr)
 
 
 def emit_vars(spec, out):
@@ -488,7 +500,12 @@ def generate(name):
     if straight:
         for suffix, emitter, arg in (("pip", emit_pip, trie), ("pip_e", emit_pip_energy, trie)):
             body = head + ["#pragma once", '#include "%s.cuh"' % name]
-            emitter(arg, nv, "%s_%s" % (name, suffix), body, nparts)
+            coef = Coefficients(wt.nterms <= LEAF_ORDER_TERMS)
+            emitter(arg, nv, "%s_%s" % (name, suffix), body, coef, nparts)
+            if coef.by_leaf:
+                body.append("// (orbit + 1) of every coefficient, negative for -1")
+                body.append("#define %s_%s_LEAVES %s" % (name, suffix, ",".join(
+                    str((k + 1) * int(c)) for k, c in coef.leaves)))
             write_if_changed(os.path.join(OUT, "%s_%s.cuh" % (name, suffix)), "\n".join(body) + "\n")
         if name in QF_TYPES:
             from mbx_b200.codegen import qf
@@ -505,15 +522,50 @@ TU_HEAD = """// Generated by mbx_b200/codegen/gen_kernels.py -- do not edit.
 #include "../launch_cache.cuh"
 #include "%(name)s.cuh"
 %(include)s
-static __constant__ double c_%(name)s[%(ncw)d];
+static __constant__ double c_%(name)s[%(nc)d];
 struct %(name)s_CC {
     __device__ __forceinline__ double operator[](int k) const { return c_%(name)s[k]; }
 };
 
-// the coefficients in the w variables (%(ncw)d doubles, on the host or the device)
+%(setter)s"""
+
+# coefficients by orbit: the w coefficients as they are
+SET_ORBIT = """// the coefficients in the w variables (%(nc)d doubles, on the host or the device)
 int mbx_set_coef_%(name)s_%(v)s(const double* c, int from_device, cudaStream_t s) {
-    return (int)cudaMemcpyToSymbolAsync(c_%(name)s, c, sizeof(double) * %(ncw)d, 0,
+    return (int)cudaMemcpyToSymbolAsync(c_%(name)s, c, sizeof(double) * %(nc)d, 0,
                                         from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s);
+}
+"""
+
+# coefficients by leaf of the trie
+SET_LEAF = """// the coefficients in the w variables (on the host or the device), one per leaf
+static const short leaf_h_%(name)s[%(nc)d] = {%(name)s_%(pip)s_LEAVES};
+static __device__ const short leaf_d_%(name)s[%(nc)d] = {%(name)s_%(pip)s_LEAVES};
+static __device__ double leaf_c_%(name)s[%(nc)d];
+
+static __global__ void k_leaf_%(name)s(const double* __restrict__ c) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= %(nc)d) return;
+    const int o = leaf_d_%(name)s[i];
+    leaf_c_%(name)s[i] = o > 0 ? c[o - 1] : -c[-o - 1];
+}
+
+int mbx_set_coef_%(name)s_%(v)s(const double* c, int from_device, cudaStream_t s) {
+    if (!from_device) {
+        std::vector<double> h(%(nc)d);
+        for (int i = 0; i < %(nc)d; ++i) h[i] = leaf_h_%(name)s[i] > 0 ? c[leaf_h_%(name)s[i] - 1] : -c[-leaf_h_%(name)s[i] - 1];
+        cudaError_t e = cudaMemcpyToSymbolAsync(c_%(name)s, h.data(), sizeof(double) * %(nc)d, 0, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        return (int)e;
+    }
+    void* p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&p, leaf_c_%(name)s);
+    if (e != cudaSuccess) return (int)e;
+    k_leaf_%(name)s<<<(%(nc)d + 127) / 128, 128, 0, s>>>(c);
+    e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cudaMemcpyToSymbolAsync(c_%(name)s, p, sizeof(double) * %(nc)d, 0, cudaMemcpyDeviceToDevice, s);
+    return (int)e;
 }
 """
 
@@ -908,8 +960,10 @@ def write_kernels_cu(name):
         else:
             what, body = VARIANTS[v]
             wt = wtable(name)
-            d = {"name": name, "NAME": name.upper(), "ncw": wt.ncoef, "v": v, "what": what,
+            by_leaf = wt.nterms <= LEAF_ORDER_TERMS
+            d = {"name": name, "v": v, "what": what, "pip": inc[v], "nc": wt.nterms if by_leaf else wt.ncoef,
                  "include": '#include "%s_%s.cuh"\n' % (name, inc[v])}
+            d["setter"] = (SET_LEAF if by_leaf else SET_ORBIT) % d
             write_tu(path, (TU_HEAD + body) % d)
         paths.append(path)
     return paths

@@ -44,7 +44,7 @@ sys.path.insert(0, os.path.dirname(PKG))
 
 from mbx_b200.specs import SPECS, ONEBODY_SPECS, LP_GAMMA_IN, LP_GAMMA_OUT  # noqa: E402
 from mbx_b200.tables import load_pip  # noqa: E402
-from mbx_b200.codegen.wbasis import by_key as wtable_by_key, emit as emit_transforms, table_key, wtable  # noqa: E402
+from mbx_b200.codegen.wbasis import by_key as wtable_by_key, emit as emit_transforms, emit_chain, table_key, wtable  # noqa: E402
 
 OUT = os.path.join(PKG, "csrc", "gen")
 
@@ -442,6 +442,9 @@ def emit_traits(spec, table, straight, npieces, out):
     w("    template <class G, class Q> __device__ __forceinline__ static void chain_q(const double (&s)[%d][3], "
       "const G& g, const Q& q, double (&sg)[%d][3]) { %s_chain_q(s, g, q, sg); }" % (ns, ns, n))
     if straight:
+        w("    template <int S> __device__ __forceinline__ static void chain_w(const double (&s)[%d][3], "
+          "const double* __restrict__ x, const double* __restrict__ g, double (&sg)[%d][3]) "
+          "{ %s_chain_w<S>(s, x, g, sg); }" % (ns, ns, n))
         w("    static constexpr int NPIECES = %d, NPIECES_E = %d;  // of the two tries" % (npieces, npieces))
         w("    template <int S, class C> __device__ __forceinline__ static double pip_piece(int k, const C& c, "
           "const double* __restrict__ x, double* __restrict__ g) { return %s_pip_piece<S>(k, c, x, g); }" % n)
@@ -479,6 +482,7 @@ def generate(name):
     out.append("// %d terms in the w variables" % wt.nterms)
     emit_transforms(wt, name, out)
     if straight:
+        emit_chain(wt, spec, out)
         out += ["template <int S, class Coef> __device__ __forceinline__ double %s_pip_piece(int, const Coef&, "
                 "const double* __restrict__, double* __restrict__);" % name,
                 "template <int S, class Coef> __device__ __forceinline__ double %s_pip_e_piece(int, const Coef&, "
@@ -791,20 +795,25 @@ static __device__ int qfd_sj_%(name)s[%(name)s_Q::NB];
 static __device__ float qfd_colf_%(name)s[%(name)s_Q::NB];   // to constant memory by a copy
 static __device__ double qfd_b0_%(name)s[1];
 
-// a warp per row; the terms of a row are added in order, as on the host
-__global__ void k_qf_b_%(name)s() {
-    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+// a warp per row; the products of a row are added in order, as on the host
+__global__ void __launch_bounds__(128) k_qf_b_%(name)s() {
+    __shared__ double stage[4][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, j = blockIdx.x * 4 + w;
     if (j > %(norb)d) return;
     const bool c0 = j == %(norb)d;   // the constant term
     const int b = c0 ? 0 : dF_row_%(name)s[j], e = c0 ? %(nnz0)d : dF_row_%(name)s[j + 1];
     double acc = 0.0;
     for (int q0 = b; q0 < e; q0 += 32) {
         const int q = q0 + lane;
-        double p = 0.0;
+        double p = -0.0;   // (adding it changes nothing)
         if (q < e)
             p = c0 ? __dmul_rn(dF0_f_%(name)s[q], qfd_a_%(name)s[dF0_k_%(name)s[q]])
                    : __dmul_rn(dF_f_%(name)s[q], qfd_a_%(name)s[dF_k_%(name)s[q]]);
-        for (int i = 0; i < 32 && q0 + i < e; ++i) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, p, i));
+        stage[w][lane] = p;
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc = __dadd_rn(acc, stage[w][i]);
+        __syncwarp();
     }
     if (lane == 0) (c0 ? qfd_b0_%(name)s[0] : qfd_b_%(name)s[j]) = acc;
 }
@@ -828,7 +837,7 @@ __global__ void k_qf_cols_%(name)s() {
     const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (j >= NB) return;
     double m = 0.0;
-    for (int i = lane; i < NB; i += 32) m = fmax(m, fabs(qfd_C_%(name)s[i * NB + j]));
+    for (int i = lane; i < NB; i += 32) m = fmax(m, fabs(qfd_C_%(name)s[j * NB + i]));   // (C is symmetric)
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (lane) return;
     int sj = 0;
@@ -871,7 +880,7 @@ int mbx_set_coef_%(name)s_s(const double* a, int from_device, cudaStream_t s) {
     if (e == cudaSuccess) e = cudaMemsetAsync(C, 0, sizeof(qfd_C_%(name)s), s);
     if (e != cudaSuccess) return (int)e;
     constexpr int NB = %(name)s_Q::NB;
-    k_qf_b_%(name)s<<<((%(norb)d + 1) * 32 + 127) / 128, 128, 0, s>>>();
+    k_qf_b_%(name)s<<<(%(norb)d + 4) / 4, 128, 0, s>>>();
     k_qf_c_%(name)s<<<(qf_nmono_%(name)s + 127) / 128, 128, 0, s>>>();
     k_qf_cols_%(name)s<<<(NB * 32 + 127) / 128, 128, 0, s>>>();
     k_qf_image_%(name)s<<<(%(name)s_Q::KS * NB * 16 + 127) / 128, 128, 0, s>>>();
@@ -1058,7 +1067,10 @@ def write_term_tables():
                 raise ValueError("%s: half-monomial %s has more than three distinct variables" % (tname, m))
             rr = rr + [(255, 0)] * (3 - len(rr))
             half[i] = [sum(v << (8 * n) for n, (v, _) in enumerate(rr)), sum(e << (8 * n) for n, (_, e) in enumerate(rr))]
-        offs += [put(half), put(np.array([i | (j << 16) for i, j in pairs], np.int32))]
+        # (terms in the order of their first half: a warp's lanes share it)
+        by_half = sorted(range(t.nterms), key=lambda q: pairs[q])
+        offs += [put(half), put(np.array([pairs[q][0] | (pairs[q][1] << 16) for q in by_half], np.int32)),
+                 put(np.array(by_half, np.int32))]
         # first term of every coefficient (the table is sorted by them), and F
         # transposed
         offs.append(put(np.searchsorted(t.k, np.arange(t.ncoef + 1)).astype(np.int32)))
@@ -1077,10 +1089,11 @@ def write_term_tables():
              "// term tables in terms.bin: name, number of terms, (variable, exponent) pairs per",
              "// term at most, coefficients in the w variables; byte offsets of the int4 terms, the",
              "// double signs, the rows of F (starts, columns, factors), of W and of its transpose",
-             "// (starts, signed columns), of w0, of the half-monomials, of the terms' pairs of them, of the",
+             "// (starts, signed columns), of w0, of the half-monomials, of the terms' pairs of them (by",
+             "// the first one) and the terms in that order, of the",
              "// first term of every coefficient and of the rows of F transposed",
              "struct TermTableInfo { const char* name; long nterms; int pairs, ncw, nhalf; long off_terms, off_tcoef, "
-             "off_frow, off_fk, off_ff, off_wrow, off_w, off_wtrow, off_wt, off_w0, off_half, off_pair, "
+             "off_frow, off_fk, off_ff, off_wrow, off_w, off_wtrow, off_wt, off_w0, off_half, off_pair, off_term, "
              "off_first, off_ftrow, off_ftk, off_ftf; };",
              "static const TermTableInfo mbx_term_tables[] = {"]
     for tname, nt, npair, ncw, nhalf, offs in index:

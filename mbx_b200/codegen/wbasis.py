@@ -394,3 +394,46 @@ def emit(w, name, out):
             out.append("    for (int i = 0; i < %d; ++i) t[i] = x[i];" % nv)
             out.extend(text)
         out.append("}")
+
+
+def emit_chain(w, spec, out):
+    """NAME_chain_w: the chain rule from shared-memory columns of the w
+    (xm[i * S]) and of dP/dw (gm[i * S]), orbit by orbit of the variables: an
+    orbit's variables and their gradients from its few w, then each variable's
+    share of the site gradients.  The variables are not evaluated again (no
+    exponential, square root or division), and no array of all of them is
+    held in registers."""
+    nv, name, ns = w.nvars, spec.name, len(spec.sites)
+    a = out.append
+    a("template <int S>")
+    a("__device__ __forceinline__ void %s_chain_w(const double (&s)[%d][3], const double* __restrict__ xm, "
+      "const double* __restrict__ gm, double (&sg)[%d][3]) {" % (name, ns, ns))
+    a("#pragma unroll")
+    a("    for (int i = 0; i < %d; ++i) { sg[i][0] = 0.0; sg[i][1] = 0.0; sg[i][2] = 0.0; }" % ns)
+    inverse = np.linalg.inv(w.W)
+    done = set()
+    for v in range(nv):
+        if v in done:
+            continue
+        rows = [i for i in range(nv) if w.W[i, v] != 0.0]
+        orbit = sorted({u for i in rows for u in range(nv) if w.W[i, u] != 0.0})
+        assert sorted({i for u in orbit for i in range(nv) if w.W[i, u] != 0.0}) == rows
+        done |= set(orbit)
+        a("    {")
+        for i in rows:
+            base = "" if w.w0[i] == 0.0 else " + %r" % float(w.w0[i])
+            a("        const double w%d = xm[%d * S]%s, g%d = gm[%d * S];" % (i, i, base, i, i))
+        for u in orbit:
+            kind, p, q, k, _ = spec.variables[u]
+            scale = abs(inverse[u, rows[0]])
+            assert all(abs(inverse[u, i]) == scale for i in rows)
+            x = " ".join("%s w%d" % ("+" if inverse[u, i] > 0 else "-", i) for i in rows).lstrip("+ ")
+            g = " ".join("%s g%d" % ("+" if w.W[i, u] > 0 else "-", i) for i in rows).lstrip("+ ")
+            x = x if scale == 1.0 else "%r * (%s)" % (float(scale), x)
+            fn = "dvar_exp_v" if kind == "exp" else "dvar_coul_v"
+            a("        %s(s[%d], s[%d], %r, %s, %s, sg[%d], sg[%d]);" % (fn, p, q, float(k), x, g, p, q))
+        a("    }")
+    for (m, o, xp, xm) in spec.lp:
+        a("    lp_grads(s[%d], s[%d], s[%d], sg[%d], sg[%d], sg[%d], sg[%d], sg[%d]);" %
+          (o, o + 1, o + 2, xp, xm, o, o + 1, o + 2))
+    a("}")

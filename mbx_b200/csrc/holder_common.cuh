@@ -91,6 +91,25 @@ __device__ __forceinline__ void dvar_coul(const double (&p1)[3], const double (&
     sg2[0] -= f * a; sg2[1] -= f * b; sg2[2] -= f * c;
 }
 
+// dvar_exp / dvar_coul from the variable's value v (1 / r from one reciprocal
+// square root).
+__device__ __forceinline__ void dvar_exp_v(const double (&p1)[3], const double (&p2)[3], double k, double v, double gv,
+                                           double (&sg1)[3], double (&sg2)[3]) {
+    const double a = p1[0] - p2[0], b = p1[1] - p2[1], c = p1[2] - p2[2];
+    const double f = gv * (-k * v * rsqrt(a * a + b * b + c * c));
+    sg1[0] += f * a; sg1[1] += f * b; sg1[2] += f * c;
+    sg2[0] -= f * a; sg2[1] -= f * b; sg2[2] -= f * c;
+}
+
+__device__ __forceinline__ void dvar_coul_v(const double (&p1)[3], const double (&p2)[3], double k, double v,
+                                            double gv, double (&sg1)[3], double (&sg2)[3]) {
+    const double a = p1[0] - p2[0], b = p1[1] - p2[1], c = p1[2] - p2[2];
+    const double rinv = rsqrt(a * a + b * b + c * c);
+    const double f = gv * (-(k + rinv) * v * rinv);
+    sg1[0] += f * a; sg1[1] += f * b; sg1[2] += f * c;
+    sg2[0] -= f * a; sg2[1] -= f * b; sg2[2] -= f * c;
+}
+
 // The variable together with its radial factor q, dv/d(p1 - p2) = q (p1 - p2),
 // for the mixed path (pair_vars_kernel): 1 / r from one reciprocal square
 // root instead of a square root and a division (1-2 ulp, far below what the

@@ -271,6 +271,18 @@ __device__ __forceinline__ void chain_rule(const double (&s)[T::NSITES][3], cons
     T::chain_q(s, f.g, f.q, sg);
 }
 
+// The w and dP/dw of the lockstep kernels, in shared-memory columns of stride S.
+template <int S>
+struct WColumns {
+    const double* x;
+    const double* g;
+};
+template <class T, int S>
+__device__ __forceinline__ void chain_rule(const double (&s)[T::NSITES][3], const WColumns<S>& f,
+                                           double (&sg)[T::NSITES][3]) {
+    T::template chain_w<S>(s, f.x, f.g, sg);
+}
+
 // Everything after the polynomial: chain rule, switch, virial, scatter.  g:
 // dP/dv as chain_rule takes it.  share: ep and g are a part of the n-mer's
 // polynomial whose rest is added by other threads (per-n-mer outputs by
@@ -500,13 +512,7 @@ __global__ void __launch_bounds__(T::LOCK_THREADS, 1) holder_lock_kernel(const H
             if (busy) ep += piece(k, xs, gs);
             __syncthreads();
         }
-        if (live) {
-            double g[T::NVARS];
-#pragma unroll
-            for (int v = 0; v < T::NVARS; ++v) g[v] = grads ? gs[v * L] : 0.0;
-            T::from_w(g);
-            finish_nmer<T>(A, t, ep, g, grads, acc, shared_nmer);
-        }
+        if (live) finish_nmer<T>(A, t, ep, WColumns<L>{xs, gs}, grads, acc, shared_nmer);
         u += gridDim.x;
     }
     block_reduce_add<7>(acc, A.out);

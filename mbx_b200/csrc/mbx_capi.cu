@@ -55,6 +55,7 @@ struct AdjointTable {
     int nterms, nhalf, nvars, ncoef, ncw;
     const int2* half;
     const unsigned* pair;
+    const int* term;
     const int *first, *ftrow, *ftk;
     const double* ftf;
 };
@@ -1831,6 +1832,7 @@ extern "C" int mbx_evaluate_dcoef(mbx_ctx* c, const char* name, long n, const do
         const AdjointTable P{A.terms, A.tcoef, (int)A.nterms, T.nhalf, E->nvars, E->ncoef, T.ncw,
                              reinterpret_cast<const int2*>(c->tables.blob + T.off_half),
                              reinterpret_cast<const unsigned*>(c->tables.blob + T.off_pair),
+                             reinterpret_cast<const int*>(c->tables.blob + T.off_term),
                              reinterpret_cast<const int*>(c->tables.blob + T.off_first),
                              reinterpret_cast<const int*>(c->tables.blob + T.off_ftrow),
                              reinterpret_cast<const int*>(c->tables.blob + T.off_ftk),

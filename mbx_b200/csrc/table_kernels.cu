@@ -106,8 +106,8 @@ int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double
 // are added up in a fixed order (adjoint_terms_kernel), then the terms of
 // every coefficient (adjoint_coef_kernel) and F^T of those
 // (adjoint_out_kernel): the result is the same from call to call.  Bound by the shared-memory reads of two
-// scattered doubles per term and n-mer: 20000 MB-pol 3b trimers (7425 terms)
-// 180 us, where walking the 33525 terms in x, a lane per n-mer, took 14 ms.
+// doubles per term and n-mer, the second scattered, the first mostly the same
+// for a warp's lanes: 20000 MB-pol 3b trimers (7425 terms) 163 us, where walking the 33525 terms in x, a lane per n-mer, took 14 ms.
 #define MBX_ADJ_THREADS 512
 #define MBX_ADJ_N 8
 #define MBX_ADJ_Q 8
@@ -117,7 +117,8 @@ struct AdjointTable {
     const double* tcoef;
     int nterms, nhalf, nvars, ncoef, ncw;
     const int2* half;
-    const unsigned* pair;
+    const unsigned* pair;     // half-monomials of the terms, in the order of the first one
+    const int* term;          // the terms in that order
     const int *first, *ftrow, *ftk;   // first term of every coefficient; rows of F transposed
     const double* ftf;
 };
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(MBX_ADJ_THREADS)
 #pragma unroll
     for (int q = 0; q < MBX_ADJ_Q; ++q) {
         const int t = t0 + q * MBX_ADJ_THREADS;
-        if (t < P.nterms) part[(size_t)blockIdx.x * P.nterms + t] = acc[q];
+        if (t < P.nterms) part[(size_t)blockIdx.x * P.nterms + P.term[t]] = acc[q];
     }
 }
 

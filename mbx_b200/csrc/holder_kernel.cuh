@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(256, 2) pair_vars_kernel(const HolderArgs A) {
 }
 
 template <class T>
-__global__ void __launch_bounds__(128, 4) pair_finish_kernel(const HolderArgs A) {
+__global__ void __launch_bounds__(128, 3) pair_finish_kernel(const HolderArgs A) {
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     const long n = nmer_count(A);
     const long cap = A.ps.cap;

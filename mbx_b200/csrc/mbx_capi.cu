@@ -340,11 +340,13 @@ void sorted_slots(int nb, const std::string* ids, int* idx) {
 // several, so that the searches of a batch's configurations can run side by
 // side on their own streams.
 struct BuildScratch {
-    DevBuf<double> cloud;
-    DevBuf<int> cell_of, cell_count, cell_start, cell_fill, cell_items, cell_sorted, nb_count, copy_dir;
+    DevBuf<double> cloud, spos;
+    DevBuf<int> sdir, cell_of, cell_count, cell_start, cell_fill, cell_items, cell_sorted, nb_count, copy_dir;
     DevBuf<NbEntry> nb;
     void release() {
         cloud.release();
+        spos.release();
+        sdir.release();
         copy_dir.release();
         cell_of.release();
         cell_count.release();
@@ -933,6 +935,8 @@ static int launch_build_scope(mbx_ctx* c, int nbody, const BuildScope& S, const 
     const int ncell = cg.n[0] * cg.n[1] * cg.n[2];
     CUCHK(c, B.cloud.ensure((size_t)std::max(nmem, 1) * 24));
     CUCHK(c, B.copy_dir.ensure(std::max(nmem, 1)));
+    CUCHK(c, B.spos.ensure((size_t)std::max(nmem, 1) * 3));
+    CUCHK(c, B.sdir.ensure(std::max(nmem, 1)));
     CUCHK(c, B.cell_of.ensure(std::max(nmem, 1)));
     CUCHK(c, B.cell_items.ensure(std::max(nmem, 1)));
     CUCHK(c, B.cell_sorted.ensure(std::max(nmem, 1)));
@@ -946,7 +950,7 @@ static int launch_build_scope(mbx_ctx* c, int nbody, const BuildScope& S, const 
         // the whole cell list in one block
         k_cells_small<<<1, 1024, 0, st>>>(xyz, c->d_first.p, S.members, nmem, S.bp, cg, ncell, B.cloud.p, B.cell_of.p,
                                           B.copy_dir.p, B.cell_count.p, B.cell_start.p, B.cell_fill.p, B.cell_items.p,
-                                          B.cell_sorted.p);
+                                          B.cell_sorted.p, B.spos.p, B.sdir.p);
         *kernels += 1;
     } else {
         CUCHK(c, cudaMemsetAsync(B.cell_count.p, 0, (ncell + 1) * sizeof(int), st));
@@ -954,7 +958,8 @@ static int launch_build_scope(mbx_ctx* c, int nbody, const BuildScope& S, const 
                                                   B.copy_dir.p, B.cell_count.p);
         k_cell_scan<<<1, 1024, 0, st>>>(B.cell_count.p, ncell, B.cell_start.p, B.cell_fill.p);
         k_cell_fill<<<(nmem + T - 1) / T, T, 0, st>>>(B.cell_of.p, nmem, B.cell_fill.p, B.cell_items.p);
-        k_cell_sort<<<(ncell * 32 + T - 1) / T, T, 0, st>>>(B.cell_start.p, ncell, B.cell_items.p, B.cell_sorted.p);
+        k_cell_sort<<<(ncell * 32 + T - 1) / T, T, 0, st>>>(B.cell_start.p, ncell, B.cell_items.p, B.cloud.p,
+                                                            B.copy_dir.p, B.cell_sorted.p, B.spos.p, B.sdir.p);
         *kernels += 4;
     }
     // neighbour search: warps per query and unroll depth are tunable; one
@@ -962,8 +967,8 @@ static int launch_build_scope(mbx_ctx* c, int nbody, const BuildScope& S, const 
     const auto& K = c->knobs[nbody];
     const int nbw = (size_t)4 * c->nb_cap * sizeof(NbEntry) <= 160 * 1024 ? K.nb_warps : 1;
     if ((size_t)c->nb_cap * sizeof(NbEntry) > 227 * 1024) return fail(c, MBX_ENOMEM, "neighbour staging");
-    RCHK(c, launch_neighbors(nbw, K.nb_unroll, B.cloud.p, B.copy_dir.p, B.cell_of.p, B.cell_start.p, B.cell_sorted.p,
-                             S.query, nq, cg, S.bp.use_pbc, rc2, c->nb_cap, B.nb_count.p, B.nb.p, c->status.p,
+    RCHK(c, launch_neighbors(nbw, K.nb_unroll, B.cloud.p, B.spos.p, B.sdir.p, B.cell_of.p, B.cell_start.p,
+                             B.cell_sorted.p, S.query, nq, cg, S.bp, rc2, c->nb_cap, B.nb_count.p, B.nb.p, c->status.p,
                              st));
     if (nbody == 2) {
         DimerRules R = c->drules;
@@ -974,15 +979,11 @@ static int launch_build_scope(mbx_ctx* c, int nbody, const BuildScope& S, const 
             S.query, nq, S.members, c->d_tag.p, c->d_type.p, B.nb_count.p, B.nb.p, c->nb_cap, rc2, R, c->listed.p,
             list_cap > 0 ? c->list.p : nullptr, list_cap, c->buckets.p, c->bucket_count.p, c->status.p);
     } else {
-        // a block per query (tunable threads); its matches staged in shared memory
-        const size_t smem = (size_t)c->nb_cap * MBX_TRIMATCH_BYTES;
-        if (smem > 227 * 1024) return fail(c, MBX_ENOMEM, "trimer staging exceeds shared memory");
-        if (smem > 48 * 1024)
-            CUCHK(c, cudaFuncSetAttribute(k_trimers, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_trimers<<<nq, K.tri_threads, smem, st>>>(
-            S.query, nq, S.members, c->d_tag.p, c->d_type.p, B.cloud.p, B.nb_count.p, B.nb.p, c->nb_cap, rc2,
-            c->trules, c->listed.p, list_cap > 0 ? c->list.p : nullptr, list_cap, c->buckets.p, c->bucket_count.p,
-            c->status.p);
+        if ((size_t)c->nb_cap * MBX_TRIMATCH_BYTES > 227 * 1024)
+            return fail(c, MBX_ENOMEM, "trimer staging exceeds shared memory");
+        RCHK(c, launch_trimers(K.tri_threads, S.query, nq, S.members, c->d_tag.p, c->d_type.p, B.cloud.p, B.nb_count.p,
+                               B.nb.p, c->nb_cap, rc2, c->trules, c->listed.p, list_cap > 0 ? c->list.p : nullptr,
+                               list_cap, c->buckets.p, c->bucket_count.p, c->status.p, st));
     }
     CUCHK(c, cudaGetLastError());
     *kernels += 2;
@@ -1045,6 +1046,8 @@ static int launch_build_batch(mbx_ctx* c, int nbody, const double* xyz, int* ker
     const int* ids = c->d_members[0].p;   // identity: member position = monomer = query
     CUCHK(c, B.cloud.ensure((size_t)nmem * 24));
     CUCHK(c, B.copy_dir.ensure(nmem));
+    CUCHK(c, B.spos.ensure((size_t)nmem * 3));
+    CUCHK(c, B.sdir.ensure(nmem));
     CUCHK(c, B.cell_of.ensure(nmem));
     CUCHK(c, B.cell_items.ensure(nmem));
     CUCHK(c, B.cell_sorted.ensure(nmem));
@@ -1059,12 +1062,12 @@ static int launch_build_batch(mbx_ctx* c, int nbody, const double* xyz, int* ker
                                                     B.cloud.p, B.cell_of.p, B.copy_dir.p, B.cell_count.p);
     k_cell_scan<<<1, 1024, 0, st>>>(B.cell_count.p, ncell, B.cell_start.p, B.cell_fill.p);
     k_cell_fill<<<(nmem + T - 1) / T, T, 0, st>>>(B.cell_of.p, nmem, B.cell_fill.p, B.cell_items.p);
-    k_cell_sort<<<(int)(((long)ncell * 32 + T - 1) / T), T, 0, st>>>(B.cell_start.p, ncell, B.cell_items.p,
-                                                                      B.cell_sorted.p);
+    k_cell_sort<<<(int)(((long)ncell * 32 + T - 1) / T), T, 0, st>>>(B.cell_start.p, ncell, B.cell_items.p, B.cloud.p,
+                                                                      B.copy_dir.p, B.cell_sorted.p, B.spos.p, B.sdir.p);
     const auto& K = c->knobs[nbody];
     const int nbw = (size_t)4 * c->nb_cap * sizeof(NbEntry) <= 160 * 1024 ? K.nb_warps : 1;
     if ((size_t)c->nb_cap * sizeof(NbEntry) > 227 * 1024) return fail(c, MBX_ENOMEM, "neighbour staging");
-    RCHK(c, launch_neighbors_batch(nbw, K.nb_unroll, B.cloud.p, B.copy_dir.p, B.cell_of.p, B.cell_start.p,
+    RCHK(c, launch_neighbors_batch(nbw, K.nb_unroll, B.cloud.p, B.spos.p, B.sdir.p, B.cell_of.p, B.cell_start.p,
                                    B.cell_sorted.p, ids, nq,
                                    c->d_mon_conf.p, c->d_bgrid[nbody].p, rc2, c->nb_cap, B.nb_count.p, B.nb.p,
                                    c->status.p, st));
@@ -1077,13 +1080,11 @@ static int launch_build_batch(mbx_ctx* c, int nbody, const double* xyz, int* ker
             ids, nq, ids, c->d_tag.p, c->d_type.p, B.nb_count.p, B.nb.p, c->nb_cap, rc2, R, c->listed.p, nullptr, 0,
             c->buckets.p, c->bucket_count.p, c->status.p);
     } else {
-        const size_t smem = (size_t)c->nb_cap * MBX_TRIMATCH_BYTES;
-        if (smem > 227 * 1024) return fail(c, MBX_ENOMEM, "trimer staging exceeds shared memory");
-        if (smem > 48 * 1024)
-            CUCHK(c, cudaFuncSetAttribute(k_trimers, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_trimers<<<nq, K.tri_threads, smem, st>>>(ids, nq, ids, c->d_tag.p, c->d_type.p, B.cloud.p, B.nb_count.p,
-                                                    B.nb.p, c->nb_cap, rc2, c->trules, c->listed.p, nullptr, 0,
-                                                    c->buckets.p, c->bucket_count.p, c->status.p);
+        if ((size_t)c->nb_cap * MBX_TRIMATCH_BYTES > 227 * 1024)
+            return fail(c, MBX_ENOMEM, "trimer staging exceeds shared memory");
+        RCHK(c, launch_trimers(K.tri_threads, ids, nq, ids, c->d_tag.p, c->d_type.p, B.cloud.p, B.nb_count.p, B.nb.p,
+                               c->nb_cap, rc2, c->trules, c->listed.p, nullptr, 0, c->buckets.p, c->bucket_count.p,
+                               c->status.p, st));
     }
     CUCHK(c, cudaGetLastError());
     *kernels += 6;

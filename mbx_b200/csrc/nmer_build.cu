@@ -12,8 +12,7 @@
 //
 // Here the same cloud is built explicitly (k_cloud), monomers are binned into
 // a cell grid over fractional coordinates (k_cells*), every local monomer
-// collects its matches from the 27 surrounding cells by testing all eight
-// cloud points of each candidate (k_neighbors), and the dimer and trimer rules
+// collects its matches from the 27 surrounding cells (k_neighbors), and the dimer and trimer rules
 // run on those matches (k_dimers, k_trimers).  Every distance that decides
 // membership is computed with explicitly rounded operations in the
 // reference's operand order, so the sets are bit-for-bit the reference's.
@@ -23,6 +22,8 @@
 // image anchor (GetCloseDimerImage/GetCloseTrimerImage image relative to it).
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "holder_common.cuh"
 #include "nmer_build.h"
@@ -213,7 +214,9 @@ __device__ __forceinline__ void scan_cells(const int* cell_count, int ncell, int
 // the neighbour lists, and with them the slot order of every n-mer, are then
 // the same from run to run.  One warp; an item's place is the number of
 // smaller items of its cell (all items differ).
-__device__ __forceinline__ void sort_cell(int c, const int* cell_start, const int* items, int* sorted) {
+// spos / sdir: their wrapped first atoms and copy directions in that order.
+__device__ __forceinline__ void sort_cell(int c, const int* cell_start, const int* items, const double* cloud,
+                                          const int* copy_dir, int* sorted, double* spos, int* sdir) {
     const int lane = threadIdx.x & 31;
     const int b = cell_start[c], n = cell_start[c + 1] - b;
     for (int i0 = 0; i0 < n; i0 += 32) {
@@ -221,7 +224,13 @@ __device__ __forceinline__ void sort_cell(int c, const int* cell_start, const in
         const int v = i < n ? items[b + i] : 0;
         int rank = 0;
         for (int j = 0; j < n; ++j) rank += items[b + j] < v;
-        if (i < n) sorted[b + rank] = v;
+        if (i < n) {
+            const int slot = b + rank;
+            sorted[slot] = v;
+            sdir[slot] = copy_dir[v];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) spos[3 * (size_t)slot + a] = cloud[(size_t)v * 24 + a];
+        }
     }
 }
 
@@ -239,15 +248,17 @@ __global__ void k_cell_fill(const int* __restrict__ cell_of, int nmem, int* __re
 }
 
 __global__ void k_cell_sort(const int* __restrict__ cell_start, int ncell, const int* __restrict__ items,
-                            int* __restrict__ sorted) {
+                            const double* __restrict__ cloud, const int* __restrict__ copy_dir,
+                            int* __restrict__ sorted, double* __restrict__ spos, int* __restrict__ sdir) {
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (c < ncell) sort_cell(c, cell_start, items, sorted);
+    if (c < ncell) sort_cell(c, cell_start, items, cloud, copy_dir, sorted, spos, sdir);
 }
 
 __global__ void __launch_bounds__(1024) k_cells_small(const double* xyz, const int* first_index, const int* members,
                                                       int nmem, BoxParams bp, CellGrid cg, int ncell, double* cloud,
                                                       int* cell_of, int* copy_dir, int* cell_count, int* cell_start,
-                                                      int* cell_fill, int* cell_items, int* cell_sorted) {
+                                                      int* cell_fill, int* cell_items, int* cell_sorted, double* spos,
+                                                      int* sdir) {
     for (int i = threadIdx.x; i < ncell; i += blockDim.x) cell_count[i] = 0;
     __syncthreads();
     for (int q = threadIdx.x; q < nmem; q += blockDim.x) {
@@ -262,37 +273,47 @@ __global__ void __launch_bounds__(1024) k_cells_small(const double* xyz, const i
     __syncthreads();
     for (int q = threadIdx.x; q < nmem; q += blockDim.x) cell_items[atomicAdd(cell_fill + cell_of[q], 1)] = q;
     __syncthreads();
-    for (int c = threadIdx.x >> 5; c < ncell; c += blockDim.x >> 5) sort_cell(c, cell_start, cell_items, cell_sorted);
+    for (int c = threadIdx.x >> 5; c < ncell; c += blockDim.x >> 5) 
+        sort_cell(c, cell_start, cell_items, cloud, copy_dir, cell_sorted, spos, sdir);
 }
 
-// Matches of one query monomer: NW warps of a block split the 27 surrounding
-// cells (each warp a contiguous run of them, in the order below), stage their
-// hits in shared memory and write them out in cell order, so the list is the
-// same as a single warp scanning all cells.  A query with more than `cap`
-// matches sets MBX_STATUS_NB_OVERFLOW and its count in status[1].
+// Matches of one query monomer: the points of the (up to 27) surrounding cells,
+// cell after cell, are one run; the NW warps of a block take a share of it
+// each, 32 U points at a time (U independent loads in flight), stage their hits
+// in shared memory and write them out in the order of the run, so the list is
+// the same whatever NW and U.  A query with more than `cap` matches sets
+// MBX_STATUS_NB_OVERFLOW and its count in status[1].
+//
+// Where a cell's members have one point each (one_copy, or no PBC), the points
+// are read from the cell-ordered copies spos / sdir (coalesced) and moved by
+// the cell's own shift, the sum k_cloud makes; with eight copies from cloud.
+// Bound by the latency of these loads: the cells' ranges are read by one lane
+// per cell at once, and no lane is idle at the end of a cell (18.5k waters in 24
+// configurations, 9 and 7 A: 442 us cell by cell with gathered points, 164 us).
 namespace {
 
+struct CellRun {
+    int off[28];             // first point of every cell in the run; the total
+    int begin[27];           // its first item
+    int need[27], dirs[27];  // axes a member must be shifted along, and their directions
+    int cat[27];             // and the copy that is
+    double shift[27][3];
+};
+
 template <int NW, int U>
-__device__ __forceinline__ void neighbors_block(const double* __restrict__ cloud, const int* __restrict__ copy_dir,
-                            const int* __restrict__ cell_of,
+__device__ __forceinline__ void neighbors_block(const double* __restrict__ cloud, const double* __restrict__ spos,
+                            const int* __restrict__ sdir, const int* __restrict__ cell_of,
                             const int* __restrict__ cell_start, const int* __restrict__ cell_items,
-                            const int* __restrict__ query, int nquery, const CellGrid& cg, int use_pbc,
-                            int cell_off, double rc2, int cap, int* __restrict__ nb_count, NbEntry* __restrict__ nb,
-                            int* __restrict__ status, NbEntry* stage, int* wcount) {
+                            const int* __restrict__ query, int nquery, const CellGrid& cg, const double (&box)[9],
+                            int use_pbc, int cell_off, double rc2, int cap, int* __restrict__ nb_count,
+                            NbEntry* __restrict__ nb, int* __restrict__ status, NbEntry* stage, int* wcount,
+                            CellRun& R) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wq = blockIdx.x;
     if (wq >= nquery) return;
     const int qi = query[wq];
     const double* pi = cloud + (size_t)qi * 24;
     const double x0 = pi[0], x1 = pi[1], x2 = pi[2];
-    const int c = cell_of[qi] - cell_off;   // the cell in the query's own grid
-    const int cx = c % cg.n[0], cy = (c / cg.n[0]) % cg.n[1], cz = c / (cg.n[0] * cg.n[1]);
-    // neighbouring cells; an axis with fewer than 3 cells is scanned once
-    const int rx = cg.n[0] >= 3 ? 1 : 0, ry = cg.n[1] >= 3 ? 1 : 0, rz = cg.n[2] >= 3 ? 1 : 0;
-    const int sx = cg.n[0] >= 3 ? 3 : cg.n[0], sy = cg.n[1] >= 3 ? 3 : cg.n[1], sz = cg.n[2] >= 3 ? 3 : cg.n[2];
-    const int ncell = sx * sy * sz;
-    const int k0 = w * ncell / NW, k1 = (w + 1) * ncell / NW;
-    const int ncopy = use_pbc ? 8 : 1;
     // One copy per member (cg.one_copy): a point within the cutoff of the
     // query lies in the 3 x 3 x 3 block of cells around it in real space
     // (every cell is wider than the cutoff), so a member of a scanned cell can
@@ -301,84 +322,122 @@ __device__ __forceinline__ void neighbors_block(const double* __restrict__ cloud
     // in that direction, it cannot match at all.  The hits, and their order,
     // are those of the full eight-point test.
     const bool one = use_pbc && cg.one_copy;
-    const int npts = one ? 1 : ncopy;
-    // cloud category of a shift pattern (x, y, z shifted) -> copy index (k_cloud's order)
-    const int cat_of[8] = {0, 1, 2, 5, 3, 6, 7, 4};
-    NbEntry* mine = stage + (size_t)w * cap;
-    int count = 0;
-    for (int k = k0; k < k1; ++k) {
-        const int dx = k % sx, dy = (k / sx) % sy, dz = k / (sx * sy);
-        // periodic in index space both with PBC and for the hashed grid
-        // without PBC (n >= 3 there, so the 27 cells are distinct)
-        int ax = rx ? cx + dx - 1 : dx, ay = ry ? cy + dy - 1 : dy, az = rz ? cz + dz - 1 : dz;
-        // wrap of the cell in real space (one-copy mode: n >= 3, rx = ry = rz = 1)
-        const int tx = ax < 0 ? -1 : (ax >= cg.n[0] ? 1 : 0);
-        const int ty = ay < 0 ? -1 : (ay >= cg.n[1] ? 1 : 0);
-        const int tz = az < 0 ? -1 : (az >= cg.n[2] ? 1 : 0);
-        const int need = (tx != 0 ? 1 : 0) | (ty != 0 ? 2 : 0) | (tz != 0 ? 4 : 0);   // axes that must be shifted
-        const int dirs = (tx > 0 ? 1 : 0) | (ty > 0 ? 2 : 0) | (tz > 0 ? 4 : 0);       // and their directions
-        const int cat = cat_of[(tx != 0 ? 4 : 0) | (ty != 0 ? 2 : 0) | (tz != 0 ? 1 : 0)];
-        ax = (ax + cg.n[0]) % cg.n[0];
-        ay = (ay + cg.n[1]) % cg.n[1];
-        az = (az + cg.n[2]) % cg.n[2];
-        const int cell = cell_off + (az * cg.n[1] + ay) * cg.n[0] + ax;
-        const int b = cell_start[cell], e = cell_start[cell + 1];
-        // the cell's items in chunks of 32 (one load per lane, then shuffled);
-        // its (item, copy) points in item-major order, lanes over consecutive
-        // points (coalesced cloud loads), U independent 32-point blocks at a time
-        for (int c0 = b; c0 < e; c0 += 32) {
-            const int nit = e - c0 < 32 ? e - c0 : 32;
-            const int my_item = lane < nit ? cell_items[c0 + lane] : 0;
-            const int total = nit * npts;
-            for (int base = 0; base < total; base += 32 * U) {
-                bool hit[U];
-                NbEntry ent[U];
+    const bool eight = use_pbc && !one;
+    if (w == 0) {
+        const int c = cell_of[qi] - cell_off;   // the cell in the query's own grid
+        const int cx = c % cg.n[0], cy = (c / cg.n[0]) % cg.n[1], cz = c / (cg.n[0] * cg.n[1]);
+        // neighbouring cells; an axis with fewer than 3 cells is scanned once
+        const int rx = cg.n[0] >= 3 ? 1 : 0, ry = cg.n[1] >= 3 ? 1 : 0, rz = cg.n[2] >= 3 ? 1 : 0;
+        const int sx = cg.n[0] >= 3 ? 3 : cg.n[0], sy = cg.n[1] >= 3 ? 3 : cg.n[1], sz = cg.n[2] >= 3 ? 3 : cg.n[2];
+        const int ncell = sx * sy * sz, k = lane;
+        int points = 0;
+        if (k < ncell) {
+            const int dx = k % sx, dy = (k / sx) % sy, dz = k / (sx * sy);
+            // periodic in index space both with PBC and for the hashed grid
+            // without PBC (n >= 3 there, so the 27 cells are distinct)
+            int ax = rx ? cx + dx - 1 : dx, ay = ry ? cy + dy - 1 : dy, az = rz ? cz + dz - 1 : dz;
+            // wrap of the cell in real space (one-copy mode: n >= 3, rx = ry = rz = 1)
+            const int tx = ax < 0 ? -1 : (ax >= cg.n[0] ? 1 : 0);
+            const int ty = ay < 0 ? -1 : (ay >= cg.n[1] ? 1 : 0);
+            const int tz = az < 0 ? -1 : (az >= cg.n[2] ? 1 : 0);
+            ax = (ax + cg.n[0]) % cg.n[0];
+            ay = (ay + cg.n[1]) % cg.n[1];
+            az = (az + cg.n[2]) % cg.n[2];
+            const int cell = cell_off + (az * cg.n[1] + ay) * cg.n[0] + ax;
+            const int b = cell_start[cell], n = cell_start[cell + 1] - b;
+            points = eight ? 8 * n : n;
+            R.begin[k] = b;
+            R.need[k] = one ? (tx != 0 ? 1 : 0) | (ty != 0 ? 2 : 0) | (tz != 0 ? 4 : 0) : 0;
+            R.dirs[k] = one ? (tx > 0 ? 1 : 0) | (ty > 0 ? 2 : 0) | (tz > 0 ? 4 : 0) : 0;
+            // cloud category of a shift pattern (x, y, z shifted) -> copy index (k_cloud's order)
+            const int cat_of[8] = {0, 1, 2, 5, 3, 6, 7, 4};
+            R.cat[k] = one ? cat_of[(tx != 0 ? 4 : 0) | (ty != 0 ? 2 : 0) | (tz != 0 ? 1 : 0)] : 0;
+            const double m = tx, n1 = ty, l = tz;
 #pragma unroll
-                for (int h = 0; h < U; ++h) {
-                    const int t = base + 32 * h + lane;
-                    const int it = t < total ? t / npts : 0;
-                    const int qj = __shfl_sync(0xffffffffu, my_item, it);
-                    const bool ok = t < total && (!one || (copy_dir[qj] & need) == dirs);
-                    hit[h] = false;
-                    if (ok) {
-                        const int s = one ? cat : t - it * npts;
-                        const double* pj = cloud + (size_t)qj * 24 + 3 * s;
-                        const double d2 = dist2_rn(x0, x1, x2, pj[0], pj[1], pj[2]);
-                        if (d2 < rc2) {
-                            hit[h] = true;
-                            ent[h].member = qj;
-                            ent[h].copy = s;
-                            ent[h].d2 = d2;
-                        }
+            for (int a = 0; a < 3; ++a)
+                R.shift[k][a] = __dadd_rn(__dadd_rn(__dmul_rn(m, box[a]), __dmul_rn(n1, box[3 + a])),
+                                          __dmul_rn(l, box[6 + a]));
+        }
+        int x = points;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (k < 27) R.off[k] = x - points;
+        if (k == 26) R.off[27] = x;
+    }
+    __syncthreads();
+    const int total = R.off[27];
+    const int per = ((total + NW - 1) / NW + 31) / 32 * 32;
+    const int t1 = (w + 1) * per < total ? (w + 1) * per : total;
+    NbEntry* out = nb + (size_t)wq * cap;
+    NbEntry* mine = NW == 1 ? out : stage + (size_t)w * cap;   // (one warp's hits are in order as they come)
+    int count = 0, k = 0;
+    for (int base = w * per; base < t1; base += 32 * U) {
+        while (base >= R.off[k + 1]) ++k;   // the run's cell at base (empty cells have none)
+        bool hit[U];
+        NbEntry ent[U];
+#pragma unroll
+        for (int h = 0; h < U; ++h) {
+            const int t = base + 32 * h + lane;
+            hit[h] = false;
+            if (t < t1) {
+                int c = k;
+                while (t >= R.off[c + 1]) ++c;
+                const int i = t - R.off[c];
+                const int slot = R.begin[c] + (eight ? i >> 3 : i);
+                const int qj = cell_items[slot];
+                double y[3];
+                bool ok = true;
+                if (eight) {
+                    const double* pj = cloud + (size_t)qj * 24 + 3 * (i & 7);
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) y[a] = pj[a];
+                } else {
+                    const double* pj = spos + 3 * (size_t)slot;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) y[a] = pj[a];
+                    if (R.cat[c]) {
+                        ok = (sdir[slot] & R.need[c]) == R.dirs[c];
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) y[a] = __dadd_rn(y[a], R.shift[c][a]);
                     }
                 }
-#pragma unroll
-                for (int h = 0; h < U; ++h) {
-                    const unsigned m = __ballot_sync(0xffffffffu, hit[h]);
-                    if (hit[h]) {
-                        const int pos = count + __popc(m & ((1u << lane) - 1u));
-                        if (pos < cap) mine[pos] = ent[h];
-                    }
-                    count += __popc(m);
+                const double d2 = dist2_rn(x0, x1, x2, y[0], y[1], y[2]);
+                if (ok && d2 < rc2) {
+                    hit[h] = true;
+                    ent[h].member = qj;
+                    ent[h].copy = eight ? i & 7 : R.cat[c];
+                    ent[h].d2 = d2;
                 }
             }
+        }
+#pragma unroll
+        for (int h = 0; h < U; ++h) {
+            const unsigned m = __ballot_sync(0xffffffffu, hit[h]);
+            if (hit[h]) {
+                const int pos = count + __popc(m & ((1u << lane) - 1u));
+                if (pos < cap) mine[pos] = ent[h];
+            }
+            count += __popc(m);
         }
     }
     if (lane == 0) wcount[w] = count;
     __syncthreads();
-    int off = 0, total = 0;
+    int off = 0, found = 0;
     for (int j = 0; j < NW; ++j) {
         off += j < w ? wcount[j] : 0;
-        total += wcount[j];
+        found += wcount[j];
     }
-    NbEntry* out = nb + (size_t)wq * cap;
-    const int lim = count < cap ? count : cap;
-    for (int i = lane; i < lim && off + i < cap; i += 32) out[off + i] = mine[i];
+    if (NW > 1) {
+        const int lim = count < cap ? count : cap;
+        for (int i = lane; i < lim && off + i < cap; i += 32) out[off + i] = mine[i];
+    }
     if (threadIdx.x == 0) {
-        nb_count[wq] = total < cap ? total : cap;
-        if (total > cap) {
+        nb_count[wq] = found < cap ? found : cap;
+        if (found > cap) {
             atomicOr(status, MBX_STATUS_NB_OVERFLOW);
-            atomicMax(status + 1, total);
+            atomicMax(status + 1, found);
         }
     }
 }
@@ -387,23 +446,26 @@ __device__ __forceinline__ void neighbors_block(const double* __restrict__ cloud
 
 template <int NW, int U>
 __global__ void __launch_bounds__(NW * 32) k_neighbors(const double* __restrict__ cloud,
-                                                       const int* __restrict__ copy_dir,
+                                                       const double* __restrict__ spos,
+                                                       const int* __restrict__ sdir,
                                                        const int* __restrict__ cell_of,
                                                        const int* __restrict__ cell_start,
                                                        const int* __restrict__ cell_items,
                                                        const int* __restrict__ query, int nquery, CellGrid cg,
-                                                       int use_pbc, double rc2, int cap, int* __restrict__ nb_count,
+                                                       BoxParams bp, double rc2, int cap, int* __restrict__ nb_count,
                                                        NbEntry* __restrict__ nb, int* __restrict__ status) {
     extern __shared__ unsigned char smem[];
     __shared__ int wcount[NW];
-    neighbors_block<NW, U>(cloud, copy_dir, cell_of, cell_start, cell_items, query, nquery, cg, use_pbc, 0, rc2, cap,
-                           nb_count, nb, status, reinterpret_cast<NbEntry*>(smem), wcount);
+    __shared__ CellRun run;
+    neighbors_block<NW, U>(cloud, spos, sdir, cell_of, cell_start, cell_items, query, nquery, cg, bp.box, bp.use_pbc, 0,
+                           rc2, cap, nb_count, nb, status, reinterpret_cast<NbEntry*>(smem), wcount, run);
 }
 
 // The same over a batch: each query searches its own configuration's grid.
 template <int NW, int U>
 __global__ void __launch_bounds__(NW * 32) k_neighbors_batch(const double* __restrict__ cloud,
-                                                             const int* __restrict__ copy_dir,
+                                                             const double* __restrict__ spos,
+                                                             const int* __restrict__ sdir,
                                                              const int* __restrict__ cell_of,
                                                              const int* __restrict__ cell_start,
                                                              const int* __restrict__ cell_items,
@@ -414,21 +476,23 @@ __global__ void __launch_bounds__(NW * 32) k_neighbors_batch(const double* __res
                                                              int* __restrict__ status) {
     extern __shared__ unsigned char smem[];
     __shared__ int wcount[NW];
+    __shared__ CellRun run;
     if (blockIdx.x >= nquery) return;
     const BatchGrid& G = grids[conf_of[query[blockIdx.x]]];
-    neighbors_block<NW, U>(cloud, copy_dir, cell_of, cell_start, cell_items, query, nquery, G.cg, G.bp.use_pbc,
-                           G.cell_off, rc2, cap, nb_count, nb, status, reinterpret_cast<NbEntry*>(smem), wcount);
+    neighbors_block<NW, U>(cloud, spos, sdir, cell_of, cell_start, cell_items, query, nquery, G.cg, G.bp.box,
+                           G.bp.use_pbc, G.cell_off, rc2, cap, nb_count, nb, status, reinterpret_cast<NbEntry*>(smem),
+                           wcount, run);
 }
 
 // Host side: one block of `warps` warps per query (1 or 4), U = `unroll`
 // independent 32-point blocks per iteration (1, 2 or 4); the hits of each
 // warp are staged in warps x cap NbEntry of dynamic shared memory.
-int launch_neighbors(int warps, int unroll, const double* cloud, const int* copy_dir, const int* cell_of,
-                     const int* cell_start, const int* cell_items, const int* query, int nquery, CellGrid cg,
-                     int use_pbc, double rc2, int cap, int* nb_count, NbEntry* nb, int* status, cudaStream_t s) {
+int launch_neighbors(int warps, int unroll, const double* cloud, const double* spos, const int* sdir,
+                     const int* cell_of, const int* cell_start, const int* cell_items, const int* query, int nquery,
+                     CellGrid cg, const BoxParams& bp, double rc2, int cap, int* nb_count, NbEntry* nb, int* status, cudaStream_t s) {
     if (nquery <= 0) return 0;
-    const size_t smem = (size_t)warps * cap * sizeof(NbEntry);
-    if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
+    const size_t smem = warps > 1 ? (size_t)warps * cap * sizeof(NbEntry) : 0;
+    if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
 #define MBX_NB_CASE(NW, UU)                                                                                      \
     if (warps == NW && unroll == UU) {                                                                           \
         if (smem > 48 * 1024) {                                                                                  \
@@ -436,9 +500,9 @@ int launch_neighbors(int warps, int unroll, const double* cloud, const int* copy
                                                  (int)smem);                                                    \
             if (e != cudaSuccess) return (int)e;                                                                 \
         }                                                                                                        \
-        k_neighbors<NW, UU><<<nquery, NW * 32, smem, s>>>(cloud, copy_dir, cell_of, cell_start, cell_items, query, \
-                                                           nquery,                                                \
-                                                           cg, use_pbc, rc2, cap, nb_count, nb, status);          \
+        k_neighbors<NW, UU><<<nquery, NW * 32, smem, s>>>(cloud, spos, sdir, cell_of, cell_start, cell_items,   \
+                                                           query, nquery, cg, bp, rc2, cap, nb_count, nb,       \
+                                                           status);                                             \
         return (int)cudaGetLastError();                                                                          \
     }
     MBX_NB_CASE(4, 1)
@@ -451,14 +515,13 @@ int launch_neighbors(int warps, int unroll, const double* cloud, const int* copy
     return (int)cudaErrorInvalidValue;
 }
 
-int launch_neighbors_batch(int warps, int unroll, const double* cloud, const int* copy_dir, const int* cell_of,
-                           const int* cell_start,
-                           const int* cell_items, const int* query, int nquery, const int* conf_of,
+int launch_neighbors_batch(int warps, int unroll, const double* cloud, const double* spos, const int* sdir,
+                           const int* cell_of, const int* cell_start, const int* cell_items, const int* query, int nquery, const int* conf_of,
                            const BatchGrid* grids, double rc2, int cap, int* nb_count, NbEntry* nb, int* status,
                            cudaStream_t s) {
     if (nquery <= 0) return 0;
-    const size_t smem = (size_t)warps * cap * sizeof(NbEntry);
-    if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
+    const size_t smem = warps > 1 ? (size_t)warps * cap * sizeof(NbEntry) : 0;
+    if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
 #define MBX_NB_CASE(NW, UU)                                                                                      \
     if (warps == NW && unroll == UU) {                                                                           \
         if (smem > 48 * 1024) {                                                                                  \
@@ -466,10 +529,9 @@ int launch_neighbors_batch(int warps, int unroll, const double* cloud, const int
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
             if (e != cudaSuccess) return (int)e;                                                                 \
         }                                                                                                        \
-        k_neighbors_batch<NW, UU><<<nquery, NW * 32, smem, s>>>(cloud, copy_dir, cell_of, cell_start, cell_items, \
-                                                                 query,                                          \
-                                                                 nquery, conf_of, grids, rc2, cap, nb_count, nb, \
-                                                                 status);                                        \
+        k_neighbors_batch<NW, UU><<<nquery, NW * 32, smem, s>>>(cloud, spos, sdir, cell_of, cell_start,         \
+                                                                 cell_items, query, nquery, conf_of, grids, rc2, \
+                                                                 cap, nb_count, nb, status);                    \
         return (int)cudaGetLastError();                                                                          \
     }
     MBX_NB_CASE(4, 1)
@@ -492,6 +554,51 @@ struct TriMatch {
     int member, m, tag, type;
 };
 static_assert(sizeof(TriMatch) == MBX_TRIMATCH_BYTES, "TriMatch layout");
+
+// Accepted n-mers of a block, collected in shared memory and written to their
+// buckets together: one atomicAdd per bucket and flush, where one per warp and
+// 32 candidates queued up at the counters (2048 waters: 74k of them).
+constexpr int kCollect = 512;   // two rounds of the widest block at least
+
+struct Collected {
+    int n, at[MBX_MAX_BUCKETS], base[MBX_MAX_BUCKETS];
+    int4 nmer[kCollect];
+    unsigned char bucket[kCollect];
+};
+
+struct CollectedNone {
+    int n, at[1], base[1];
+    int4 nmer[1];
+    unsigned char bucket[1];
+};
+
+// Writes the collected n-mers out and empties the collection.  All threads of
+// the block.
+template <class Collection, class Rules>
+__device__ __forceinline__ void flush_collected(Collection& S, const Rules& R, int4* __restrict__ bucket_data,
+                                                int* __restrict__ bucket_count, int* __restrict__ status) {
+    __syncthreads();
+    const int n = S.n < kCollect ? S.n : kCollect;
+    if (threadIdx.x < MBX_MAX_BUCKETS) S.at[threadIdx.x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&S.at[S.bucket[i]], 1);
+    __syncthreads();
+    if (threadIdx.x < MBX_MAX_BUCKETS) {
+        const int m = S.at[threadIdx.x];
+        S.base[threadIdx.x] = m ? atomicAdd(bucket_count + threadIdx.x, m) : 0;
+        S.at[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int b = S.bucket[i];
+        const int pos = S.base[b] + atomicAdd(&S.at[b], 1);
+        if (pos < R.cap[b]) bucket_data[R.offset[b] + pos] = S.nmer[i];
+        else atomicOr(status, MBX_STATUS_BUCKET_OVERFLOW);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) S.n = 0;
+    __syncthreads();
+}
 
 // One slot per lane that wants one, in counters[key]: lanes with the same key
 // share one atomicAdd.  Called by all 32 lanes of the warp.
@@ -579,6 +686,7 @@ __global__ void k_dimers(const int* __restrict__ query, int nquery, const int* _
 // Trimers: a block of warps per query monomer i.  Its matches within rc are
 // staged in shared memory with everything the rules read (cloud point,
 // member, tag, type), then the block's lanes run over the pairs of matches.
+template <bool COLLECT>
 __global__ void __launch_bounds__(256) k_trimers(const int* __restrict__ query, int nquery,
                           const int* __restrict__ members,
                           const int* __restrict__ tag, const int* __restrict__ type, const double* __restrict__ cloud,
@@ -589,6 +697,8 @@ __global__ void __launch_bounds__(256) k_trimers(const int* __restrict__ query, 
     extern __shared__ unsigned char smem[];
     TriMatch* sh = reinterpret_cast<TriMatch*>(smem);
     __shared__ int s_n;
+    __shared__ typename std::conditional<COLLECT, Collected, CollectedNone>::type S;
+    if (threadIdx.x == 0) S.n = 0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wq = blockIdx.x;
     if (wq >= nquery) return;
@@ -628,19 +738,29 @@ __global__ void __launch_bounds__(256) k_trimers(const int* __restrict__ query, 
     }
     __syncthreads();
     const int n = s_n;
-    const long npair = (long)n * (n - 1) / 2;
+    const int npair = n * (n - 1) / 2;   // (n is a few thousand at most)
     unsigned long long mine = 0;
-    for (long base = 32L * w; base < npair; base += blockDim.x) {
-        const long p = base + lane;
+    // rounds of one pair per thread; a round adds at most blockDim.x n-mers
+    for (int round = 0; round < npair; round += blockDim.x) {
+        if constexpr (COLLECT) {
+            if (round > 0) {
+                __syncthreads();
+                const int have = S.n;
+                __syncthreads();   // (every thread has read it before any adds to it)
+                if (have + (int)blockDim.x > kCollect) flush_collected(S, R, bucket_data, bucket_count, status);
+            }
+        }
+        const int p = round + threadIdx.x;
         bool keep = false;
         int mj = 0, mk = 0, bk = -1, code = 0;
         if (p < npair) {
-            // pair index -> (a, b), a < b
-            int a = (int)((2.0 * n - 1 - sqrt((2.0 * n - 1) * (2.0 * n - 1) - 8.0 * p)) / 2.0);
-            if (a < 0) a = 0;
-            while ((long)(a + 1) * (2 * n - a - 2) / 2 <= p) ++a;
-            while ((long)a * (2 * n - a - 1) / 2 > p) --a;
-            const int b = (int)(p - (long)a * (2 * n - a - 1) / 2) + a + 1;
+            // pair index -> (a, b), a < b: counted from the end, the rows have
+            // 1, 2, 3, ... pairs (FP32 root, then exact)
+            int a = n - 2 - (int)((sqrtf(8.0f * (float)(npair - 1 - p) + 1.0f) - 1.0f) * 0.5f);
+            a = a < 0 ? 0 : a;
+            while ((a + 1) * (2 * n - a - 2) / 2 <= p) ++a;
+            while (a * (2 * n - a - 1) / 2 > p) --a;
+            const int b = p - a * (2 * n - a - 1) / 2 + a + 1;
             const TriMatch& ea = sh[a];
             const TriMatch& eb = sh[b];
             if (ea.member != eb.member) {
@@ -666,21 +786,44 @@ __global__ void __launch_bounds__(256) k_trimers(const int* __restrict__ query, 
             if (keep && pos < list_cap) list[pos] = make_int4(mi, mj, mk, 0);
         }
         const bool ins = bk >= 0;
-        const int pos = warp_reserve(bucket_count, ins ? bk : 0, ins);
+        const int pos = COLLECT ? warp_reserve(&S.n, 0, ins) : warp_reserve(bucket_count, ins ? bk : 0, ins);
         if (ins) {
-            if (pos < R.cap[bk]) {
-                const int perm = R.perm[code];   // slot s of the holder takes original slot (perm >> 2s) & 3
-                const int orig[3] = {mi, mj, mk};
-                const int s0 = perm & 3, s1 = (perm >> 2) & 3, s2 = (perm >> 4) & 3;
-                int anchor = 0;
-                if (s1 == 0) anchor = 1;
-                if (s2 == 0) anchor = 2;
-                bucket_data[R.offset[bk] + pos] = make_int4(orig[s0], orig[s1], orig[s2], anchor);
+            const int perm = R.perm[code];   // slot s of the holder takes original slot (perm >> 2s) & 3
+            const int orig[3] = {mi, mj, mk};
+            const int s0 = perm & 3, s1 = (perm >> 2) & 3, s2 = (perm >> 4) & 3;
+            int anchor = 0;
+            if (s1 == 0) anchor = 1;
+            if (s2 == 0) anchor = 2;
+            const int4 nm = make_int4(orig[s0], orig[s1], orig[s2], anchor);
+            if constexpr (COLLECT) {
+                S.nmer[pos] = nm;
+                S.bucket[pos] = (unsigned char)bk;
+            } else if (pos < R.cap[bk]) {
+                bucket_data[R.offset[bk] + pos] = nm;
             } else {
                 atomicOr(status, MBX_STATUS_BUCKET_OVERFLOW);
             }
         }
     }
+    if constexpr (COLLECT) flush_collected(S, R, bucket_data, bucket_count, status);
     for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
     if (lane == 0 && mine) atomicAdd(listed, mine);
+}
+
+// A block of `threads` per query, its matches (at most cap) staged in shared
+// memory; the n-mers are collected there too where both fit.
+int launch_trimers(int threads, const int* query, int nquery, const int* members, const int* tag, const int* type,
+                   const double* cloud, const int* nb_count, const NbEntry* nb, int cap, double rc2,
+                   const TrimerRules& R, unsigned long long* listed, int4* list, long list_cap, int4* bucket_data,
+                   int* bucket_count, int* status, cudaStream_t s) {
+    const size_t smem = (size_t)cap * MBX_TRIMATCH_BYTES;
+    if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
+    auto kern = smem + sizeof(Collected) + 64 <= 227 * 1024 ? k_trimers<true> : k_trimers<false>;
+    if (smem + sizeof(Collected) + 64 > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    kern<<<nquery, threads, smem, s>>>(query, nquery, members, tag, type, cloud, nb_count, nb, cap, rc2, R, listed, list,
+                                       list_cap, bucket_data, bucket_count, status);
+    return (int)cudaGetLastError();
 }

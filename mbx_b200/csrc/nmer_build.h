@@ -68,32 +68,33 @@ __global__ void k_cloud(const double* xyz, const int* first_index, const int* me
 // cells), in one block.
 __global__ void k_cells_small(const double* xyz, const int* first_index, const int* members, int nmem, BoxParams bp,
                               CellGrid cg, int ncell, double* cloud, int* cell_of, int* copy_dir, int* cell_count,
-                              int* cell_start, int* cell_fill, int* cell_items, int* cell_sorted);
+                              int* cell_start, int* cell_fill, int* cell_items, int* cell_sorted, double* spos,
+                              int* sdir);
 // The same for a batch: members are the batch's monomers in order (member
 // position = monomer), each with the grid of its configuration conf_of[q].
 __global__ void k_cloud_batch(const double* xyz, const int* first_index, int nmem, const int* conf_of,
                               const BatchGrid* grids, double* cloud, int* cell_of, int* copy_dir, int* cell_count);
 __global__ void k_cell_scan(const int* cell_count, int ncell, int* cell_start, int* cell_fill);
 __global__ void k_cell_fill(const int* cell_of, int nmem, int* cell_fill, int* cell_items);
-__global__ void k_cell_sort(const int* cell_start, int ncell, const int* items, int* sorted);
+__global__ void k_cell_sort(const int* cell_start, int ncell, const int* items, const double* cloud,
+                            const int* copy_dir, int* sorted, double* spos, int* sdir);
 // Matches of every query monomer (k_neighbors): `warps` warps per query (1 or
 // 4), `unroll` independent 32-point blocks per iteration (1, 2 or 4).
-int launch_neighbors(int warps, int unroll, const double* cloud, const int* copy_dir, const int* cell_of,
-                     const int* cell_start, const int* cell_items, const int* query, int nquery, CellGrid cg,
-                     int use_pbc, double rc2,
-                     int cap, int* nb_count, NbEntry* nb, int* status, cudaStream_t s);
+int launch_neighbors(int warps, int unroll, const double* cloud, const double* spos, const int* sdir,
+                     const int* cell_of, const int* cell_start, const int* cell_items, const int* query, int nquery,
+                     CellGrid cg, const BoxParams& bp, double rc2, int cap, int* nb_count, NbEntry* nb, int* status, cudaStream_t s);
 // The same over a batch (queries are member positions, conf_of and grids as
 // for k_cloud_batch).
-int launch_neighbors_batch(int warps, int unroll, const double* cloud, const int* copy_dir, const int* cell_of,
-                           const int* cell_start,
-                           const int* cell_items, const int* query, int nquery, const int* conf_of,
-                           const BatchGrid* grids, double rc2, int cap, int* nb_count, NbEntry* nb, int* status,
-                           cudaStream_t s);
+int launch_neighbors_batch(int warps, int unroll, const double* cloud, const double* spos, const int* sdir,
+                           const int* cell_of, const int* cell_start, const int* cell_items, const int* query,
+                           int nquery, const int* conf_of, const BatchGrid* grids, double rc2, int cap, int* nb_count,
+                           NbEntry* nb, int* status, cudaStream_t s);
 __global__ void k_dimers(const int* query, int nquery, const int* members, const int* tag, const int* type,
                          const int* nb_count, const NbEntry* nb, int cap, double rc2, DimerRules R,
                          unsigned long long* listed, int4* list, long list_cap, int4* bucket_data,
                          int* bucket_count, int* status);
-__global__ void k_trimers(const int* query, int nquery, const int* members, const int* tag, const int* type,
-                          const double* cloud, const int* nb_count, const NbEntry* nb, int cap, double rc2,
-                          TrimerRules R, unsigned long long* listed, int4* list, long list_cap, int4* bucket_data,
-                          int* bucket_count, int* status);
+// The trimer rules over the matches of every query, a block of `threads` each.
+int launch_trimers(int threads, const int* query, int nquery, const int* members, const int* tag, const int* type,
+                   const double* cloud, const int* nb_count, const NbEntry* nb, int cap, double rc2,
+                   const TrimerRules& R, unsigned long long* listed, int4* list, long list_cap, int4* bucket_data,
+                   int* bucket_count, int* status, cudaStream_t s);

@@ -1,0 +1,124 @@
+"""Kernels of the symmetry-adapted path at the sizes where they can go wrong:
+chunks cut by pieces of the polynomial, the one-block and the gridded cell
+list, every launch shape of the search, the coefficient adjoint around its
+tiles, coefficients set from the host and from the device (GPU)."""
+import numpy as np
+import pytest
+
+import mbx_oracle as mo
+from mbx_b200 import system as msys, workloads
+from mbx_b200.specs import SPECS
+from mbx_b200.tables import load_fit
+
+pytestmark = pytest.mark.gpu
+
+E_REL = 1e-10
+G_ABS = 1e-8
+E_ABS_NMER = 1e-8   # one n-mer: its terms are up to 1e6 times their sum (test_gpu_parity)
+
+
+# 1 dimer and no trimer; 1 trimer; a few; around one chunk of 384 n-mers (28
+# waters have 378 dimers, 29 have 406); several chunks
+@pytest.mark.parametrize("n", [2, 3, 9, 28, 29, 60])
+def test_chunks_cut_by_pieces(n):
+    ids, xyz = workloads.water_cluster(n, seed=n)
+    s = msys.from_arrays(ids, xyz, None, 20.0, 20.0)
+    ref = mo.OracleSystem(ids, xyz, None, 20.0, 20.0)
+    for nb in (2, 3):
+        e, er = (s.TwoBodyEnergy(True) if nb == 2 else s.ThreeBodyEnergy(True)), ref.energy(nb)
+        assert abs(e - er) <= E_REL * abs(er) + E_ABS_NMER
+        assert np.abs(s.GetRealGrads() - ref.real_grads()).max() <= G_ABS
+        eo = s.TwoBodyEnergy(False) if nb == 2 else s.ThreeBodyEnergy(False)
+        assert abs(eo - er) <= E_REL * abs(er) + E_ABS_NMER
+
+
+# one block builds the cell list up to 1024 members
+@pytest.mark.parametrize("n", [1023, 1024, 1025])
+def test_search_around_one_block(n):
+    edge = 39.44 * (n / 2048) ** (1 / 3)
+    ids, xyz, box = workloads.water_box(12, n, edge, seed=n)
+    s = msys.from_arrays(ids, xyz, box, 9.0, 7.0)
+    o = xyz.reshape(-1, 9)[:, :3]
+    d = o[:, None, :] - o[None, :, :]
+    d -= edge * np.round(d / edge)
+    i, j = np.nonzero(np.triu((d ** 2).sum(2) < 81.0, 1))
+    assert np.array_equal(s.GetPairList(2, 9.0), np.stack([i, j], 1))
+
+
+@pytest.mark.parametrize("box", ["wide", "narrow", "none"])
+def test_search_launch_shapes(box):
+    """wide: three or more cells per axis (one copy of every member); narrow:
+    two cells (eight copies); none: no periodic boundaries."""
+    if box == "none":
+        ids, xyz = workloads.water_cluster(150, seed=4)
+        b = None
+    else:
+        n = 700 if box == "wide" else 230
+        ids, xyz, b = workloads.water_box(10 if box == "wide" else 7, n, 39.44 * (n / 2048) ** (1 / 3), seed=4)
+    s = msys.from_arrays(ids, xyz, b, 9.0, 7.0)
+    want = {nb: s.GetPairList(nb, 7.0) for nb in (2, 3)}
+    assert len(want[3]) > 1000
+    for warps, unroll, threads in ((1, 1, 64), (1, 4, 256), (4, 1, 256), (4, 4, 64)):
+        for nb in (2, 3):
+            s._ctx.set_knobs(nb, nb_warps=warps, nb_unroll=unroll, tri_threads=threads)
+            assert np.array_equal(s.GetPairList(nb, 7.0), want[nb])
+
+
+def nmers(name, n, seed):
+    rng = np.random.default_rng(seed)
+    parts = []
+    for k, m in enumerate(SPECS[name].monomers):
+        v = rng.normal(size=(n, 3))
+        r = rng.uniform(2.8, 5.0, size=n) * (k > 0)
+        body = workloads.BODIES[m]() if m in workloads.BODIES else np.zeros((1, 3))
+        parts.append(workloads.place(rng, body, v / np.linalg.norm(v, axis=1, keepdims=True) * r[:, None]))
+    return np.ascontiguousarray(np.concatenate(parts, 1).reshape(n, -1))
+
+
+# one n-mer; a tile of 8 and one more; several blocks; more than one chunk of
+# 32768; one range of terms (mbpol2b), two (mbpol3b), half-monomials of degree
+# 3 (h2oli2b) and more (nana2b, one variable)
+@pytest.mark.parametrize("name,n", [("mbpol2b", 1), ("mbpol2b", 8), ("mbpol2b", 9), ("mbpol2b", 32769),
+                                    ("mbpol3b", 1000), ("h2oli2b", 77), ("clh2o3b", 50), ("nana2b", 5)])
+def test_adjoint_is_the_energy_per_coefficient(ctx, name, n):
+    """The energy is linear in the coefficients: sum_k a_k dE/da_k = E; and the
+    sums are made in the same order every time."""
+    import torch
+    x = torch.tensor(nmers(name, n, 5), device="cuda")
+    w = torch.tensor(np.random.default_rng(6).uniform(-1, 1, n), device="cuda")
+    a = load_fit(name)
+    e = torch.empty(n, dtype=torch.float64, device="cuda")
+    ctx.evaluate(name, x, None, None, e, grads=False)
+    out = [torch.zeros(len(a), dtype=torch.float64, device="cuda") for _ in range(2)]
+    for o in out:
+        ctx.evaluate_dcoef(name, x, w, o)
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1])
+    d = out[0].cpu().numpy()
+    we = (w * e).cpu().numpy()
+    # rounding of the products a_k d_k and of their sum, and of the energies
+    bound = 64 * 2.0 ** -53 * np.abs(a * d).sum() + E_ABS_NMER * np.sqrt(n)
+    assert abs((a * d).sum() - we.sum()) <= bound
+
+
+@pytest.mark.parametrize("name", ["mbpol2b", "mbpol3b", "h2ona3b", "ch4h2o3b", "co2co22b"])
+def test_coefficients_from_host_and_device(ctx, name):
+    import torch
+    x = torch.tensor(nmers(name, 300, 7), device="cuda")
+    a = load_fit(name) * np.random.default_rng(8).uniform(0.9, 1.1, SPECS[name].ncoef)
+
+    def energies(coef, mixed):
+        ctx.set_coefficients(name, coef)
+        e, g = torch.empty(300, dtype=torch.float64, device="cuda"), torch.zeros_like(x)
+        ctx.evaluate(name, x, g, None, e, mixed=mixed)
+        torch.cuda.synchronize()
+        return e, g
+
+    for mixed in (False, True):
+        fitted = energies(None, mixed)
+        host = energies(a, mixed)
+        device = energies(torch.tensor(a, device="cuda"), mixed)
+        again = energies(None, mixed)
+        assert not torch.equal(fitted[0], host[0])
+        for p, q in ((host, device), (fitted, again)):
+            assert torch.equal(p[0], q[0]) and torch.equal(p[1], q[1])

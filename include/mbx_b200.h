@@ -41,6 +41,7 @@ enum {
 #define MBX_MIXED 2         /* FP32 monomials, FP64 accumulation (else FP64) */
 #define MBX_NO_GRADS 4      /* energy only */
 #define MBX_GRAPH 8         /* mbx_batch_energy: capture the sequence in a CUDA graph, replay it */
+#define MBX_NO_WAIT 16      /* mbx_evaluate: return without waiting for the device (see there) */
 
 /* Context on one device with its own stream.  Replaces the state a
  * bblock::System keeps for the 2b/3b path (system.h:1175ff).  One context per
@@ -120,7 +121,10 @@ int mbx_nmers(mbx_ctx* ctx, int nbody, double cutoff, const double* xyz, int use
  * answers for any name), coordinates
  * xyz[n][nreal*3] with the monomers in evaluator
  * order and already imaged.  grad (same layout, +=), virial (9, +=), e_per
- * (n switched energies) may be NULL.  *energy gets the sum. */
+ * (n switched energies) may be NULL.  *energy gets the sum.  With
+ * MBX_NO_WAIT (device pointers, FP64, energy and virial NULL; MBX_EINVAL
+ * otherwise) the call returns once its work is enqueued on the context's
+ * stream, for callers that go on on that stream. */
 int mbx_evaluate(mbx_ctx* ctx, const char* evaluator, long n, const double* xyz, double* grad, double* virial,
                  double* e_per, double* energy, int flags);
 

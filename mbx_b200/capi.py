@@ -18,6 +18,7 @@ MBX_DEVICE_PTRS = 1
 MBX_MIXED = 2
 MBX_NO_GRADS = 4
 MBX_GRAPH = 8
+MBX_NO_WAIT = 16
 
 EVALUATORS = ("mbpol2b", "mbpol3b", "ch4h2o2b", "ch4ch42b", "ch4h2o3b",
               "h2oli2b", "h2ona2b", "h2ok2b", "h2orb2b", "h2ocs2b",
@@ -315,6 +316,19 @@ class Context:
         e = ctypes.c_double()
         self._check(lib().mbx_evaluate(self.h, name.encode(), n, px, pg, pv, pe, ctypes.byref(e), flags))
         return e.value
+
+    def evaluate_async(self, name, xyz, grad=None, e_per=None):
+        """evaluate() in FP64 on CUDA tensors without waiting for the result
+        (no energy sum, no virial): the outputs are ready on the context's
+        stream."""
+        nreal = evaluator_info(name)[1]
+        ptrs = [_ptr(a) for a in (xyz, grad, e_per)]
+        if not all(dev for p, dev in ptrs if p is not None):
+            raise TypeError("CUDA tensors only")
+        self._order(True)
+        n = xyz.shape[0] if xyz.ndim > 1 else xyz.numel() // (3 * nreal)
+        flags = MBX_DEVICE_PTRS | MBX_NO_WAIT | (0 if grad is not None else MBX_NO_GRADS)
+        self._check(lib().mbx_evaluate(self.h, name.encode(), n, ptrs[0][0], ptrs[1][0], None, ptrs[2][0], None, flags))
 
     def evaluate_dcoef(self, name, xyz, w=None, out=None):
         nb, nreal, nv, nc = evaluator_info(name)

@@ -1723,6 +1723,10 @@ extern "C" int mbx_evaluate(mbx_ctx* c, const char* name, long n, const double* 
     if (!c || !name || n < 0 || (n > 0 && !xyz)) return fail(c, MBX_EINVAL, "bad arguments");
     const EvaluatorInfo* E = find_evaluator(name);
     if (!E) return fail(c, MBX_ENOTSUP, std::string("unknown evaluator ") + name);
+    // (the mixed kernels can report a timeout, which the host has to read)
+    const bool no_wait = (flags & MBX_NO_WAIT) != 0;
+    if (no_wait && (!(flags & MBX_DEVICE_PTRS) || (flags & MBX_MIXED) || energy || virial))
+        return fail(c, MBX_EINVAL, "MBX_NO_WAIT takes device arrays in FP64, no energy and no virial");
     CUCHK(c, cudaSetDevice(c->device));
     const bool dev = (flags & MBX_DEVICE_PTRS) != 0;
     const size_t nx = (size_t)n * E->nreal * 3;
@@ -1763,6 +1767,11 @@ extern "C" int mbx_evaluate(mbx_ctx* c, const char* name, long n, const double* 
     if (n > 0) {
         r = launch_eval(c, E, A, grads ? (flags & MBX_MIXED) : (flags | MBX_NO_GRADS), &kernels);
         if (r) return r;
+    }
+    if (no_wait) {
+        c->last_ms_build = c->last_ms_eval = 0;
+        c->last_kernels = kernels;
+        return MBX_OK;
     }
     CUCHK(c, cudaEventRecord(c->ev[2], c->stream));
     CUCHK(c, cudaMemcpyAsync(c->h_out, c->ctl.p, MBX_CTL_RESULTS * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

@@ -78,7 +78,8 @@ class _NmerEnergies(torch.autograd.Function):
             g = torch.zeros_like(xyz)
             c.evaluate(name, xyz, g, vir, e, mixed=mixed, grads=True)
         else:
-            c.evaluate(name, xyz, None, None, e, mixed=mixed, grads=False)
+            # (energies alone: the FP64 kernel in either precision)
+            c.evaluate_async(name, xyz, None, e)
         fctx.save_for_backward(xyz, coef)
         fctx.name = name
         fctx.mixed = mixed
@@ -97,7 +98,10 @@ class _NmerEnergies(torch.autograd.Function):
         if fctx.needs_input_grad[0]:
             # reverse pass: the gradient kernel, everything recomputed from xyz
             g = torch.zeros_like(xyz)
-            c.evaluate(fctx.name, xyz, g, None, None, mixed=fctx.mixed, grads=True)
+            if fctx.mixed:
+                c.evaluate(fctx.name, xyz, g, None, None, mixed=True, grads=True)
+            else:
+                c.evaluate_async(fctx.name, xyz, g)
             dxyz = g * ge[:, None]
         if fctx.needs_input_grad[1]:
             dcoef = torch.zeros_like(coef)

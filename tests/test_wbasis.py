@@ -24,12 +24,18 @@ def test_w_polynomial_is_the_polynomial(name):
     for _ in range(3):
         x = rng.uniform(0.1, 1.2, table.nvars)
         a = rng.normal(size=table.ncoef)
+        v = w.W @ x - w.w0
         direct = terms_of(table, a, x)
-        t = terms_of(w, w.coefficients(a), w.W @ x)
+        t = terms_of(w, w.coefficients(a), v)
         # both are sums of at most nterms products of at most degree + 2
-        # factors, each rounded to 2^-53: the terms in w are not larger in sum
+        # factors, each rounded to 2^-53
         bound = (table.degree + 4 + np.log2(table.nterms)) * 2.0 ** -53
-        assert abs(t.sum() - direct.sum()) <= 8 * bound * (np.abs(direct).sum() + np.abs(t).sum())
+        # and every w is rounded relative to its parts: |dw| <= 4 2^-53 (|W| |x|
+        # + |w0|), which a term takes in proportion to dw / w of its factors
+        dw = 4 * 2.0 ** -53 * (np.abs(w.W) @ np.abs(x) + np.abs(w.w0)) / np.abs(v)
+        carried = np.append(dw, 0.0)[np.where(w.var < 0, len(x), w.var)].sum(1)
+        assert abs(t.sum() - direct.sum()) <= 8 * bound * (np.abs(direct).sum() + np.abs(t).sum()) + \
+            (np.abs(t) * carried).sum()
 
 
 @pytest.mark.parametrize("name", NAMES)

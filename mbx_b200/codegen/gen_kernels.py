@@ -379,9 +379,9 @@ def emit_vars(spec, out):
         w("    lp_grads(s[%d], s[%d], s[%d], sg[%d], sg[%d], sg[%d], sg[%d], sg[%d]);" %
           (o, o + 1, o + 2, xp, xm, o, o + 1, o + 2))
     w("}")
-    # chain rule: site gradients from dP/dv (g, an array of NVARS doubles or
-    # anything indexable the same way, e.g. a reader of the FP32 gradients in
-    # global memory that loads each where it is used), scaled by sw
+    if spec.name not in ONEBODY_SPECS:
+        return   # the n-mer kernels' chain rules are chain_w (wbasis.py) and chain_q
+    # chain rule of the 1-body kernel: site gradients from dP/dv
     w("template <class G>")
     w("__device__ __forceinline__ void %s_chain(const double (&s)[%d][3], const G& g, "
       "double (&sg)[%d][3]) {" % (spec.name, ns, ns))
@@ -435,8 +435,9 @@ def emit_traits(spec, table, straight, npieces, out):
       (spec.nreal, ns, n))
     w("    __device__ __forceinline__ static void vars(const double (&s)[%d][3], double (&x)[%d]) { %s_vars(s, x); }" %
       (ns, spec.nvars, n))
-    w("    template <class G> __device__ __forceinline__ static void chain(const double (&s)[%d][3], const G& g, "
-      "double (&sg)[%d][3]) { %s_chain(s, g, sg); }" % (ns, ns, n))
+    if not straight:
+        w("    template <class G> __device__ __forceinline__ static void chain(const double (&s)[%d][3], const G& g, "
+          "double (&sg)[%d][3]) { %s_chain(s, g, sg); }" % (ns, ns, n))
     w("    template <class QW> __device__ __forceinline__ static void vars_q(const double (&s)[%d][3], "
       "double (&x)[%d], QW& q) { %s_vars_q(s, x, q); }" % (ns, spec.nvars, n))
     w("    template <class G, class Q> __device__ __forceinline__ static void chain_q(const double (&s)[%d][3], "

@@ -181,20 +181,3 @@ def shifted_coefficients(sp, a):
     b = np.array([sum(f * a[k] for k, f in row.items()) for row in sp.F])
     b0 = sum(f * a[k] for k, f in sp.const_F.items())
     return b0, b
-
-
-class ShiftedTable:
-    """The shifted monomials in the layout of tables.PipTable (k = orbit)."""
-
-    def __init__(self, sp, name):
-        n = len(sp.monos)
-        self.name = name
-        self.nvars = sp.nvars
-        self.ncoef = sp.norb
-        self.nterms = n
-        self.k = np.array(sp.orbit_of, np.int32)
-        self.coef = np.ones(n)
-        self.deg = np.array([len(m) for m in sp.monos], np.int32)
-        self.var = np.full((n, 4), -1, np.int32)
-        for t, m in enumerate(sp.monos):
-            self.var[t, :len(m)] = m

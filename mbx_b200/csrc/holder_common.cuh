@@ -17,11 +17,6 @@
 // Two FP32 lanes in one 64-bit register (low half: first value), operated on
 // by the paired FP32 instructions of sm_100 (one instruction, two results).
 typedef unsigned long long f2_t;
-__device__ __forceinline__ f2_t f2_fma(f2_t a, f2_t b, f2_t c) {
-    f2_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 __device__ __forceinline__ f2_t f2_mul(f2_t a, f2_t b) {
     f2_t d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));

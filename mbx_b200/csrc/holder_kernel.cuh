@@ -241,14 +241,7 @@ __device__ __forceinline__ void conf_accumulate(double* dst, const double (&v)[7
     }
 }
 
-// The chain rule from dP/dv: g is an array of T::NVARS doubles, or a reader
-// indexed the same way; PairFactors (below) also brings the variables'
-// radial factors, so that nothing is recomputed.
-template <class T, class G>
-__device__ __forceinline__ void chain_rule(const double (&s)[T::NSITES][3], const G& g, double (&sg)[T::NSITES][3]) {
-    T::chain(s, g, sg);
-}
-
+// The chain rule, from what the kernel at hand holds: PairFactors or WColumns.
 // dP/dv (FP32) and the radial factors (FP64) of n-mer t in the mixed path's
 // scratch, read where the chain rule uses them
 struct PairGrad {

@@ -7,9 +7,9 @@ library.  Incremental: a unit is rebuilt when its source or any header it can
 see is newer than its object.  A file lock keeps concurrent builds (two
 processes importing the package on a fresh checkout) from racing.
 
-The straight-line kernels of the four trie-compiled evaluators are the long
-units (about 1-2 minutes each in ptxas); everything else is table-driven and
-compiles in seconds, so a clean build takes a few minutes on 8 cores.
+The straight-line kernels of the widest polynomials (CH4-CH4, the halides' 3b)
+are the long units, half a minute to a minute each in ptxas; a clean build takes
+about four minutes on 8 cores.
 
 Usage: ``python -m mbx_b200.build [-j N] [--verbose]``
 """
@@ -32,7 +32,7 @@ LIB = os.path.join(PKG, "libmbx_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # (--compress-mode=size: the straight-line code with its line tables would make
-# the library 190 MB, compressed 35 MB)
+# the library 190 MB; compressed it has 56 MB, 26 of them tables)
 FLAGS = ["-O3", "-lineinfo", "--compress-mode=size", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 HAND = ("mbx_capi.cu", "nmer_build.cu", "peaks.cu", "noalloc.cu", "table_kernels.cu", "onebody.cu")

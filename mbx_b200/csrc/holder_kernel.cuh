@@ -17,9 +17,9 @@
 // The polynomial is that in the symmetry-adapted variables w
 // (mbx_b200/codegen/wbasis.py): T::to_w takes the variables x to w, T::from_w
 // the gradient back.  It has 3 to 8 times fewer terms (MB-pol 3b gradients of
-// 132k trimers: 1.36 ms in x, 0.41 ms in w; the types that had no
+// 132k trimers: 1.36 ms in x, 0.35 ms in w; the types that had no
 // straight-line code ran from their term tables, 1 M NaCl 29 ms a step, now
-// 1.2).
+// 1.05).
 #pragma once
 #include "holder_common.cuh"
 #include "term_table.cuh"

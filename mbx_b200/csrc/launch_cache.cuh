@@ -17,6 +17,7 @@ struct LaunchCache {
     std::once_flag once[MBX_MAX_DEVICES];
     int sms[MBX_MAX_DEVICES] = {0};
     int bps[MBX_MAX_DEVICES] = {0};
+    size_t most[MBX_MAX_DEVICES] = {0};
     int err[MBX_MAX_DEVICES] = {0};
 };
 
@@ -42,4 +43,34 @@ int launch_facts(LaunchCache& lc, K kern, int block, int smem_attr, int smem_occ
     *sms = lc.sms[dev];
     *bps = lc.bps[dev];
     return lc.err[dev];
+}
+
+// KERN<<<grid, block, smem, s>>>(args...) for a kernel whose dynamic shared
+// memory differs from call to call.  Its limit is set once per device, to all
+// that its static shared memory leaves of a block's: a limit set by each call
+// to its own size could be lowered by another host thread between this
+// thread's setting and its launch, and the default limit counts the static
+// part too.  Returns a cudaError_t value (invalid value: smem above the limit).
+template <auto KERN, class... A>
+int launch_any_smem(dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+    static LaunchCache lc;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= MBX_MAX_DEVICES) return (int)cudaErrorInvalidDevice;
+    std::call_once(lc.once[dev], [&] {
+        int optin = 0;
+        cudaFuncAttributes f;
+        cudaError_t r = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (r == cudaSuccess) r = cudaFuncGetAttributes(&f, KERN);
+        if (r == cudaSuccess) {
+            lc.most[dev] = (size_t)optin - f.sharedSizeBytes;
+            r = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lc.most[dev]);
+        }
+        lc.err[dev] = (int)r;
+    });
+    if (lc.err[dev]) return lc.err[dev];
+    if (smem > lc.most[dev]) return (int)cudaErrorInvalidValue;
+    KERN<<<grid, block, smem, s>>>(args...);
+    return (int)cudaGetLastError();
 }

@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "holder_common.cuh"
+#include "launch_cache.cuh"
 #include "nmer_build.h"
 
 namespace {
@@ -492,19 +493,11 @@ int launch_neighbors(int warps, int unroll, const double* cloud, const double* s
                      CellGrid cg, const BoxParams& bp, double rc2, int cap, int* nb_count, NbEntry* nb, int* status, cudaStream_t s) {
     if (nquery <= 0) return 0;
     const size_t smem = warps > 1 ? (size_t)warps * cap * sizeof(NbEntry) : 0;
-    if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
 #define MBX_NB_CASE(NW, UU)                                                                                      \
-    if (warps == NW && unroll == UU) {                                                                           \
-        if (smem > 48 * 1024) {                                                                                  \
-            cudaError_t e = cudaFuncSetAttribute(k_neighbors<NW, UU>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                                 (int)smem);                                                    \
-            if (e != cudaSuccess) return (int)e;                                                                 \
-        }                                                                                                        \
-        k_neighbors<NW, UU><<<nquery, NW * 32, smem, s>>>(cloud, spos, sdir, cell_of, cell_start, cell_items,   \
-                                                           query, nquery, cg, bp, rc2, cap, nb_count, nb,       \
-                                                           status);                                             \
-        return (int)cudaGetLastError();                                                                          \
-    }
+    if (warps == NW && unroll == UU)                                                                             \
+        return launch_any_smem<k_neighbors<NW, UU>>(nquery, NW * 32, smem, s, cloud, spos, sdir, cell_of,        \
+                                                    cell_start, cell_items, query, nquery, cg, bp, rc2, cap,     \
+                                                    nb_count, nb, status);
     MBX_NB_CASE(4, 1)
     MBX_NB_CASE(4, 2)
     MBX_NB_CASE(4, 4)
@@ -521,19 +514,11 @@ int launch_neighbors_batch(int warps, int unroll, const double* cloud, const dou
                            cudaStream_t s) {
     if (nquery <= 0) return 0;
     const size_t smem = warps > 1 ? (size_t)warps * cap * sizeof(NbEntry) : 0;
-    if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
 #define MBX_NB_CASE(NW, UU)                                                                                      \
-    if (warps == NW && unroll == UU) {                                                                           \
-        if (smem > 48 * 1024) {                                                                                  \
-            cudaError_t e = cudaFuncSetAttribute(k_neighbors_batch<NW, UU>,                                      \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
-            if (e != cudaSuccess) return (int)e;                                                                 \
-        }                                                                                                        \
-        k_neighbors_batch<NW, UU><<<nquery, NW * 32, smem, s>>>(cloud, spos, sdir, cell_of, cell_start,         \
-                                                                 cell_items, query, nquery, conf_of, grids, rc2, \
-                                                                 cap, nb_count, nb, status);                    \
-        return (int)cudaGetLastError();                                                                          \
-    }
+    if (warps == NW && unroll == UU)                                                                             \
+        return launch_any_smem<k_neighbors_batch<NW, UU>>(nquery, NW * 32, smem, s, cloud, spos, sdir, cell_of,  \
+                                                          cell_start, cell_items, query, nquery, conf_of, grids, \
+                                                          rc2, cap, nb_count, nb, status);
     MBX_NB_CASE(4, 1)
     MBX_NB_CASE(4, 2)
     MBX_NB_CASE(4, 4)
@@ -566,16 +551,12 @@ struct Collected {
     unsigned char bucket[kCollect];
 };
 
-struct CollectedNone {
-    int n, at[1], base[1];
-    int4 nmer[1];
-    unsigned char bucket[1];
-};
+struct NotCollected {};
 
 // Writes the collected n-mers out and empties the collection.  All threads of
 // the block.
-template <class Collection, class Rules>
-__device__ __forceinline__ void flush_collected(Collection& S, const Rules& R, int4* __restrict__ bucket_data,
+template <class Rules>
+__device__ __forceinline__ void flush_collected(Collected& S, const Rules& R, int4* __restrict__ bucket_data,
                                                 int* __restrict__ bucket_count, int* __restrict__ status) {
     __syncthreads();
     const int n = S.n < kCollect ? S.n : kCollect;
@@ -697,8 +678,10 @@ __global__ void __launch_bounds__(256) k_trimers(const int* __restrict__ query, 
     extern __shared__ unsigned char smem[];
     TriMatch* sh = reinterpret_cast<TriMatch*>(smem);
     __shared__ int s_n;
-    __shared__ typename std::conditional<COLLECT, Collected, CollectedNone>::type S;
-    if (threadIdx.x == 0) S.n = 0;
+    __shared__ typename std::conditional<COLLECT, Collected, NotCollected>::type S;
+    if constexpr (COLLECT) {
+        if (threadIdx.x == 0) S.n = 0;
+    }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int wq = blockIdx.x;
     if (wq >= nquery) return;
@@ -786,7 +769,9 @@ __global__ void __launch_bounds__(256) k_trimers(const int* __restrict__ query, 
             if (keep && pos < list_cap) list[pos] = make_int4(mi, mj, mk, 0);
         }
         const bool ins = bk >= 0;
-        const int pos = COLLECT ? warp_reserve(&S.n, 0, ins) : warp_reserve(bucket_count, ins ? bk : 0, ins);
+        int pos;
+        if constexpr (COLLECT) pos = warp_reserve(&S.n, 0, ins);
+        else pos = warp_reserve(bucket_count, ins ? bk : 0, ins);
         if (ins) {
             const int perm = R.perm[code];   // slot s of the holder takes original slot (perm >> 2s) & 3
             const int orig[3] = {mi, mj, mk};
@@ -817,13 +802,11 @@ int launch_trimers(int threads, const int* query, int nquery, const int* members
                    const TrimerRules& R, unsigned long long* listed, int4* list, long list_cap, int4* bucket_data,
                    int* bucket_count, int* status, cudaStream_t s) {
     const size_t smem = (size_t)cap * MBX_TRIMATCH_BYTES;
-    if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
-    auto kern = smem + sizeof(Collected) + 64 <= 227 * 1024 ? k_trimers<true> : k_trimers<false>;
-    if (smem + sizeof(Collected) + 64 > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
-    kern<<<nquery, threads, smem, s>>>(query, nquery, members, tag, type, cloud, nb_count, nb, cap, rc2, R, listed, list,
-                                       list_cap, bucket_data, bucket_count, status);
-    return (int)cudaGetLastError();
+    if (smem + sizeof(Collected) + 64 <= 227 * 1024)
+        return launch_any_smem<k_trimers<true>>(nquery, threads, smem, s, query, nquery, members, tag, type, cloud,
+                                                nb_count, nb, cap, rc2, R, listed, list, list_cap, bucket_data,
+                                                bucket_count, status);
+    return launch_any_smem<k_trimers<false>>(nquery, threads, smem, s, query, nquery, members, tag, type, cloud,
+                                             nb_count, nb, cap, rc2, R, listed, list, list_cap, bucket_data,
+                                             bucket_count, status);
 }

@@ -12,6 +12,7 @@
 // the warp.
 #include <cuda_runtime.h>
 
+#include "launch_cache.cuh"
 #include "term_table.cuh"
 
 #define MBX_POLY_WARPS 4
@@ -233,14 +234,12 @@ int mbx_coef_adjoint_blocks(const AdjointTable& P, int sms) {
 int mbx_launch_coef_adjoint(const double* wv, int count, const AdjointTable& P, double* work, double* out, int sms,
                             cudaStream_t s) {
     const size_t smem = ((size_t)(P.nvars + 1) * MBX_ADJ_N + 2 * (size_t)P.nhalf * (MBX_ADJ_N + 1)) * sizeof(double);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(coef_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-    }
     const int want = (count + MBX_ADJ_N - 1) / MBX_ADJ_N, most = mbx_coef_adjoint_blocks(P, sms);
     const int nx = want < most ? (want > 0 ? want : 1) : most;
     double* sum = work + (size_t)most * P.nterms;
-    coef_adjoint_kernel<<<dim3(nx, adjoint_ranges(P)), MBX_ADJ_THREADS, smem, s>>>(wv, count, P, work);
+    const int r = launch_any_smem<coef_adjoint_kernel>(dim3(nx, adjoint_ranges(P)), MBX_ADJ_THREADS, smem, s, wv, count, P,
+                                                       work);
+    if (r) return r;
     adjoint_terms_kernel<<<(P.nterms + 31) / 32, dim3(32, 8), 0, s>>>(work, nx, P.nterms, sum);
     double* dc = sum + P.nterms;
     adjoint_coef_kernel<<<(P.ncw + 127) / 128, 128, 0, s>>>(P, sum, dc);

@@ -182,14 +182,17 @@ class Context:
     def _order(self, dev_ptrs):
         """Device arrays from torch: when the library runs on another stream
         than torch's current one, torch's work on them (allocation, zeroing)
-        must be complete before the library's kernels start."""
+        must be complete before the library's kernels start.  Returns whether
+        the two are the same stream."""
         if not dev_ptrs:
-            return
+            return False
         import torch
         cur = torch.cuda.current_stream(self.device)
         mine = self.stream if self.stream != 1 else 0   # 1: cudaStreamLegacy, torch's default stream
         if self.stream in (0, None) or mine != cur.cuda_stream:
             cur.synchronize()
+            return False
+        return True
 
     def close(self):
         if getattr(self, "h", None):
@@ -319,15 +322,17 @@ class Context:
 
     def evaluate_async(self, name, xyz, grad=None, e_per=None):
         """evaluate() in FP64 on CUDA tensors without waiting for the result
-        (no energy sum, no virial): the outputs are ready on the context's
-        stream."""
+        (no energy sum, no virial): the outputs are ready on torch's current
+        stream.  A context that runs on another stream waits all the same:
+        its caller has no way to wait for that stream, and torch may hand the
+        memory of tensors dropped meanwhile to others."""
         nreal = evaluator_info(name)[1]
         ptrs = [_ptr(a) for a in (xyz, grad, e_per)]
         if not all(dev for p, dev in ptrs if p is not None):
             raise TypeError("CUDA tensors only")
-        self._order(True)
+        same = self._order(True)
         n = xyz.shape[0] if xyz.ndim > 1 else xyz.numel() // (3 * nreal)
-        flags = MBX_DEVICE_PTRS | MBX_NO_WAIT | (0 if grad is not None else MBX_NO_GRADS)
+        flags = MBX_DEVICE_PTRS | (MBX_NO_WAIT if same else 0) | (0 if grad is not None else MBX_NO_GRADS)
         self._check(lib().mbx_evaluate(self.h, name.encode(), n, ptrs[0][0], ptrs[1][0], None, ptrs[2][0], None, flags))
 
     def evaluate_dcoef(self, name, xyz, w=None, out=None):

@@ -56,3 +56,36 @@ def test_registered_torch_ops_shapes():
         assert e.shape == (32,) and e.dtype == torch.float64
         gx, gc = torch.ops.mbxgpu.nmer_energies_backward(e, x, c, "mbpol3b", False)
         assert gx.shape == x.shape and gc.shape == c.shape
+
+
+def test_evaluate_async_waits_on_a_stream_of_its_own(monkeypatch):
+    """Without waiting only where the context runs on torch's current stream."""
+    import types
+
+    import torch
+    from mbx_b200 import capi
+
+    calls, synced = [], []
+
+    class Library:
+        def mbx_evaluate(self, h, name, n, x, g, v, e, energy, flags):
+            calls.append(flags)
+            return 0
+
+    current = types.SimpleNamespace(cuda_stream=0, synchronize=lambda: synced.append(1))
+    monkeypatch.setattr(capi, "lib", Library)
+    monkeypatch.setattr(capi, "evaluator_info", lambda name: (2, 6, 31, 1153))
+    monkeypatch.setattr(capi, "_ptr", lambda a: (None, None) if a is None else (1, True))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: current)
+    x = torch.zeros(4, 18)
+    # (context's stream, torch's current stream): 0 is a stream of the
+    # context's own, 1 the legacy default stream, whose handle torch gives as 0
+    for mine, other, same in ((1, 0, True), (77, 77, True), (0, 0, False), (1, 77, False), (77, 0, False)):
+        c = capi.Context.__new__(capi.Context)
+        c.h, c.device, c.stream = None, 0, mine
+        current.cuda_stream = other
+        calls.clear()
+        synced.clear()
+        c.evaluate_async("mbpol2b", x, None, x)
+        assert [bool(f & capi.MBX_NO_WAIT) for f in calls] == [same]
+        assert bool(synced) == (not same)

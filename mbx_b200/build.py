@@ -31,10 +31,14 @@ LIB = os.path.join(PKG, "libmbx_b200.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-# (--compress-mode=size: the straight-line code with its line tables would make
-# the library 190 MB; compressed it has 56 MB, 26 of them tables)
-FLAGS = ["-O3", "-lineinfo", "--compress-mode=size", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+FLAGS = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
+# The straight-line units get no line tables and stay uncompressed: the first
+# context of a process loads the coefficients of every evaluator, and with
+# them its code.  That took 260 ms with line tables and compression (library
+# of 56 MB), 110 ms with compression alone (40 MB), 47 ms with neither (79 MB).
+GEN_FLAGS = ["--compress-mode=none"]
+HAND_FLAGS = ["-lineinfo"]
 HAND = ("mbx_capi.cu", "nmer_build.cu", "peaks.cu", "noalloc.cu", "table_kernels.cu", "onebody.cu")
 HEADERS = ("holder_common.cuh", "holder_kernel.cuh", "term_table.cuh", "launch_cache.cuh", "device_state.h",
            "qf_kernel.cuh")
@@ -70,7 +74,8 @@ def compile_one(src, verbose):
     if src.endswith(".cpp"):
         cmd = ["g++", "-O2", "-fPIC", "-c", src, "-o", obj + ".tmp"]
     else:
-        cmd = [NVCC] + ARCH + FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-c", src, "-o", obj + ".tmp"]
+        own = GEN_FLAGS if os.path.dirname(src) == GEN else HAND_FLAGS
+        cmd = [NVCC] + ARCH + FLAGS + own + (["-Xptxas", "-v"] if verbose else []) + ["-c", src, "-o", obj + ".tmp"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         return obj, r.stderr[-6000:], time.time() - t0

@@ -203,6 +203,27 @@ static std::vector<double> w_coefficients(int table, const double* a) {
     return c;
 }
 
+// The w coefficients of all evaluators' fitted ones, in the layout of
+// DeviceTables::cw, summed once per process (8 ms).  Caller holds g_dev_mu.
+static const std::vector<double>& fitted_w_coefficients() {
+    static std::vector<double> all;
+    if (all.empty()) {
+        coef_layout();
+        all.resize(g_cw_total);
+        auto put = [&](int table, const double* fit, long off) {
+            const std::vector<double> c = w_coefficients(table, fit);
+            std::copy(c.begin(), c.end(), all.begin() + off);
+        };
+        for (int i = 0; i < mbx_num_evaluators; ++i) {
+            const EvaluatorInfo& E = mbx_evaluators[i];
+            put(E.table, E.fit, g_cw_off[i]);
+            if (E.ptable != E.table) put(E.ptable, E.fit, g_cp_off[i]);
+        }
+        for (int i = 0; i < mbx_num_onebody; ++i) put(mbx_onebody[i].table, mbx_onebody[i].fit, g_cw_off_1b[i]);
+    }
+    return all;
+}
+
 // (a warp per row: each lane a strand of the row, the strands joined in order)
 __global__ void k_w_coefficients(const int* __restrict__ row, const int* __restrict__ k, const double* __restrict__ f,
                                  int ncw, const double* __restrict__ a, double* __restrict__ c) {
@@ -243,15 +264,13 @@ static int device_constants_locked(int dev) {
     if (cudaGetDevice(&cur) != cudaSuccess) return MBX_ENODEV;
     if (cur != dev && cudaSetDevice(dev) != cudaSuccess) return MBX_ECUDA;
     int rc = MBX_OK;
+    const std::vector<double>& c = fitted_w_coefficients();
     for (int i = 0; i < mbx_num_evaluators && rc == MBX_OK; ++i) {
         const EvaluatorInfo& E = mbx_evaluators[i];
         if (E.kern != i) continue;   // an alias shares its target's kernels and coefficients
-        const std::vector<double> c = w_coefficients(E.table, E.fit);
         for (int v = 0; v < 2; ++v)
-            if (E.set[v] && E.set[v](c.data(), 0, nullptr) != 0) rc = MBX_ECUDA;
+            if (E.set[v] && E.set[v](c.data() + g_cw_off[i], 0, nullptr) != 0) rc = MBX_ECUDA;
         if (E.set_s && E.set_s(E.fit, 0, nullptr) != 0) rc = MBX_ECUDA;
-        // c and the staging of its copies must outlive them
-        if (cudaStreamSynchronize(nullptr) != cudaSuccess) rc = MBX_ECUDA;
     }
     if (rc == MBX_OK && cudaDeviceSynchronize() != cudaSuccess) rc = MBX_ECUDA;
     if (rc == MBX_OK) g_dev_constants[dev] = true;
@@ -282,19 +301,12 @@ int mbx_device_tables(int dev, DeviceTables* out) {
         if (e == cudaSuccess) e = cudaMalloc(&cw, (size_t)g_cw_total * sizeof(double));
         if (e == cudaSuccess) e = cudaMemcpy(blob, mbx_terms_blob, (size_t)mbx_terms_bytes, cudaMemcpyHostToDevice);
         // the fitted coefficients of all evaluators, in one copy each
-        std::vector<double> ha(g_coef_total), hc(g_cw_total);
-        auto put = [&](int table, const double* fit, int ncoef, long off, long off_cw) {
-            std::copy(fit, fit + ncoef, ha.begin() + off);
-            const std::vector<double> c = w_coefficients(table, fit);
-            std::copy(c.begin(), c.end(), hc.begin() + off_cw);
-        };
-        for (int i = 0; i < mbx_num_evaluators; ++i) {
-            const EvaluatorInfo& E = mbx_evaluators[i];
-            put(E.table, E.fit, E.ncoef, g_coef_off[i], g_cw_off[i]);
-            if (E.ptable != E.table) put(E.ptable, E.fit, E.ncoef, g_coef_off[i], g_cp_off[i]);
-        }
+        std::vector<double> ha(g_coef_total);
+        const std::vector<double>& hc = fitted_w_coefficients();
+        for (int i = 0; i < mbx_num_evaluators; ++i)
+            std::copy(mbx_evaluators[i].fit, mbx_evaluators[i].fit + mbx_evaluators[i].ncoef, ha.begin() + g_coef_off[i]);
         for (int i = 0; i < mbx_num_onebody; ++i)
-            put(mbx_onebody[i].table, mbx_onebody[i].fit, mbx_onebody[i].ncoef, g_coef_off_1b[i], g_cw_off_1b[i]);
+            std::copy(mbx_onebody[i].fit, mbx_onebody[i].fit + mbx_onebody[i].ncoef, ha.begin() + g_coef_off_1b[i]);
         if (e == cudaSuccess) e = cudaMemcpy(coef, ha.data(), ha.size() * sizeof(double), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(cw, hc.data(), hc.size() * sizeof(double), cudaMemcpyHostToDevice);
         if (cur != dev) cudaSetDevice(cur);

@@ -40,7 +40,7 @@ FLAGS = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
 GEN_FLAGS = ["--compress-mode=none"]
 HAND_FLAGS = ["-lineinfo"]
 HAND = ("mbx_capi.cu", "nmer_build.cu", "peaks.cu", "noalloc.cu", "table_kernels.cu", "onebody.cu")
-HEADERS = ("holder_common.cuh", "holder_kernel.cuh", "term_table.cuh", "launch_cache.cuh", "device_state.h",
+HEADERS = ("holder_common.cuh", "holder_kernel.cuh", "term_table.cuh", "launch_cache.cuh", "device_state.h", "table_kernels.h",
            "qf_kernel.cuh")
 
 
@@ -52,7 +52,7 @@ def deps(src):
     if os.path.dirname(src) == GEN:
         name, v = base[:-3].rsplit("_", 1)
         common.append(os.path.join(GEN, name + ".cuh"))
-        for variant in {"g": ("pip",), "e": ("pip_e",), "s": ("pip_s32", "qf")}.get(v, ()):
+        for variant in {"g": ("pip",), "e": ("pip_e",), "s": ("qf",)}.get(v, ()):
             common.append(os.path.join(GEN, "%s_%s.cuh" % (name, variant)))
     else:
         common += [os.path.join(CSRC, "nmer_build.h"), os.path.join(ROOT, "include", "mbx_b200.h"),

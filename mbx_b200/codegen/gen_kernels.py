@@ -9,8 +9,8 @@ For each evaluator in ``mbx_b200.specs.SPECS`` this writes
 * ``<name>_pip``: the polynomial and its reverse-mode gradient, as a
   multivariate Horner trie over the expanded term table;
 * ``<name>_pip_e``: the energy-only Horner evaluation;
-* ``<name>_pip_s32`` (types in SHIFT_TYPES): the FP32 trie of the type's FP32
-  basis (codegen/shift.py), the mixed-precision polynomial.
+* ``<name>_qf`` (types in QF_TYPES): the quadratic form of the type's FP32
+  basis (codegen/shift.py, codegen/qf.py), the mixed-precision polynomial.
 
 The tries are those of the polynomial in the symmetry-adapted variables w
 (codegen/wbasis.py), which has 3 to 8 times fewer terms than in the variables
@@ -61,8 +61,9 @@ class Trie:
     """The monomials as a tree.  At every node the variable that occurs in
     the most of the remaining monomials is split off first (a multivariate
     Horner scheme): fewer inner nodes than one variable order for the whole
-    tree (MB-pol 3b: 1274 against 2249, 16.0k against 19.4k FP64 operations
-    per trimer)."""
+    tree (MB-pol 3b: 1390, 17.5k FP64 operations a trimer; with the variables
+    in the order of the model 2611 and 20.5k, the rarest first 2137 and
+    18.4k)."""
 
     def __init__(self, table):
         self.root = self._node([(table.var[t, :table.deg[t]].tolist(), (int(table.k[t]), float(table.coef[t])))
@@ -396,7 +397,7 @@ def emit_vars(spec, out):
     w("}")
 
 
-def emit_traits(spec, table, straight, npieces, out):
+def emit_traits(spec, straight, npieces, out):
     """Compile-time description the kernel templates in holder_kernel.cuh use."""
     w = out.append
     n = spec.name
@@ -404,14 +405,13 @@ def emit_traits(spec, table, straight, npieces, out):
     first = [0, nat[0], nat[0] + nat[1]]
     ns = len(spec.sites)
     w("struct %s_T {" % n)
-    w("    static constexpr int NBODY = %d, NVARS = %d, NREAL = %d, NSITES = %d, NCOEF = %d;" %
-      (spec.nbody, spec.nvars, spec.nreal, ns, spec.ncoef))
+    w("    static constexpr int NBODY = %d, NVARS = %d, NREAL = %d, NSITES = %d;" %
+      (spec.nbody, spec.nvars, spec.nreal, ns))
     w("    static constexpr int NAT0 = %d, NAT1 = %d, NAT2 = %d;" % tuple(nat))
     w("    static constexpr int FIRST0 = %d, FIRST1 = %d, FIRST2 = %d;" % tuple(first))
-    w("    static constexpr int SWITCH_TRIPLE = %d, SKIP = %d, DEGREE = %d;" %
+    w("    static constexpr int SWITCH_TRIPLE = %d, SKIP = %d;" %
       ({"pair": 0, "triple": 1, "triple2": 2, "cos2": 3, "none": 0}[spec.switch],
-       {"pair_gt": 0, "two_of_three_gt": 1, "all_three_gt": 2, "none": 0}[spec.skip],
-       spec.degree))
+       {"pair_gt": 0, "two_of_three_gt": 1, "all_three_gt": 2, "none": 0}[spec.skip]))
     w("    static constexpr int TPAIRS = %d;  // (variable, exponent) pairs of a term, at most" %
       term_pairs_max(table_key(n)))
     w("    static constexpr double RI = %s, RF = %s;" % (lit(spec.ri), lit(spec.rf)))
@@ -419,16 +419,10 @@ def emit_traits(spec, table, straight, npieces, out):
       (1 if spec.virial == "raw" else 0))
     w("    static constexpr int LOCK_THREADS = %d;  // threads of a lockstep evaluation block" %
       lock_threads(spec.nvars))
-    shifted_type = straight and n in SHIFT_TYPES
-    w("    static constexpr int SHIFTED = %d, LOCK_THREADS_S = %d;  // paired FP32 (shifted-basis) kernel" %
-      (1 if shifted_type else 0, 256 if shifted_type else lock_threads(spec.nvars)))
-    w("    static constexpr int NORB = %d;  // coefficients of the FP32 basis" %
-      (shifted_pip(n).norb if shifted_type else 1))
-    w("    static constexpr int NCW = %d;  // coefficients of the polynomial in the w variables" % wtable(n).ncoef)
     w("    __device__ __forceinline__ static void to_w(double (&x)[%d]) { %s_to_w(x); }" % (spec.nvars, n))
-    w("    __device__ __forceinline__ static void from_w(double (&g)[%d]) { %s_from_w(g); }" % (spec.nvars, n))
-
-    if shifted_type:
+    if not straight:
+        w("    __device__ __forceinline__ static void from_w(double (&g)[%d]) { %s_from_w(g); }" % (spec.nvars, n))
+    if straight and n in SHIFT_TYPES:
         w("    __device__ __forceinline__ static void shift(const double (&x)[%d], float (&xf)[%d]) "
           "{ %s_shift(x, xf); }" % (spec.nvars, spec.nvars, n))
     w("    __device__ __forceinline__ static void sites(const double (&r)[%d][3], double (&s)[%d][3]) { %s_sites(r, s); }" %
@@ -474,14 +468,13 @@ def generate(name):
     head = ["// Generated by mbx_b200/codegen/gen_kernels.py from mbx_b200/specs.py and",
             "// mbx_b200/data/%s.pip.gz -- do not edit." % name]
     out = head + ["// %d terms: %d leaves, %d inner nodes" % (table.nterms, leaves, inner),
-                  "#pragma once",
-                  "#define %s_STRAIGHT_LINE %d" % (name.upper(), 1 if straight else 0)]
+                  "#pragma once"]
     emit_vars(spec, out)
     nv = spec.nvars
     nparts = parts_for(wt.nterms, nv) if straight else 0
     npieces = len(split_terms(trie, nparts)) if straight else 0
     out.append("// %d terms in the w variables" % wt.nterms)
-    emit_transforms(wt, name, out)
+    emit_transforms(wt, name, out, back=not straight)
     if straight:
         emit_chain(wt, spec, out)
         out += ["template <int S, class Coef> __device__ __forceinline__ double %s_pip_piece(int, const Coef&, "
@@ -499,7 +492,7 @@ def generate(name):
                 else:
                     out.append("    xf[%d] = (float)(x[%d] - %s);" % (v, v, lit(float(sp.x0[v]))))
             out.append("}")
-    emit_traits(spec, table, straight, npieces, out)
+    emit_traits(spec, straight, npieces, out)
     os.makedirs(OUT, exist_ok=True)
     write_if_changed(os.path.join(OUT, name + ".cuh"), "\n".join(out) + "\n")
     if straight:

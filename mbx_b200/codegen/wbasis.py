@@ -369,9 +369,9 @@ def wtable(name):
     return by_key(table_key(name))
 
 
-def emit(w, name, out):
-    """CUDA code of the two transforms, NAME_to_w (x -> w = W x - w0 in place) and
-    NAME_from_w (dP/dw -> dP/dx in place)."""
+def emit(w, name, out, back):
+    """CUDA code of the transform NAME_to_w (x -> w = W x - w0 in place) and,
+    with back, of NAME_from_w (dP/dw -> dP/dx in place)."""
     nv = w.nvars
 
     def rows(M, w0):
@@ -385,7 +385,7 @@ def emit(w, name, out):
             text.append("    x[%d] = %s;" % (i, " ".join("%s %s" % p for p in parts).lstrip("+ ")))
         return text
 
-    for fn, M, w0 in (("to_w", w.W, w.w0), ("from_w", w.W.T, np.zeros(nv))):
+    for fn, M, w0 in (("to_w", w.W, w.w0), ("from_w", w.W.T, np.zeros(nv)))[:2 if back else 1]:
         out.append("__device__ __forceinline__ void %s_%s(double (&x)[%d]) {" % (name, fn, nv))
         text = rows(M, w0)
         if text:

@@ -46,8 +46,7 @@ struct HolderArgs {
     const int* n_dev;          // optional device-side count (read by the kernel, clamped to n)
     const int* status;         // optional: a nonzero word means the n-mer build failed; do nothing
     int* counter;              // work counter (zeroed before the launch): blocks claim units (LockPlan)
-    int split;                 // 1: the last round's chunks may be cut by trie pieces (sums in another order;
-                               // e_per, where given, zeroed before the launch)
+    int split;                 // system input, 1: the last round's chunks may be cut by trie pieces (sums in another order)
     const int4* nmers;         // system input: (m0, m1, m2, anchor slot), holder order
     const double* xyz;         // system input: site array (3 per site); AoS input: [n][NREAL*3]
     const int* first_index;    // system input: first site of every monomer
@@ -277,12 +276,12 @@ __device__ __forceinline__ void chain_rule(const double (&s)[T::NSITES][3], cons
 }
 
 // Everything after the polynomial: chain rule, switch, virial, scatter.  g:
-// dP/dv as chain_rule takes it.  share: ep and g are a part of the n-mer's
-// polynomial whose rest is added by other threads (per-n-mer outputs by
-// atomics, e_per zeroed before the launch).
+// dP/dv as chain_rule takes it.  For system input ep and g may be a part of
+// the n-mer's polynomial whose rest other threads add (LockPlan): all it
+// writes are sums.
 template <class T, class G>
 __device__ __forceinline__ void finish_nmer(const HolderArgs& A, long t, double ep, const G& g, bool grads,
-                                            double (&acc)[7], bool share = false) {
+                                            double (&acc)[7]) {
     double r[T::NREAL][3];
     load_nmer<T, true>(A, t, r);
     double d[3][3], rr[3];
@@ -322,10 +321,7 @@ __device__ __forceinline__ void finish_nmer(const HolderArgs& A, long t, double 
         if (!T::VIRIAL_RAW) virial();
     }
     const double es = sw * ep;
-    if (A.e_per) {
-        if (share) atomicAdd(A.e_per + t, es);
-        else A.e_per[t] = es;
-    }
+    if (A.e_per) A.e_per[t] = es;
     v[0] = es;
     if (A.conf_out) {
         conf_accumulate(A.conf_out + 8 * __ldg(A.mon_conf + __ldg(A.nmers + t).x), v);
@@ -339,10 +335,7 @@ __device__ __forceinline__ void finish_nmer(const HolderArgs& A, long t, double 
 #pragma unroll
         for (int i = 0; i < T::NREAL; ++i)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                if (share) atomicAdd(p + 3 * i + c, tg[i][c]);
-                else p[3 * i + c] += tg[i][c];
-            }
+            for (int c = 0; c < 3; ++c) p[3 * i + c] += tg[i][c];
         return;
     }
     const int4 nm = __ldg(A.nmers + t);
@@ -472,7 +465,6 @@ __global__ void __launch_bounds__(T::LOCK_THREADS, 1) holder_lock_kernel(const H
         if (u >= plan.units) break;
         int k0, k1;
         const long t = plan.unit(u, NP, k0, k1) * L + threadIdx.x;
-        const bool shared_nmer = k1 - k0 < NP;   // other blocks hold the rest of this n-mer's polynomial
         bool live = t < n;
         {
             double x[T::NVARS];
@@ -505,7 +497,7 @@ __global__ void __launch_bounds__(T::LOCK_THREADS, 1) holder_lock_kernel(const H
             if (busy) ep += piece(k, xs, gs);
             __syncthreads();
         }
-        if (live) finish_nmer<T>(A, t, ep, WColumns<L>{xs, gs}, grads, acc, shared_nmer);
+        if (live) finish_nmer<T>(A, t, ep, WColumns<L>{xs, gs}, grads, acc);
         u += gridDim.x;
     }
     block_reduce_add<7>(acc, A.out);
@@ -594,9 +586,11 @@ __global__ void __launch_bounds__(128, 3) pair_finish_kernel(const HolderArgs A)
 
 // 1-body MB-nrg evaluation (x1b_*::eval, e.g. x1b_A1B4_v1x::eval,
 // potential/1b/x1b_A1B4_deg5_exp0_v1x.cpp:361-419): no image, no switch, no
-// cutoff.  A lane per monomer, the warp walking the term table in step (as
-// holder_table_lane_kernel); variables, chain rule and the virial
-// -sum r (x) g over the monomer's atoms as the reference's evaluator does.
+// cutoff.  A lane per monomer, the warp walking the term table in step, every lane
+// applying each term to its own monomer, whose variables and gradient
+// accumulators sit in shared-memory columns [v][lane]; variables, chain rule
+// and the virial -sum r (x) g over the monomer's atoms as the reference's
+// evaluator does.
 // A.first_index: first site of each monomer to evaluate (A.n of them); one
 // thread per monomer writes its gradient, so no atomics.  Dynamic shared
 // memory: 4 warps x 2 x NVARS x 32 doubles.

@@ -23,6 +23,7 @@
 #include "../../include/mbx_b200.h"
 #include "holder_kernel.cuh"
 #include "nmer_build.h"
+#include "table_kernels.h"
 
 // The 1-body term of water (onebody.cu).
 struct OneBodyArgs {
@@ -33,35 +34,6 @@ struct OneBodyArgs {
     double* out;
 };
 int mbx_launch_ps1b(const OneBodyArgs& A, int sms, cudaStream_t s);
-
-// Generic table-driven polynomial over caller-supplied variables
-// (table_kernels.cu).
-struct PolyTable {
-    const int4* terms;
-    const double* tcoef;
-    long nterms;
-    int pairs;
-    const double* coef;
-    const int *wrow, *w, *wtrow, *wt;
-    const double* w0;
-};
-int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double* e, const PolyTable& P, int sms,
-                          cudaStream_t s);
-
-// Coefficient adjoint over n-mers whose w variables are in wv (table_kernels.cu).
-struct AdjointTable {
-    const int4* terms;
-    const double* tcoef;
-    int nterms, nhalf, nvars, ncoef, ncw;
-    const int2* half;
-    const unsigned* pair;
-    const int* term;
-    const int *first, *ftrow, *ftk;
-    const double* ftf;
-};
-int mbx_coef_adjoint_blocks(const AdjointTable& P, int sms);
-int mbx_launch_coef_adjoint(const double* wv, int count, const AdjointTable& P, double* work, double* out, int sms,
-                            cudaStream_t s);
 
 typedef int (*launch_fn)(const HolderArgs&, int, int, cudaStream_t);
 typedef int (*dcoef_fn)(const HolderArgs&, const double*, long, int, double*, cudaStream_t);
@@ -80,7 +52,7 @@ struct EvaluatorInfo {
     dcoef_fn c;       // variables of the coefficient adjoint
     launch_fn s;      // FP32 kernel of the mixed mode (FP32 basis), or null
     double split_r;   // mixed mode: n-mers with first-atom distance below this run in FP64 (0: none)
-    prime_fn pg, pe, ps;   // code prefetch of the g, e and s kernels (holder_prime_kernel), or null
+    prime_fn pg, pe, ps;   // code prefetch of the g, e and s kernels (prime_pieces), or null
     setcoef_fn set[2];     // constant-memory coefficient setters of the g and e kernels (w coefficients)
     setcoef_fn set_s;      // of the s kernel (fitted coefficients), or null
     int table;        // term table (mbx_term_tables) of the kernels
@@ -1851,7 +1823,7 @@ extern "C" int mbx_evaluate_dcoef(mbx_ctx* c, const char* name, long n, const do
         constexpr long kAdjointChunk = 32768;
         const TermTableInfo& T = mbx_term_tables[E->table];
         const int chunk = (int)std::min(n, kAdjointChunk);
-        const AdjointTable P{A.terms, A.tcoef, (int)A.nterms, T.nhalf, E->nvars, E->ncoef, T.ncw,
+        const AdjointTable P{A.tcoef, (int)A.nterms, T.nhalf, E->nvars, E->ncoef, T.ncw,
                              reinterpret_cast<const int2*>(c->tables.blob + T.off_half),
                              reinterpret_cast<const unsigned*>(c->tables.blob + T.off_pair),
                              reinterpret_cast<const int*>(c->tables.blob + T.off_term),

@@ -13,22 +13,11 @@
 #include <cuda_runtime.h>
 
 #include "launch_cache.cuh"
+#include "table_kernels.h"
 #include "term_table.cuh"
 
 #define MBX_POLY_WARPS 4
 #define MBX_POLY_MAXV 128
-
-// The term table of a polynomial in the w variables, its coefficients c = F a,
-// and the rows of W (w = W x - w0) and of its transpose: entry +-(column + 1).
-struct PolyTable {
-    const int4* terms;
-    const double* tcoef;
-    long nterms;
-    int pairs;
-    const double* coef;
-    const int *wrow, *w, *wtrow, *wt;
-    const double* w0;
-};
 
 namespace {
 
@@ -112,17 +101,6 @@ int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double
 #define MBX_ADJ_THREADS 512
 #define MBX_ADJ_N 8
 #define MBX_ADJ_Q 8
-
-struct AdjointTable {
-    const int4* terms;
-    const double* tcoef;
-    int nterms, nhalf, nvars, ncoef, ncw;
-    const int2* half;
-    const unsigned* pair;     // half-monomials of the terms, in the order of the first one
-    const int* term;          // the terms in that order
-    const int *first, *ftrow, *ftk;   // first term of every coefficient; rows of F transposed
-    const double* ftf;
-};
 
 extern __shared__ __align__(16) double mbx_adj_smem[];
 
@@ -230,7 +208,6 @@ int mbx_coef_adjoint_blocks(const AdjointTable& P, int sms) {
     return (2 * sms + ny - 1) / ny;
 }
 
-// work: (mbx_coef_adjoint_blocks + 1) * nterms + ncw doubles
 int mbx_launch_coef_adjoint(const double* wv, int count, const AdjointTable& P, double* work, double* out, int sms,
                             cudaStream_t s) {
     const size_t smem = ((size_t)(P.nvars + 1) * MBX_ADJ_N + 2 * (size_t)P.nhalf * (MBX_ADJ_N + 1)) * sizeof(double);

@@ -151,6 +151,10 @@ int mbx_poly(mbx_ctx* ctx, const char* evaluator, long nd, const double* x, doub
 int mbx_qf_image(const char* evaluator, const double* coef, long* image_bytes, int* nb, unsigned char* image,
                  float* colf, double* b0);
 
+/* The same operands as they are on the context's device now (all three
+ * arrays required, of the sizes above). */
+int mbx_qf_device_image(mbx_ctx* ctx, const char* evaluator, unsigned char* image, float* colf, double* b0);
+
 /* Replace the linear coefficients of an evaluator (ncoef doubles; NULL
  * restores the fitted ones).  Coefficients are per device, not per context:
  * they live in the kernels' constant memory and in one global-memory copy

@@ -88,6 +88,7 @@ def lib():
                                         ctypes.POINTER(ctypes.c_double), ctypes.c_int]
     L.mbx_get_knobs.argtypes = [vp, ctypes.c_int, ip]
     L.mbx_set_knobs.argtypes = [vp, ctypes.c_int, ip]
+    L.mbx_qf_device_image.argtypes = [vp, ctypes.c_char_p, ctypes.c_void_p, ctypes.POINTER(ctypes.c_float), dp]
     L.mbx_qf_image.argtypes = [ctypes.c_char_p, dp, lp, ip, ctypes.c_void_p, ctypes.POINTER(ctypes.c_float), dp]
     _lib = L
     return L
@@ -97,7 +98,8 @@ EXPORTED = ("mbx_create", "mbx_destroy", "mbx_last_error", "mbx_version", "mbx_s
             "mbx_energy", "mbx_last_counts", "mbx_nmers", "mbx_evaluate", "mbx_evaluate_dcoef", "mbx_poly",
             "mbx_set_coefficients", "mbx_evaluator_info", "mbx_last_timing", "mbx_fma_peaks", "mbx_set_batch",
             "mbx_batch_energy", "mbx_tune", "mbx_get_knobs", "mbx_set_knobs", "mbx_energy_2b3b",
-            "mbx_batch_energy_2b3b", "mbx_set_ignore_1b", "mbx_set_real_order", "mbx_energy_real", "mbx_qf_image")
+            "mbx_batch_energy_2b3b", "mbx_set_ignore_1b", "mbx_set_real_order", "mbx_energy_real", "mbx_qf_image",
+            "mbx_qf_device_image")
 
 KNOBS = ("nb_warps", "nb_unroll", "tri_threads", "dim_threads")
 
@@ -347,6 +349,14 @@ class Context:
         self._check(lib().mbx_evaluate_dcoef(self.h, name.encode(), n, px, pw, po,
                                              MBX_DEVICE_PTRS if dx else 0))
         return out
+
+    def qf_device_image(self, name):
+        """qf_image() of the coefficients that are set, read back from the device."""
+        img, colf, _ = qf_image(name)
+        img, colf, b0 = np.zeros(len(img), np.uint8), np.zeros_like(colf), ctypes.c_double()
+        self._check(lib().mbx_qf_device_image(self.h, name.encode(), img.ctypes.data,
+                                              colf.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), ctypes.byref(b0)))
+        return img.tobytes(), colf, b0.value
 
     def poly(self, name, x, g=None, e=None):
         """Generated polynomial, variable-major x[nvars][nd] (poly_*::eval(nd, a, x, t, g))."""

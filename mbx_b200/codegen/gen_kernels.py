@@ -885,6 +885,14 @@ int mbx_set_coef_%(name)s_s(const double* a, int from_device, cudaStream_t s) {
     return (int)e;
 }
 
+// The operands as they are on the current device.
+int mbx_qf_device_image_%(name)s(unsigned char* img, float* colf, double* b0) {
+    cudaError_t e = cudaMemcpyFromSymbol(img, qf_img_%(name)s, (size_t)%(name)s_Q::IMAGE_BYTES);
+    if (e == cudaSuccess) e = cudaMemcpyFromSymbol(colf, qf_colf_%(name)s, sizeof(float) * %(name)s_Q::NB);
+    if (e == cudaSuccess) e = cudaMemcpyFromSymbol(b0, qf_b0_%(name)s, sizeof(double));
+    return (int)e;
+}
+
 int mbx_launch_%(name)s_s(const HolderArgs& A, int grid, int block, cudaStream_t s) {
     // three kernels: the FP64 variables shifted to the FP32 basis at full
     // occupancy (pair_vars_kernel), the quadratic form on the tensor cores
@@ -1198,13 +1206,16 @@ def write_registry():
     # host builders of the tensor-core operands of the mixed mode (QF_TYPES)
     from mbx_b200.codegen import qf as qfmod
     lines.append("struct QfInfo { const char* name; long image_bytes; int nb; "
-                 "int (*build)(const double*, unsigned char*, float*, double*); };")
+                 "int (*build)(const double*, unsigned char*, float*, double*); "
+                 "int (*device)(unsigned char*, float*, double*); };")
     for name in sorted(QF_TYPES):
         lines.append("int mbx_qf_image_%s(const double* a, unsigned char* img, float* colf, double* b0);" % name)
+        lines.append("int mbx_qf_device_image_%s(unsigned char* img, float* colf, double* b0);" % name)
     lines.append("static const QfInfo mbx_qf_types[] = {")
     for name in sorted(QF_TYPES):
         q = qfmod.QuadForm(name, shifted_pip(name))
-        lines.append('    {"%s", %dL, %d, mbx_qf_image_%s},' % (name, qfmod.image_bytes(q), q.npad, name))
+        lines.append('    {"%s", %dL, %d, mbx_qf_image_%s, mbx_qf_device_image_%s},' %
+                     (name, qfmod.image_bytes(q), q.npad, name, name))
     lines.append("};")
     lines.append("static const int mbx_num_qf_types = %d;" % len(QF_TYPES))
     # 1-body evaluators (table-driven), by monomer id

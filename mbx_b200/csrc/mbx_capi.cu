@@ -1865,6 +1865,19 @@ extern "C" int mbx_qf_image(const char* name, const double* coef, long* image_by
     return MBX_ENOTSUP;
 }
 
+extern "C" int mbx_qf_device_image(mbx_ctx* c, const char* name, unsigned char* image, float* colf, double* b0) {
+    if (!c || !name || !image || !colf || !b0) return fail(c, MBX_EINVAL, "bad arguments");
+    const EvaluatorInfo* E = find_evaluator(name);
+    for (int i = 0; E && i < mbx_num_qf_types; ++i) {
+        const QfInfo& Q = mbx_qf_types[i];
+        if (strcmp(Q.name, mbx_evaluators[E->kern].name) != 0) continue;
+        CUCHK(c, cudaSetDevice(c->device));
+        RCHK(c, Q.device(image, colf, b0));
+        return MBX_OK;
+    }
+    return fail(c, MBX_ENOTSUP, std::string("no tensor-core operands for ") + name);
+}
+
 extern "C" int mbx_poly(mbx_ctx* c, const char* name, long nd, const double* x, double* g, double* e, int flags) {
     if (!c || !name || nd < 0 || (nd > 0 && (!x || !e))) return fail(c, MBX_EINVAL, "bad arguments");
     const EvaluatorInfo* E = find_evaluator(name);

@@ -176,9 +176,11 @@ def lock_threads(nvars):
     instructions more than for anything else, and a block's warps share every
     fetch, so as many warps as the columns of x and g leave room for in 227 KB
     of shared memory: 384 threads (168 registers) up to 36 variables, else 256
-    (255 registers), 128 above 56 variables.  MB-pol 3b gradients of 132k
-    trimers: 410 us with 384 threads, 475 with 320, 550 with 256; MB-pol 2b,
-    39k dimers: 81 us with 384, 109 with 256."""
+    (255 registers), 128 above 56 variables, where the columns of 256 do not
+    fit.  MB-pol 3b gradients of 132k trimers: 410 us with 384 threads, 475
+    with 320, 550 with 256; MB-pol 2b, 39k dimers: 81 us with 384, 109 with 256.
+    The energy kernels, which have the columns of x alone, take the same number;
+    more threads have not been measured there."""
     if nvars > 56:
         return 128
     return 384 if nvars <= 36 else 256
@@ -190,13 +192,12 @@ def parts_for(nterms, nvars=36):
     fit, and the code of a piece should stay small enough for the instruction
     cache that the warps of a lockstep block share.  Measured on 132k MB-pol 3b
     trimers (256 threads): 570, 550 and 564 us at 300, 600 and 900 terms a
-    piece.  Small batches are cut by pieces over the SMs (LockPlan), which asks
-    for no larger ones."""
+    piece; on 76k N2O5-H2O-H2O trimers, 78 variables (128 threads): 641, 574 and
+    562 us at 200, 600 and 1000.  Small batches are cut by pieces over the SMs
+    (LockPlan), which asks for no larger ones: MB-pol 2b, with 250, 400 and 600
+    terms a piece, takes 130, 125 and 120 us for 76k dimers, and a call on 8
+    waters 130, 131 and 136."""
     per = 400 if nvars <= 32 else 600
-    if nvars > 56:
-        # a piece loads every variable it uses into registers: fewer terms per
-        # piece for the widest polynomials
-        per = 200
     return max(1, (nterms + per - 1) // per)
 
 

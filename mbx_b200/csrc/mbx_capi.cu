@@ -892,10 +892,11 @@ static int prepare_buckets(mbx_ctx* c, int nbody, long nq_guess, long list_cap) 
 // Searches up to this many members and cells build their cell list in one
 // block (k_cells_small): the launches between four kernels cost more than the
 // other SMs would save.  A call for both terms, one block against four kernels:
-// 125 and 142 us for 8 waters, 198 and 208 for 256 (cluster), 257 and 262 for
-// 512 (box); from there the other way round, 346 and 333 for 1024 (box), 587
-// and 540 for 2048.
-constexpr int kSmallSearch = 512;
+// 125 and 142 us for 8 waters (cluster), 264 and 268 for 512 (box), 572 and 583
+// for 576 methanes and waters, 271 and 277 for 640 waters (box); from there
+// the other way round, 255 and 248 for 704 (cluster), 310 and 305 for 896 (box),
+// 587 and 540 for 2048.
+constexpr int kSmallSearch = 640;
 
 // One search: the monomers members[0..nmem) (global ids) searched around
 // the queries query[0..nq) (positions in members), in box bp.

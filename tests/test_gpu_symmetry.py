@@ -32,8 +32,8 @@ def test_chunks_cut_by_pieces(n):
         assert abs(eo - er) <= E_REL * abs(er) + E_ABS_NMER
 
 
-# one block of 1024 threads builds the cell list, up to 512 members
-@pytest.mark.parametrize("n", [511, 512, 513, 1023, 1024, 1025])
+# one block of 1024 threads builds the cell list, up to 640 members
+@pytest.mark.parametrize("n", [639, 640, 641, 1023, 1024, 1025])
 def test_search_around_one_block(n):
     edge = 39.44 * (n / 2048) ** (1 / 3)
     ids, xyz, box = workloads.water_box(12, n, edge, seed=n)

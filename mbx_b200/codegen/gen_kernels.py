@@ -44,7 +44,8 @@ sys.path.insert(0, os.path.dirname(PKG))
 
 from mbx_b200.specs import SPECS, ONEBODY_SPECS, LP_GAMMA_IN, LP_GAMMA_OUT  # noqa: E402
 from mbx_b200.tables import load_pip  # noqa: E402
-from mbx_b200.codegen.wbasis import by_key as wtable_by_key, emit as emit_transforms, emit_chain, table_key, wtable  # noqa: E402
+from mbx_b200.codegen.wbasis import (by_key as wtable_by_key, emit as emit_transforms, emit_chain,  # noqa: E402
+                                      prepare as prepare_tables, table_key, wtable)
 
 OUT = os.path.join(PKG, "csrc", "gen")
 
@@ -1249,6 +1250,7 @@ def main(argv=None, quiet=False):
     ap.add_argument("names", nargs="*", default=list(SPECS))
     args = ap.parse_args(argv)
     os.makedirs(OUT, exist_ok=True)
+    prepare_tables(table_names())
     write_registry()
     write_term_tables()
     write_ps1b()

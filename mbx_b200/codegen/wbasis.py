@@ -37,8 +37,13 @@ monomers is tried, and kept when it maps the variables (with their constants)
 and the term table onto themselves.
 """
 import collections
+import concurrent.futures
 import functools
 import itertools
+import os
+import pickle
+import subprocess
+import sys
 from fractions import Fraction
 
 import numpy as np
@@ -354,14 +359,44 @@ def table_key(name):
     return name if name in SHIFTED else spec.pip_table
 
 
-@functools.lru_cache(maxsize=None)
+_tables = {}
+
+
 def by_key(key):
     """WTable of a key: an evaluator of SHIFTED, or a term table (without a
     reference point, for caller-supplied variables)."""
-    if key in SHIFTED:
-        return WTable(key, True)
-    return WTable(next(n for n, spec in list(SPECS.items()) + list(ONEBODY_SPECS.items()) if spec.pip_table == key),
-                  False)
+    if key not in _tables:
+        name = key
+        if key not in SHIFTED:
+            name = next(n for n, spec in list(SPECS.items()) + list(ONEBODY_SPECS.items()) if spec.pip_table == key)
+        _tables[key] = WTable(name, key in SHIFTED)
+    return _tables[key]
+
+
+_ONE_TABLE = """
+import pickle, sys
+sys.path.insert(0, sys.argv[1])
+from mbx_b200.codegen.wbasis import by_key
+w = by_key(sys.argv[2])
+w.halves
+sys.stdout.buffer.write(pickle.dumps(w))
+"""
+
+
+def prepare(keys):
+    """Makes the WTables of the keys, half-monomials included, in processes of
+    their own side by side (all of them: 80 s in one process)."""
+    root = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+
+    def one(key):
+        r = subprocess.run([sys.executable, "-c", _ONE_TABLE, root, key], capture_output=True)
+        if r.returncode != 0:
+            raise RuntimeError("table %s:\n%s" % (key, r.stderr.decode()[-2000:]))
+        return key, pickle.loads(r.stdout)
+
+    todo = [k for k in keys if k not in _tables]
+    with concurrent.futures.ThreadPoolExecutor(os.cpu_count() or 4) as ex:
+        _tables.update(ex.map(one, todo))
 
 
 def wtable(name):

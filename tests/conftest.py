@@ -52,15 +52,19 @@ def ctx():
 
 # GPU suite order: the path itself first (evaluator goldens, boxes against the
 # reference, lists), then batching and the autograd wrapper; the
-# allocation-free entry point (tests/test_zz_no_alloc.py) stays last.  A run
+# allocation-free entry point (tests/test_zz_no_alloc.py) after all that.  A run
 # that stops at the first failure has then checked the path before anything
-# built on it.
-_ORDER = ("test_capi_load", "test_gpu_parity", "test_gpu_batch", "test_gpu_autograd", "test_cxx_boundary")
+# built on it.  The files that fail where the compiled reference is not built
+# come last, so that such a run has checked everything else.
+_ORDER = ("test_capi_load", "test_gpu_parity", "test_gpu_batch", "test_gpu_autograd")
+_LAST = ("test_oracle_goldens", "test_cxx_boundary")
 
 
 def pytest_collection_modifyitems(session, config, items):
     def rank(item):
         mod = item.module.__name__.rsplit(".", 1)[-1]
+        if mod in _LAST:
+            return len(_ORDER) + 2 + _LAST.index(mod)
         if mod.startswith("test_zz"):
             return len(_ORDER) + 1
         return _ORDER.index(mod) if mod in _ORDER else len(_ORDER)

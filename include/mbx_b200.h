@@ -129,7 +129,9 @@ int mbx_evaluate(mbx_ctx* ctx, const char* evaluator, long n, const double* xyz,
                  double* e_per, double* energy, int flags);
 
 /* Adjoint with respect to the linear coefficients: out[k] += sum_n w[n] *
- * dE_n/da_k (w may be NULL for all ones), monomials recomputed from xyz. */
+ * dE_n/da_k (w may be NULL for all ones), monomials recomputed from xyz.
+ * With device pointers the call returns once its work is enqueued on the
+ * context's stream. */
 int mbx_evaluate_dcoef(mbx_ctx* ctx, const char* evaluator, long n, const double* xyz, const double* w,
                        double* out, int flags);
 

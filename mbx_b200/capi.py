@@ -338,6 +338,8 @@ class Context:
         self._check(lib().mbx_evaluate(self.h, name.encode(), n, ptrs[0][0], ptrs[1][0], None, ptrs[2][0], None, flags))
 
     def evaluate_dcoef(self, name, xyz, w=None, out=None):
+        """out[k] += sum_n w[n] dE_n/da_k; with CUDA tensors ready on the
+        context's stream."""
         nb, nreal, nv, nc = evaluator_info(name)
         px, dx = _ptr(xyz)
         self._order(dx)

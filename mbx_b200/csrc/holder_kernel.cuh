@@ -673,7 +673,9 @@ __global__ void __launch_bounds__(128) onebody_table_kernel(const HolderArgs A) 
 // First step of the coefficient adjoint (coef_adjoint_kernel has the second):
 // the w variables of n-mers first .. first + count and, as row NVARS, their
 // weight times the switch (0 beyond the evaluator's cutoff), variable-major in
-// wv with stride count.  One n-mer per thread.
+// wv with stride count.  An n-mer without weight has zeros, so that it adds
+// nothing whatever its coordinates (padding with coincident atoms has infinite
+// variables).  One n-mer per thread.
 template <class T>
 __global__ void __launch_bounds__(128) holder_wvars_kernel(const HolderArgs A, const double* __restrict__ w,
                                                            long first, int count, double* __restrict__ wv) {
@@ -696,6 +698,6 @@ __global__ void __launch_bounds__(128) holder_wvars_kernel(const HolderArgs A, c
         scale = apply_switch<T>(d, rr, 0.0, tg, false) * (w ? w[t] : 1.0);
     }
 #pragma unroll
-    for (int v = 0; v < T::NVARS; ++v) wv[(size_t)v * count + i] = x[v];
+    for (int v = 0; v < T::NVARS; ++v) wv[(size_t)v * count + i] = scale != 0.0 ? x[v] : 0.0;
     wv[(size_t)T::NVARS * count + i] = scale;
 }

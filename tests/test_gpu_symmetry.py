@@ -117,6 +117,18 @@ def test_adjoint_is_the_energy_per_coefficient(ctx, name, n):
     assert np.all(np.abs(d - ref) <= 5e3 * 100 * 2.0 ** -53 * size)
 
 
+@pytest.mark.parametrize("name", ["mbpol2b", "mbpol3b", "clh2o3b"])
+def test_adjoint_of_weightless_nmers(ctx, name):
+    """N-mers of weight 0 add nothing, whatever their coordinates: padding with
+    all atoms at the origin has infinite variables."""
+    x = nmers(name, 64, 11)
+    w = np.random.default_rng(12).uniform(-1, 1, 64)
+    alone = ctx.evaluate_dcoef(name, x, w)
+    padded = ctx.evaluate_dcoef(name, np.concatenate([x, np.zeros_like(x)]), np.concatenate([w, np.zeros(64)]))
+    size = np.abs(w[:, None] * mo.holder_dcoef(name, x)).sum(0)
+    assert np.all(np.abs(padded - alone) <= 5e3 * 100 * 2.0 ** -53 * size)   # (sums in another order)
+
+
 @pytest.mark.parametrize("name", ["mbpol2b", "mbpol3b", "h2ona3b", "ch4h2o3b", "co2co22b"])
 def test_coefficients_from_host_and_device(ctx, name):
     import torch

@@ -95,9 +95,13 @@ int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double
 // block's n-mers, so that nothing is reduced across threads.  The blocks' sums
 // are added up in a fixed order (adjoint_terms_kernel), then the terms of
 // every coefficient (adjoint_coef_kernel) and F^T of those
-// (adjoint_out_kernel): the result is the same from call to call.  Bound by the shared-memory reads of two
-// doubles per term and n-mer, the second scattered, the first mostly the same
-// for a warp's lanes: 20000 MB-pol 3b trimers (7425 terms) 163 us, where walking the 33525 terms in x, a lane per n-mer, took 14 ms.
+// (adjoint_out_kernel): the result is the same from call to call.  Bound by
+// the shared-memory reads of two doubles per term and n-mer, the second
+// scattered, the first mostly the same for a warp's lanes: 20000 MB-pol 3b
+// trimers (7425 terms) 163 us, where walking the 33525 terms in x, a lane per
+// n-mer, took 14 ms.  Warps past the last term skip the products: a call for
+// 30000 dimers of 2226 terms (MB-pol 2b) takes 107 us, 122 with them; of 429
+// (Li-H2O) 57 and 83.
 #define MBX_ADJ_THREADS 512
 #define MBX_ADJ_N 8
 #define MBX_ADJ_Q 8
@@ -143,6 +147,7 @@ __global__ void __launch_bounds__(MBX_ADJ_THREADS)
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < MBX_ADJ_Q; ++q) {
+            if (t0 + q * MBX_ADJ_THREADS >= P.nterms) break;
             const double* a = zs + (pair[q] & 0xffff) * LD;
             const double* b = z + (pair[q] >> 16) * LD;
 #pragma unroll

@@ -631,6 +631,20 @@ int mbx_launch_%(name)s_c(const HolderArgs& A, const double* w, long first, int 
 }
 """
 
+# Polynomials of at most this many terms (MBX_SMALL_TERMS) have their whole
+# adjoint in one kernel.
+SMALL_TERMS = 32
+SMALL_TU = """
+int mbx_launch_%(name)s_d(const HolderArgs& A, const double* w, const AdjointTable& P, double* part, unsigned* ticket,
+                          double* out, int sms, cudaStream_t s) {
+    static_assert(%(nterms)d <= MBX_SMALL_TERMS, "terms");
+    const long need = (A.n + 127) / 128;
+    const int grid = (int)(need < 2L * sms ? (need > 0 ? need : 1) : 2L * sms);
+    holder_dcoef_small_kernel<%(name)s_T><<<grid, 128, 0, s>>>(A, w, P, part, ticket, out);
+    return (int)cudaGetLastError();
+}
+"""
+
 ONEBODY_TU = """// Generated by mbx_b200/codegen/gen_kernels.py -- do not edit.
 // Table-driven 1-body kernel of the %(name)s evaluator.
 #include <cstring>
@@ -653,6 +667,10 @@ int mbx_launch_%(name)s_o(const HolderArgs& A, int grid, int block, cudaStream_t
     return (int)cudaGetLastError();
 }
 """
+
+
+def has_small_adjoint(name):
+    return wtable(name).nterms <= SMALL_TERMS
 
 
 def variants_of(name):
@@ -969,7 +987,8 @@ def write_kernels_cu(name):
             continue
         path = os.path.join(OUT, "%s_%s.cu" % (name, v))
         if v == "t":
-            write_tu(path, TABLE_TU % {"name": name})
+            small = SMALL_TU % {"name": name, "nterms": wtable(name).nterms} if has_small_adjoint(name) else ""
+            write_tu(path, TABLE_TU % {"name": name} + small)
         else:
             what, body = VARIANTS[v]
             wt = wtable(name)
@@ -1176,6 +1195,9 @@ def write_registry():
         if "t" in vs:
             lines.append("int mbx_launch_%s_c(const HolderArgs& A, const double* w, long first, int count, double* wv, "
                          "cudaStream_t s);" % name)
+            if has_small_adjoint(name):
+                lines.append("int mbx_launch_%s_d(const HolderArgs& A, const double* w, const AdjointTable& P, "
+                             "double* part, unsigned* ticket, double* out, int sms, cudaStream_t s);" % name)
         fit = load_fit(name)
         lines.append("static const double mbx_fit_%s[%d] = {" % (name, len(fit)))
         for i in range(0, len(fit), 4):
@@ -1195,9 +1217,10 @@ def write_registry():
             # the table unit ("t") holds the coefficient adjoint ("c")
             have = ("t" in vs) if v == "c" else (v in vs)
             return ("mbx_%s_%s_%s" % (kind, kern, v)) if have else "nullptr"
-        lines.append('    {"%s", %d, {"%s", "%s", "%s"}, %s, %d, %d, %d, %d, mbx_fit_%s, %s, %s, %s, %s, %s,' %
+        small = "mbx_launch_%s_d" % kern if has_small_adjoint(kern) else "nullptr"
+        lines.append('    {"%s", %d, {"%s", "%s", "%s"}, %s, %d, %d, %d, %d, mbx_fit_%s, %s, %s, %s, %s, %s, %s,' %
                      (name, spec.nbody, ids[0], ids[1], ids[2], lit(spec.rf), skip, spec.ncoef, spec.nreal,
-                      spec.nvars, name, fn("g", "launch"), fn("e", "launch"), fn("c", "launch"),
+                      spec.nvars, name, fn("g", "launch"), fn("e", "launch"), fn("c", "launch"), small,
                       fn("s", "launch"), lit(MIXED_FP64_RADIUS.get(name, 0.0))))
         lines.append("     %s, %s, %s," % (fn("g", "prime"), fn("e", "prime"), fn("s", "prime")))
         lines.append("     {%s}, %s, %d, %d, %d}," %

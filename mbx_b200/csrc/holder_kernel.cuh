@@ -22,6 +22,7 @@
 // 1.05).
 #pragma once
 #include "holder_common.cuh"
+#include "table_kernels.h"
 #include "term_table.cuh"
 
 // Precision / output modes.
@@ -670,34 +671,113 @@ __global__ void __launch_bounds__(128) onebody_table_kernel(const HolderArgs A) 
     block_reduce_add<7>(acc, A.out);
 }
 
-// First step of the coefficient adjoint (coef_adjoint_kernel has the second):
-// the w variables of n-mers first .. first + count and, as row NVARS, their
-// weight times the switch (0 beyond the evaluator's cutoff), variable-major in
-// wv with stride count.  An n-mer without weight has zeros, so that it adds
-// nothing whatever its coordinates (padding with coincident atoms has infinite
-// variables).  One n-mer per thread.
+// The variables of an n-mer of AoS input in w and its weight times the switch
+// (0 beyond the evaluator's cutoff) for the coefficient adjoint.  An n-mer
+// without weight has zeros, so that it adds nothing whatever its coordinates
+// (padding with coincident atoms has infinite variables).
 template <class T>
-__global__ void __launch_bounds__(128) holder_wvars_kernel(const HolderArgs A, const double* __restrict__ w,
-                                                           long first, int count, double* __restrict__ wv) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const long t = first + i;
-    double x[T::NVARS];
-#pragma unroll
-    for (int v = 0; v < T::NVARS; ++v) x[v] = 0.0;
+__device__ __forceinline__ double adjoint_vars(const HolderArgs& A, const double* __restrict__ w, long t,
+                                               double (&x)[T::NVARS]) {
     double scale = 0.0;
     double r[T::NREAL][3];
     load_nmer<T, false>(A, t, r);
     double d[3][3], rr[3];
     if (!pair_dists<T>(r, d, rr)) {
+        double tg[T::NREAL][3];
+        scale = apply_switch<T>(d, rr, 0.0, tg, false) * (w ? w[t] : 1.0);
+    }
+    if (scale != 0.0) {
         double s[T::NSITES][3];
         T::sites(r, s);
         T::vars(s, x);
         T::to_w(x);
-        double tg[T::NREAL][3];
-        scale = apply_switch<T>(d, rr, 0.0, tg, false) * (w ? w[t] : 1.0);
-    }
+    } else {
 #pragma unroll
-    for (int v = 0; v < T::NVARS; ++v) wv[(size_t)v * count + i] = scale != 0.0 ? x[v] : 0.0;
+        for (int v = 0; v < T::NVARS; ++v) x[v] = 0.0;
+    }
+    return scale;
+}
+
+// First step of the coefficient adjoint (coef_adjoint_kernel has the second):
+// the w variables of n-mers first .. first + count and, as row NVARS, their
+// weight times the switch, variable-major in wv with stride count.  One n-mer
+// per thread.
+template <class T>
+__global__ void __launch_bounds__(128) holder_wvars_kernel(const HolderArgs A, const double* __restrict__ w,
+                                                           long first, int count, double* __restrict__ wv) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    double x[T::NVARS];
+    const double scale = adjoint_vars<T>(A, w, first + i, x);
+#pragma unroll
+    for (int v = 0; v < T::NVARS; ++v) wv[(size_t)v * count + i] = x[v];
     wv[(size_t)T::NVARS * count + i] = scale;
+}
+
+// The whole coefficient adjoint of a polynomial of at most MBX_SMALL_TERMS
+// terms: an n-mer per thread, every term's sum over a warp by shuffles, over a
+// block's warps and n-mers in shared memory, over the blocks by the block that
+// finishes last, always in the same order.  part: MBX_SMALL_TERMS doubles a
+// block; ticket: 0 before and after.  Bound by the launch and, above some 10^5
+// n-mers, by the shuffles.  A call for the 9 terms of Na-Na: 23, 31 and 36 us
+// for 1, 30,000 and 150,000 dimers, 33, 74 and 306 through the tiles of
+// coef_adjoint_kernel and its four other launches.  The line lies between the
+// library's 23 terms (He-He: 34 us for 30,000, 75) and 62 (CS-H2: 49 us through
+// the tiles; walking as many terms took 65).
+template <class T>
+__global__ void __launch_bounds__(128) holder_dcoef_small_kernel(const HolderArgs A, const double* __restrict__ w,
+                                                                 const AdjointTable P, double* part, unsigned* ticket,
+                                                                 double* out) {
+    __shared__ double xs[4][T::NVARS][32], sum[4][MBX_SMALL_TERMS];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    sum[warp][lane] = 0.0;
+    for (long base = blockIdx.x * (long)blockDim.x; base < A.n; base += (long)gridDim.x * blockDim.x) {
+        const long t = base + threadIdx.x;
+        double x[T::NVARS], scale = 0.0;
+#pragma unroll
+        for (int v = 0; v < T::NVARS; ++v) x[v] = 0.0;
+        if (t < A.n) scale = adjoint_vars<T>(A, w, t, x);
+#pragma unroll
+        for (int v = 0; v < T::NVARS; ++v) xs[warp][v][lane] = x[v];
+        __syncwarp();
+        const auto xv = [&](int v) { return xs[warp][v][lane]; };
+        for (int q = 0; q < P.nterms; ++q) {
+            double v = term_value<T::TPAIRS>(__ldg(P.terms + q), scale, xv);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) sum[warp][q] += v;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    if (warp == 0) {
+        part[blockIdx.x * MBX_SMALL_TERMS + lane] = sum[0][lane] + sum[1][lane] + sum[2][lane] + sum[3][lane];
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double v = 0.0;
+    for (int b = warp; b < gridDim.x; b += 4) v += __ldcg(part + b * MBX_SMALL_TERMS + lane);
+    sum[warp][lane] = v;
+    __syncthreads();
+    if (warp == 0) sum[0][lane] += sum[1][lane] + sum[2][lane] + sum[3][lane];
+    __syncthreads();
+    // dE/dc of every w coefficient, then F^T of those
+    double* dc = sum[1];
+    for (int j = threadIdx.x; j < P.ncw; j += blockDim.x) {
+        double d = 0.0;
+        for (int q = P.first[j]; q < P.first[j + 1]; ++q) d = fma(P.tcoef[q], sum[0][q], d);
+        dc[j] = d;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < P.ncoef; k += blockDim.x) {
+        double d = 0.0;
+        for (int q = P.ftrow[k]; q < P.ftrow[k + 1]; ++q) d = fma(P.ftf[q], dc[P.ftk[q]], d);
+        out[k] += d;
+    }
+    if (threadIdx.x == 0) *ticket = 0;
 }

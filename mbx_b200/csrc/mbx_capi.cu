@@ -37,6 +37,8 @@ int mbx_launch_ps1b(const OneBodyArgs& A, int sms, cudaStream_t s);
 
 typedef int (*launch_fn)(const HolderArgs&, int, int, cudaStream_t);
 typedef int (*dcoef_fn)(const HolderArgs&, const double*, long, int, double*, cudaStream_t);
+typedef int (*dsmall_fn)(const HolderArgs&, const double*, const AdjointTable&, double*, unsigned*, double*, int,
+                         cudaStream_t);
 typedef int (*prime_fn)(cudaStream_t);
 typedef int (*setcoef_fn)(const double*, int, cudaStream_t);
 
@@ -50,6 +52,7 @@ struct EvaluatorInfo {
     const double* fit;
     launch_fn g, e;   // straight-line FP64 kernels (energy + gradient, energy only)
     dcoef_fn c;       // variables of the coefficient adjoint
+    dsmall_fn d;      // the whole adjoint of a polynomial of few terms, or null
     launch_fn s;      // FP32 kernel of the mixed mode (FP32 basis), or null
     double split_r;   // mixed mode: n-mers with first-atom distance below this run in FP64 (0: none)
     prime_fn pg, pe, ps;   // code prefetch of the g, e and s kernels (prime_pieces), or null
@@ -354,7 +357,9 @@ struct BuildScratch {
 #define MBX_CTL_RESULTS (MBX_CTL_STATUS + 2)
 #define MBX_CTL_COUNTERS MBX_CTL_RESULTS
 #define MBX_CTL_SIZE (MBX_CTL_COUNTERS + (MBX_MAX_BUCKETS + 1) / 2)
-static_assert(MBX_CTL_SIZE <= 64, "pinned result block too small");
+// ticket of holder_dcoef_small_kernel, which leaves it 0: cleared once
+#define MBX_CTL_TICKET 63
+static_assert(MBX_CTL_SIZE <= MBX_CTL_TICKET, "pinned result block too small");
 
 // A part of the control block.
 template <class T>
@@ -407,6 +412,7 @@ struct mbx_ctx {
     CtlPart<double> out;
     CtlPart<int> bucket_count, status, counters;
     CtlPart<unsigned long long> listed;
+    CtlPart<unsigned> ticket;
     BuildScratch scratch;   // of every search (a batch searches all its configurations at once)
     // code prefetch of a term's evaluation kernels, beside its n-mer search
     cudaStream_t prime_stream = nullptr;
@@ -515,6 +521,8 @@ int mbx_create(mbx_ctx** out, int device, void* stream) {
     c->bucket_count.p = reinterpret_cast<int*>(c->ctl.p + MBX_CTL_COUNTS);
     c->status.p = reinterpret_cast<int*>(c->ctl.p + MBX_CTL_STATUS);
     c->counters.p = reinterpret_cast<int*>(c->ctl.p + MBX_CTL_COUNTERS);
+    c->ticket.p = reinterpret_cast<unsigned*>(c->ctl.p + MBX_CTL_TICKET);
+    CUCHK(c, cudaMemsetAsync(c->ctl.p, 0, 64 * sizeof(double), c->stream));
     for (int nb = 0; nb < 4; ++nb)
         for (int b = 0; b < MBX_MAX_BUCKETS; ++b) c->bucket_cap[nb][b] = 0;
     // the fitted coefficients (constant banks, per device: loaded by the
@@ -1822,12 +1830,8 @@ extern "C" int mbx_evaluate_dcoef(mbx_ctx* c, const char* name, long n, const do
     A.xyz = X;
     table_args(c, E, A);
     if (n > 0) {
-        // the variables of up to kAdjointChunk n-mers at a time in scratch, with
-        // the blocks' sums per term
-        constexpr long kAdjointChunk = 32768;
         const TermTableInfo& T = mbx_term_tables[E->table];
-        const int chunk = (int)std::min(n, kAdjointChunk);
-        const AdjointTable P{A.tcoef, (int)A.nterms, T.nhalf, E->nvars, E->ncoef, T.ncw,
+        const AdjointTable P{A.terms, A.tcoef, (int)A.nterms, T.nhalf, E->nvars, E->ncoef, T.ncw,
                              reinterpret_cast<const int2*>(c->tables.blob + T.off_half),
                              reinterpret_cast<const unsigned*>(c->tables.blob + T.off_pair),
                              reinterpret_cast<const int*>(c->tables.blob + T.off_term),
@@ -1835,12 +1839,21 @@ extern "C" int mbx_evaluate_dcoef(mbx_ctx* c, const char* name, long n, const do
                              reinterpret_cast<const int*>(c->tables.blob + T.off_ftrow),
                              reinterpret_cast<const int*>(c->tables.blob + T.off_ftk),
                              reinterpret_cast<const double*>(c->tables.blob + T.off_ftf)};
-        const size_t nv = (size_t)(E->nvars + 1) * chunk;
-        CUCHK(c, c->coef_ws.ensure(nv + (size_t)mbx_coef_adjoint_blocks(P, c->sm_count) * A.nterms + A.nterms + T.ncw));
-        for (long first = 0; first < n; first += chunk) {
-            const int count = (int)std::min<long>(chunk, n - first);
-            RCHK(c, E->c(A, W, first, count, c->coef_ws.p, c->stream));
-            RCHK(c, mbx_launch_coef_adjoint(c->coef_ws.p, count, P, c->coef_ws.p + nv, O, c->sm_count, c->stream));
+        if (E->d) {
+            CUCHK(c, c->coef_ws.ensure((size_t)2 * c->sm_count * MBX_SMALL_TERMS));
+            RCHK(c, E->d(A, W, P, c->coef_ws.p, c->ticket.p, O, c->sm_count, c->stream));
+        } else {
+            // the variables of up to kAdjointChunk n-mers at a time in scratch,
+            // with the blocks' sums per term
+            constexpr long kAdjointChunk = 32768;
+            const int chunk = (int)std::min(n, kAdjointChunk);
+            const size_t nv = (size_t)(E->nvars + 1) * chunk;
+            CUCHK(c, c->coef_ws.ensure(nv + (size_t)mbx_coef_adjoint_blocks(P, c->sm_count) * A.nterms + A.nterms + T.ncw));
+            for (long first = 0; first < n; first += chunk) {
+                const int count = (int)std::min<long>(chunk, n - first);
+                RCHK(c, E->c(A, W, first, count, c->coef_ws.p, c->stream));
+                RCHK(c, mbx_launch_coef_adjoint(c->coef_ws.p, count, P, c->coef_ws.p + nv, O, c->sm_count, c->stream));
+            }
         }
     }
     if (!dev) {

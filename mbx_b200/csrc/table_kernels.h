@@ -20,6 +20,7 @@ int mbx_launch_poly_table(long nd, int nvars, const double* x, double* g, double
                           cudaStream_t s);
 
 struct AdjointTable {
+    const int4* terms;
     const double* tcoef;
     int nterms, nhalf, nvars, ncoef, ncw;
     const int2* half;
@@ -34,3 +35,7 @@ struct AdjointTable {
 int mbx_coef_adjoint_blocks(const AdjointTable& P, int sms);
 int mbx_launch_coef_adjoint(const double* wv, int count, const AdjointTable& P, double* work, double* out, int sms,
                             cudaStream_t s);
+
+// Polynomials of at most this many terms have their adjoint in one kernel
+// (holder_dcoef_small_kernel).
+#define MBX_SMALL_TERMS 32

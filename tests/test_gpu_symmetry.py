@@ -81,10 +81,14 @@ def nmers(name, n, seed):
 
 # one n-mer; a tile of 8 and one more; several blocks; more than one chunk of
 # 32768; one range of terms (mbpol2b), two (mbpol3b), half-monomials of degree
-# 3 (h2oli2b) and more (nana2b, one variable)
+# 3 (h2oli2b); fewer terms than a warp's lanes times two (csh22b); few enough
+# for one kernel (nana2b, hehe2b), with one block, two, and more n-mers than
+# threads
 @pytest.mark.parametrize("name,n", [("mbpol2b", 1), ("mbpol2b", 8), ("mbpol2b", 9), ("mbpol2b", 32769),
                                     ("mbpol3b", 1000), ("h2oli2b", 77), ("clh2o3b", 50), ("nana2b", 5),
-                                    ("h2ona3b", 60), ("ch4ch42b", 20)])
+                                    ("h2ona3b", 60), ("ch4ch42b", 20),
+                                    ("nana2b", 128), ("nana2b", 129), ("nana2b", 40000), ("hehe2b", 300),
+                                    ("csh22b", 33), ("csh22b", 33000)])
 def test_adjoint_is_the_energy_per_coefficient(ctx, name, n):
     """The energy is linear in the coefficients: sum_k a_k dE/da_k = E; every
     dE/da_k is the oracle's sum over the terms in x; and the sums are made in

@@ -194,7 +194,8 @@ def _op_nmer_energies(xyz: torch.Tensor, coef: torch.Tensor, name: str, mixed: b
     c.set_coefficients(name, coef.contiguous())
     x = xyz.contiguous()
     e = torch.empty(x.shape[0], dtype=torch.float64, device=x.device)
-    c.evaluate(name, x, None, None, e, mixed=mixed, grads=False)
+    # (energies alone: the FP64 kernel in either precision)
+    c.evaluate_async(name, x, None, e)
     return e
 
 
@@ -213,7 +214,10 @@ def _op_nmer_energies_backward(ge: torch.Tensor, xyz: torch.Tensor, coef: torch.
     c.set_coefficients(name, coef.contiguous())
     x = xyz.contiguous()
     g = torch.zeros_like(x)
-    c.evaluate(name, x, g, None, None, mixed=mixed, grads=True)
+    if mixed:
+        c.evaluate(name, x, g, None, None, mixed=True, grads=True)
+    else:
+        c.evaluate_async(name, x, g)
     dcoef = torch.zeros_like(coef)
     c.evaluate_dcoef(name, x, ge.contiguous(), dcoef)
     return g * ge[:, None], dcoef
